@@ -30,6 +30,10 @@ struct jr_plan3d {
   std::vector<double> wall_mid;
   double* work = nullptr;      // the Newton step's vectors
   int* flag = nullptr;
+  // the linearised J.v's buffers, made by the first Newton steps (a plan that only evaluates
+  // residuals never pays for them)
+  double *lin_face = nullptr, *lin_cell = nullptr, *lin_dq = nullptr;
+  bool lin_made = false;
   cudaStream_t st = nullptr;
 };
 
@@ -49,6 +53,54 @@ template <class T> static int copy3(jr_plan3d* p, const T** dst, const T* src, s
     return report_error(JR_ECUDA, "cudaMemcpy to the device failed");
   *dst = static_cast<const T*>(d);
   return JR_OK;
+}
+
+// The linearised J.v's buffers.  Where they do not fit, the plan keeps its Newton steps on
+// the dual-number J.v, which needs none.
+static void make_lin(jr_plan3d* p) {
+  if (p->lin_made) return;
+  p->lin_made = true;
+  size_t face, cell, tangents;
+  lin3_sizes(p->dev, face, cell, tangents);
+  void* mem = nullptr;
+  if (cudaMalloc(&mem, (face + cell + tangents) * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  p->allocs.push_back(mem);
+  p->lin_face = static_cast<double*>(mem);
+  p->lin_cell = p->lin_face + face;
+  p->lin_dq = p->lin_cell + cell;
+}
+
+// Every ghost's program (Plan3Dev::ghost_of): the record that writes it last, back through
+// the records that had filled each source before its stage, to a cell of its own state.
+static void ghost_programs(const jr_plan3d_desc* d, size_t n, std::vector<int>& ghost_of, std::vector<int>& root,
+                           std::vector<int>& off, std::vector<int>& rec) {
+  std::vector<int> last(n, -1), parent;
+  int at = 0;
+  for (int s = 0; s < d->n_stages; ++s) {
+    const int end = at + d->stage_records[s];
+    for (int r = at; r < end; ++r) parent.push_back(last[d->source[r]]);
+    for (int r = at; r < end; ++r) last[d->ghost[r]] = r;
+    at = end;
+  }
+  ghost_of.assign(n, -1);
+  off.assign(1, 0);
+  std::vector<int> chain;
+  for (size_t c = 0; c < n; ++c) {
+    if (last[c] < 0) continue;
+    ghost_of[c] = (int)root.size();
+    chain.clear();
+    int r = last[c];
+    for (;; r = parent[r]) {
+      if (d->kind[r] != 0) chain.push_back(r);
+      if (parent[r] < 0) break;
+    }
+    root.push_back(d->source[r]);
+    rec.insert(rec.end(), chain.rbegin(), chain.rend());
+    off.push_back((int)rec.size());
+  }
 }
 
 #define TRY3(x)              \
@@ -132,8 +184,14 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   dv.n_stages = d->n_stages;
   dv.stage_off[0] = 0;
   for (int s = 0; s < d->n_stages; ++s) dv.stage_off[s + 1] = dv.stage_off[s] + d->stage_records[s];
-  TRY3(copy3(p, &dv.g_ghost, d->ghost, n_rec));
-  TRY3(copy3(p, &dv.g_source, d->source, n_rec));
+  {
+    std::vector<int> ghost_of, root, off, rec;
+    ghost_programs(d, n, ghost_of, root, off, rec);
+    TRY3(copy3(p, &dv.ghost_of, ghost_of.data(), ghost_of.size()));
+    TRY3(copy3(p, &dv.gp_root, root.data(), root.size()));
+    TRY3(copy3(p, &dv.gp_off, off.data(), off.size()));
+    TRY3(copy3(p, &dv.gp_rec, rec.data(), rec.size()));
+  }
   TRY3(copy3(p, &dv.g_kind, d->kind, n_rec));
   TRY3(copy3(p, &dv.g_normal, d->normal, 3 * n_rec));
   TRY3(copy3(p, &dv.neighbours, d->neighbours, n));
@@ -186,17 +244,6 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
     }
     p->allocs.push_back(sc);
     p->factor = sc;
-  }
-  {
-    size_t most = 1;
-    for (int s = 0; s < d->n_stages; ++s) most = (size_t)d->stage_records[s] > most ? (size_t)d->stage_records[s] : most;
-    void* gb = nullptr;
-    if (cudaMalloc(&gb, most * d->nvar * sizeof(Dual)) != cudaSuccess) {
-      jr_plan3d_destroy(p);
-      return report_error(JR_ENOMEM, "cudaMalloc failed");
-    }
-    p->allocs.push_back(gb);
-    dv.ghost_buf = gb;
   }
   {
     const size_t nf = (size_t)(d->NI + 1) * d->NJ * d->NK + (size_t)d->NI * (d->NJ + 1) * d->NK +
@@ -306,6 +353,10 @@ int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, 
   ops.factor = plan->factor;
   ops.line = plan->cfg.preconditioner >= 1;
   ops.st = plan->st;
+  make_lin(plan);
+  ops.lin_face = plan->lin_face;
+  ops.lin_cell = plan->lin_cell;
+  ops.lin_dq = plan->lin_dq;
   ops.bind(plan->work, plan->flag, plan->cfg.restart);
   double c = *cfl, r = *residual_norm;
   for (int s = 0; s < n_steps; ++s) {

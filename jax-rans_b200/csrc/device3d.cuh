@@ -46,7 +46,15 @@ struct Plan3Dev {
   int line_fp32;               // the line factor and apply in FP32 (the mixed form)
   int line_coupled;            // the SA row coupled to the neighbours' mean flow (6x6 blocks)
   double* face_buf;            // the residual's face fluxes: nvar x (all three families' faces)
-  void* ghost_buf;             // one ghost stage's values: nvar x (the largest stage's records), Dual-sized
+  // The ghost fill as one gather: every ghost the stages write ends as a chain of conditions
+  // applied to one cell's own state (each record has one source, which an earlier stage may
+  // have filled in turn).  ghost_of: canvas cell -> its program, -1 where the cell keeps its
+  // own state; program g starts from cell gp_root[g] and applies records gp_rec[gp_off[g]] ..
+  // gp_rec[gp_off[g + 1] - 1] in order (copies left out).
+  const int* ghost_of;
+  const int* gp_root;
+  const int* gp_off;
+  const int* gp_rec;
   const double* face_geo;      // viscous: per face (flat over the families) its diamond gradient's
                                // geometry, 10 planes: the cross products c23, c31, c12 (3 each), det
   void* node_buf;              // viscous: per node (NI+1)(NJ+1)(NK+1) the mean of its eight cells'
@@ -240,6 +248,15 @@ __host__ __device__ __forceinline__ void condition3(int kind, const T* q, double
 void launch_residual3(const Plan3Dev& p, const double* U, double* R, void* A, bool first_order, cudaStream_t st);
 // the exact tangent of the first-order residual at U along v (A: a Dual-sized canvas)
 void launch_jvp3(const Plan3Dev& p, const double* U, const double* v, double* Jv, void* A, cudaStream_t st);
+// U's ghost-filled primitive canvas into Q (nvar planes), and its node values into p.node_buf
+void launch_canvas3(const Plan3Dev& p, const double* U, double* Q, cudaStream_t st);
+void launch_nodes3(const Plan3Dev& p, const double* Q, cudaStream_t st);
+// the linearised J.v (linearize3d.cuh): its buffers' sizes in doubles, the factors at U, and
+// w = vdt z + dR1/dU z from them
+void lin3_sizes(const Plan3Dev& p, size_t& face, size_t& cell, size_t& tangents);
+void launch_linearize3(const Plan3Dev& p, const double* U, double* Q, double* face, double* cell, cudaStream_t st);
+void launch_lin_jv3(const Plan3Dev& p, const double* U, const double* Q, const double* face, const double* cell,
+                    double* dq, const double* z, const double* vdt, double* w, cudaStream_t st);
 void launch_wave_speeds3(const Plan3Dev& p, const double* U, double* lam, cudaStream_t st);
 void launch_wall_loads3(const Plan3Dev& p, const double* U, double* loads, void* A, cudaStream_t st);
 // the viscous faces' diamond-gradient geometry into geo (10 x all faces), once per plan

@@ -170,11 +170,18 @@ void DeviceOps3::prepare(const double* U, double cfl) {
   counted3();
   k3_vdt<<<grid_of(n), 128, 0, st>>>(p, U, cfl, vdt);
   if (line) launch_line_factor3(p, U, cfl, factor, st);
+  // the tangent map of this step's products; its canvas (A) is the residual's too, which
+  // leaves the same values there
+  if (lin_face != nullptr) launch_linearize3(p, U, static_cast<double*>(A), lin_face, lin_cell, st);
 }
 
 void DeviceOps3::residual(const double* U, int out) { launch_residual3(p, U, v(out), A, false, st); }
 
 void DeviceOps3::matvec(const double* U, double, int src, int out) {
+  if (lin_face != nullptr) {
+    launch_lin_jv3(p, U, static_cast<const double*>(A), lin_face, lin_cell, lin_dq, v(src), vdt, v(out), st);
+    return;
+  }
   launch_jvp3(p, U, v(src), v(out), A, st);
   counted3();
   k3_vdt_add<<<grid_of(N), 256, 0, st>>>(N, n, vdt, v(src), v(out));

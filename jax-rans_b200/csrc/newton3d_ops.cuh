@@ -15,6 +15,9 @@ struct DeviceOps3 {
   void* A = nullptr;                 // the primitive canvas of the residual / J.v (Dual-sized)
   void* factor = nullptr;            // the line factor (computed in prepare when line)
   bool line = false;
+  // the linearised J.v's buffers (linearize3d.cuh); null where they did not fit the device's
+  // memory: the products are then evaluated by the dual-number J.v
+  double *lin_face = nullptr, *lin_cell = nullptr, *lin_dq = nullptr;
   double* vecs = nullptr;
   double* vdt = nullptr;
   double* partial = nullptr;

@@ -2,8 +2,8 @@
 // wing's C-H block; the reference's 3D path, src/jaxrans/numerics/residual.py:54-91,
 // 273-334, on the canvas of src/jaxrans/mesh/atlas3d.py:119-210).
 //
-// The ghost fill runs its gather stages as record kernels (one thread per ghost record,
-// double-buffered so every read of a stage precedes its writes); then one thread per
+// One kernel fills the primitive canvas, ghosts included (each by its chain of conditions);
+// then one thread per
 // face evaluates its flux once -- MUSCL on the flow rows, HLLC or Roe with a vector
 // normal, the 3D diamond face gradient, the viscous flux (with QCR2000), the SA row's
 // convection and diffusion -- into a face buffer, and one thread per cell sums F_hi -
@@ -17,31 +17,36 @@
 
 namespace jr {
 
+// U's (and, for Dual, its tangent dU's) ghost-filled primitive canvas Q, one thread a cell: a
+// cell's own state, or a ghost's by its program.  One launch in place of a canvas pass and
+// two launches for each of the fill's three to twelve stages.
 template <class T, int NV>
-__global__ void k3_prim(Plan3Dev p, const double* __restrict__ U, const double* __restrict__ dU, T* __restrict__ Q) {
+__global__ void __launch_bounds__(128, 8) k3_canvas(Plan3Dev p, const double* __restrict__ U,
+                                                 const double* __restrict__ dU, T* __restrict__ Q) {
   const int n = p.NI * p.NJ * p.NK;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    prim_cell_n<NV>(p, U, dU, Q, c);
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+    const int g = p.ghost_of[c];
+    if (g < 0) {
+      prim_cell_n<NV>(p, U, dU, Q, c);
+    } else {
+      T q[NV3_MAX];
+      ghost_state<NV>(p, U, dU, g, q);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) Q[(size_t)v * n + c] = q[v];
+    }
+  }
 }
 
-// the primitive canvas of U (and dU) into Q
 template <class T>
-static void prim_canvas(const Plan3Dev& p, const double* U, const double* dU, T* Q, cudaStream_t st) {
+static void canvas3(const Plan3Dev& p, const double* U, const double* dU, T* Q, cudaStream_t st) {
   const int blocks = (p.NI * p.NJ * p.NK + 127) / 128;
-  if (p.nvar > 5) k3_prim<T, 6><<<blocks, 128, 0, st>>>(p, U, dU, Q);
-  else k3_prim<T, 5><<<blocks, 128, 0, st>>>(p, U, dU, Q);
+  counted3();
+  if (p.nvar > 5) k3_canvas<T, 6><<<blocks, 128, 0, st>>>(p, U, dU, Q);
+  else k3_canvas<T, 5><<<blocks, 128, 0, st>>>(p, U, dU, Q);
 }
 
-template <class T>
-__global__ void k3_ghost_values(Plan3Dev p, const T* __restrict__ Q, int r0, int r1, T* __restrict__ buf) {
-  for (int r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1; r += gridDim.x * blockDim.x)
-    ghost_value(p, Q, r, r0, r1 - r0, buf);
-}
-
-template <class T>
-__global__ void k3_ghost_store(Plan3Dev p, const T* __restrict__ buf, int r0, int r1, T* __restrict__ Q) {
-  for (int r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1; r += gridDim.x * blockDim.x)
-    ghost_store(p, buf, r, r0, r1 - r0, Q);
+void launch_canvas3(const Plan3Dev& p, const double* U, double* Q, cudaStream_t st) {
+  canvas3<double>(p, U, nullptr, Q, st);
 }
 
 // phase 1: every face's flux once (one thread per face of the three families)
@@ -117,32 +122,15 @@ __global__ void __launch_bounds__(128) k3_cell_sum(Plan3Dev p, const T* __restri
 }
 
 // ---- launchers
-// the ghost stages on the canvas A in place, each in two passes through p.ghost_buf
-template <class T>
-static void fill3(const Plan3Dev& p, T* A, cudaStream_t st) {
-  T* buf = static_cast<T*>(p.ghost_buf);
-  for (int s = 0; s < p.n_stages; ++s) {
-    const int r0 = p.stage_off[s], r1 = p.stage_off[s + 1];
-    const int blocks = (r1 - r0 + 127) / 128;
-    if (blocks > 0) {
-      counted3(2);
-      k3_ghost_values<T><<<blocks, 128, 0, st>>>(p, A, r0, r1, buf);
-      k3_ghost_store<T><<<blocks, 128, 0, st>>>(p, buf, r0, r1, A);
-    }
-  }
-}
-
 template <class T>
 static void residual3_t(const Plan3Dev& p, const double* U, const double* dU, double* R, T* A, bool first_order,
                         cudaStream_t st) {
   const int n = p.NI * p.NJ * p.NK;
   const int blocks = (n + 127) / 128;
-  counted3(2);   // the primitive canvas and, below, the residual
-  prim_canvas<T>(p, U, dU, A, st);
-  fill3(p, A, st);
+  canvas3<T>(p, U, dU, A, st);
   const bool visc = p.P.mu_inf > 0.0, sa = p.nvar > 5;
   const int nf = face_count(p, 0) + face_count(p, 1) + face_count(p, 2);
-  counted3();   // the face phase (the cell phase is counted with the primitive canvas)
+  counted3(2);   // the face phase and the cell phase
   if (sa)
     face_phase<T, true, true>(p, A, first_order, nf, st);
   else if (visc)
@@ -163,10 +151,16 @@ __global__ void k3_wall_loads(Plan3Dev p, const double* __restrict__ Q, double* 
 // the loads on every wall face (7 each) at U: the primitive canvas ghost-filled first
 void launch_wall_loads3(const Plan3Dev& p, const double* U, double* loads, void* A, cudaStream_t st) {
   const int n = p.NI * p.NJ * p.NK;
-  counted3(p.n_walls > 0 ? 2 : 1);
-  prim_canvas<double>(p, U, nullptr, (double*)A, st);
-  fill3(p, (double*)A, st);
+  counted3(p.n_walls > 0);
+  canvas3<double>(p, U, nullptr, (double*)A, st);
   if (p.n_walls > 0) k3_wall_loads<<<(p.n_walls + 127) / 128, 128, 0, st>>>(p, (const double*)A, loads);
+}
+
+void launch_nodes3(const Plan3Dev& p, const double* Q, cudaStream_t st) {
+  const int nn = node_count(p);
+  counted3();
+  if (p.nvar > 5) k3_node_phi<double, 5><<<(nn + 127) / 128, 128, 0, st>>>(p, Q);
+  else k3_node_phi<double, 4><<<(nn + 127) / 128, 128, 0, st>>>(p, Q);
 }
 
 void launch_residual3(const Plan3Dev& p, const double* U, double* R, void* A, bool first_order, cudaStream_t st) {

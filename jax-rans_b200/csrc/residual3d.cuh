@@ -66,6 +66,27 @@ __host__ __device__ __forceinline__ void ghost_store(const Plan3Dev& p, const T*
   for (int v = 0; v < p.nvar; ++v) Q[(size_t)v * n + ghost] = buf[(size_t)v * count + (r - r0)];
 }
 
+// The state of the ghost whose program is g (Plan3Dev::ghost_of), from U (and its tangent
+// dU for Dual): the records of the stages one after another on the root cell's own state --
+// what the stages leave in that ghost, without the canvases between them.
+template <int NV, class T>
+__host__ __device__ __forceinline__ void ghost_state(const Plan3Dev& p, const double* U, const double* dU, int g,
+                                                     T* q) {
+  const int n = p.NI * p.NJ * p.NK;
+  const int c = p.gp_root[g];
+  T u[NV3_MAX];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) u[v] = mk<T>(U[(size_t)v * n + c], dU ? dU[(size_t)v * n + c] : 0.0);
+  to_prim3(u, q, NV, p.P.gamma);
+  for (int e = p.gp_off[g]; e < p.gp_off[g + 1]; ++e) {
+    const int r = p.gp_rec[e];
+    T o[NV3_MAX];
+    condition3(p.g_kind[r], q, p.g_normal[3 * r], p.g_normal[3 * r + 1], p.g_normal[3 * r + 2], p.P, NV, o);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) q[v] = o[v];
+  }
+}
+
 // ---- geometry access
 // faces of family a on the canvas (one more than the cells along a)
 __host__ __device__ __forceinline__ int face_count(const Plan3Dev& p, int a) {
