@@ -1,5 +1,6 @@
 // The C ABI of the 3D path: a plan of one 3D case (device copies of its canvas tables
 // and ghost records, two work buffers, a stream), its residual and its J.v.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -23,7 +24,7 @@ struct jr_plan3d {
   Plan3Dev dev{};
   std::vector<void*> allocs;
   void* A = nullptr;   // primitive canvases (Dual-sized: the J.v needs value and tangent)
-  void* factor = nullptr;      // the line factor: n_chains * chain_L * FACTOR3 words (FP32 in the mixed form)
+  void* factor = nullptr;      // the line factor: line_factor_words3 words (FP32 in the mixed form)
   size_t n_canvas = 0;
   Newton3Config cfg{};
   double* loads = nullptr;     // 7 per wall face
@@ -78,7 +79,9 @@ static void make_lin(jr_plan3d* p) {
 static void ghost_programs(const jr_plan3d_desc* d, size_t n, std::vector<int>& ghost_of, std::vector<int>& root,
                            std::vector<int>& off, std::vector<int>& rec) {
   std::vector<int> last(n, -1), parent;
-  int at = 0;
+  int at = 0, total = 0;
+  for (int s = 0; s < d->n_stages; ++s) total += d->stage_records[s];
+  parent.reserve(total);
   for (int s = 0; s < d->n_stages; ++s) {
     const int end = at + d->stage_records[s];
     for (int r = at; r < end; ++r) parent.push_back(last[d->source[r]]);
@@ -87,12 +90,14 @@ static void ghost_programs(const jr_plan3d_desc* d, size_t n, std::vector<int>& 
   }
   ghost_of.assign(n, -1);
   off.assign(1, 0);
+  off.reserve((size_t)total + 1);
+  root.reserve(total);
   std::vector<int> chain;
-  for (size_t c = 0; c < n; ++c) {
-    if (last[c] < 0) continue;
-    ghost_of[c] = (int)root.size();
+  for (int w = 0; w < total; ++w) {
+    if (last[d->ghost[w]] != w) continue;   // written again by a later record
+    ghost_of[d->ghost[w]] = (int)root.size();
     chain.clear();
-    int r = last[c];
+    int r = w;
     for (;; r = parent[r]) {
       if (d->kind[r] != 0) chain.push_back(r);
       if (parent[r] < 0) break;
@@ -200,6 +205,23 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   TRY3(copy3(p, &dv.ch_cells, d->chain_cells, n_links));
   TRY3(copy3(p, &dv.ch_face, d->chain_up_face, n_links));
   TRY3(copy3(p, &dv.ch_sign, d->chain_up_sign, n_links));
+  {
+    // each chain's length (to its first -1) and the cells on none
+    std::vector<int> len(d->n_chains), off;
+    std::vector<char> on(n, 0);
+    for (int c = 0; c < d->n_chains; ++c) {
+      const int* cells = d->chain_cells + (size_t)c * d->chain_L;
+      int k = 0;
+      for (; k < d->chain_L && cells[k] >= 0; ++k) on[cells[k]] = 1;
+      len[c] = k;
+    }
+    off.reserve(n - std::min(n, n_links));
+    for (size_t c = 0; c < n; ++c)
+      if (!on[c]) off.push_back((int)c);
+    dv.n_offchain = (int)off.size();
+    TRY3(copy3(p, &dv.ch_len, len.data(), len.size()));
+    TRY3(copy3(p, &dv.offchain, off.data(), off.size()));
+  }
   if (d->n_walls < 0 || (d->n_walls > 0 && (!d->wall_cell || !d->wall_family || !d->wall_face || !d->wall_into ||
                                             !d->wall_mid))) {
     jr_plan3d_destroy(p);
@@ -238,7 +260,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   dv.line_coupled = d->preconditioner == 2;
   if (n_links > 0) {
     void* sc = nullptr;
-    if (cudaMalloc(&sc, n_links * FACTOR3 * (dv.line_fp32 ? sizeof(float) : sizeof(double))) != cudaSuccess) {
+    if (cudaMalloc(&sc, line_factor_words3(dv) * (dv.line_fp32 ? sizeof(float) : sizeof(double))) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }

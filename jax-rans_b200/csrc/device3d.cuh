@@ -62,6 +62,9 @@ struct Plan3Dev {
   const int* ch_cells;         // [chain * chain_L + k], -1 past the chain's end
   const int* ch_face;          // link k -> k+1: flat index into the three face families, concatenated
   const int* ch_sign;          // +1 / -1: the link face's vector points out of / into cell k; 0 none
+  const int* ch_len;           // each chain's cells before its first -1
+  int n_offchain;              // the cells on no chain
+  const int* offchain;
   int n_walls;                 // wall faces: the cell on each, the face's family and index in it,
   const int* w_cell;           // +1 where its vector points into the fluid
   const int* w_family;
@@ -261,11 +264,13 @@ void launch_wave_speeds3(const Plan3Dev& p, const double* U, double* lam, cudaSt
 void launch_wall_loads3(const Plan3Dev& p, const double* U, double* loads, void* A, cudaStream_t st);
 // the viscous faces' diamond-gradient geometry into geo (10 x all faces), once per plan
 void launch_face_geometry3(const Plan3Dev& p, double* geo, cudaStream_t st);
-void launch_line_factor3(const Plan3Dev& p, const double* U, double cfl, void* F, cudaStream_t st);
-void launch_line_apply3(const Plan3Dev& p, const void* F, const double* r, double* z, cudaStream_t st);
+size_t line_factor_words3(const Plan3Dev& p);
+void launch_line_factor3(const Plan3Dev& p, const double* U, double cfl, void* F, double* vdt, cudaStream_t st);
+void launch_line_apply3(const Plan3Dev& p, const void* F, const double* r, double* z, const double* scale, double* vout,
+                        cudaStream_t st);
 void launch_precondition3(const Plan3Dev& p, const double* U, double cfl, const double* r, double* z, void* F,
                           cudaStream_t st);
-// words per chain element of the line factor (linesolve3d.cuh): three 5x5 blocks, three
+// words per chain element of the host form's line factor (linesolve3d.cuh): three 5x5 blocks, three
 // SA scalars and the SA row's two coupling rows to the mean flow (the coupled form)
 constexpr int FACTOR3 = 88;
 

@@ -1,5 +1,4 @@
-// The 3D wave speeds and line preconditioner kernels: one thread per canvas face, one
-// thread per chain (the bodies are in linesolve3d.cuh, host-and-device code).
+// The 3D wave speeds and line preconditioner kernels (bodies and layout in linesolve3d.cuh).
 #include "linesolve3d.cuh"
 
 namespace jr {
@@ -14,25 +13,383 @@ __global__ void k3_wave_speeds(Plan3Dev p, const double* __restrict__ U, double*
   }
 }
 
-__global__ void k3_copy_rows(int n, const double* __restrict__ r, double* __restrict__ z) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) z[e] = r[e];
-}
-
-template <class TF>
-__global__ void __launch_bounds__(64) k3_chain_factor(Plan3Dev p, const double* __restrict__ U, double cfl,
-                                                      TF* __restrict__ F) {
-  for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < p.n_chains; ch += gridDim.x * blockDim.x) {
-    chain_factor_flow(p, U, cfl, ch, F);
-    if (p.nvar > 5) chain_factor_sa(p, U, cfl, ch, F);
+template <bool SA>
+__global__ void __launch_bounds__(128) k3_line_faces(Plan3Dev p, const double* __restrict__ U, double* __restrict__ lam,
+                                                     double* __restrict__ mflux, double* __restrict__ dflux, int nf) {
+  for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
+    int a, i, j, k;
+    face_of(p, f, a, i, j, k);
+    double l, m = 0.0, d = 0.0;
+    line_face_terms<SA>(p, U, a, i, j, k, l, m, d);
+    lam[f] = l;
+    if constexpr (SA) {
+      mflux[f] = m;
+      dflux[f] = d;
+    }
   }
 }
 
-template <class TF>
-__global__ void __launch_bounds__(128) k3_chain_apply(Plan3Dev p, const TF* __restrict__ F,
-                                                      const double* __restrict__ r, double* __restrict__ z) {
-  for (int ch = blockIdx.x * blockDim.x + threadIdx.x; ch < p.n_chains; ch += gridDim.x * blockDim.x) {
-    chain_apply_flow(p, ch, F, r, z);
-    if (p.nvar > 5) chain_apply_sa(p, ch, F, r, z);
+// V/dt on every cell, and where chains run (block cells) their diagonals
+template <bool SA>
+__global__ void __launch_bounds__(128) k3_line_cells(Plan3Dev p, const double* __restrict__ U,
+                                                     const double* __restrict__ lam, const double* __restrict__ mflux,
+                                                     const double* __restrict__ dflux, double cfl,
+                                                     double* __restrict__ dflow, double* __restrict__ dsa,
+                                                     double* __restrict__ vdt) {
+  const int n = p.NI * p.NJ * p.NK;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+    double sum, d = 0.0;
+    line_cell_terms<SA>(p, U, lam, mflux, dflux, cfl, c, sum, d);
+    if (vdt != nullptr) vdt[c] = sum / cfl;
+    dflow[c] = sum * (1.0 / cfl + 0.5);
+    if constexpr (SA) dsa[c] = d;
+  }
+}
+
+// The elimination down a chain: T = D - lower C_{k-1}, P = T^-1 (Gauss-Jordan, one
+// reciprocal a pivot), C = P upper, and the SA row's scalars.  One thread a chain: a step is
+// a serial chain of five pivots, so its neighbours' chains are what hides it; its rows leave
+// eight at a time, a sector a chain and word.  61,440 chains of 64: 1.1 ms, and the faces' and
+// cells' terms 1.0 ms (assembling the blocks, every wave speed of a cell twice among them,
+// as the one thread walked its chain: 16.2 ms).
+template <class TF, bool SA>
+__global__ void __launch_bounds__(64) k3_line_factor(Plan3Dev p, const double* __restrict__ U,
+                                                     const double* __restrict__ lam, const double* __restrict__ mflux,
+                                                     const double* __restrict__ dflux,
+                                                     const double* __restrict__ dflow,
+                                                     const double* __restrict__ dsa, TF* __restrict__ F) {
+  const int ch = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ch >= p.n_chains) return;
+  const double g = p.P.gamma;
+  const int groups = line_groups(p), len = p.ch_len[ch];
+  TF* out = F + ((size_t)(ch / LW_CHAINS) * LW_WORDS) * 32 + (ch % LW_CHAINS) * LW_ROWS;
+  const size_t stride = (size_t)groups * LW_WORDS * 32;
+  const bool coupled = SA && p.line_coupled;
+  double C[5][5] = {}, q[NV3_MAX] = {}, qb[NV3_MAX] = {};   // this cell's state, the one below's
+  double sl[3] = {0.0, 0.0, 0.0}, ll = 0.0, csa = 0.0, lsa = 0.0;   // the link below, outward from this cell
+  bool linked = false;
+  if (len > 0) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L], q);
+  for (int k = 0; k < len; ++k, out += stride) {
+    const int c = p.ch_cells[(size_t)ch * p.chain_L + k];
+    double T[5][5], L[5][5];
+    if (linked) coupling5_closed(qb, sl[0], sl[1], sl[2], ll, g, L);
+    else
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) L[a][b] = 0.0;
+    const double dg = dflow[c];
+#pragma unroll
+    for (int a = 0; a < 5; ++a)
+#pragma unroll
+      for (int b = 0; b < 5; ++b) {
+        double m = L[a][0] * C[0][b];
+#pragma unroll
+        for (int t = 1; t < 5; ++t) m = m + L[a][t] * C[t][b];
+        T[a][b] = (a == b ? dg : 0.0) - m;
+      }
+    // the SA row's scalars beside the mean flow's blocks, and the coupled form's rows
+    double slo = 0.0, spiv = 0.0, sc = 0.0, cpl[2][5] = {};
+    if constexpr (SA) {
+      if (!coupled) {
+        slo = lsa;
+        spiv = 1.0 / (dsa[c] - lsa * csa);
+      } else if (linked) {
+        sa_coupling_row(qb, sl, 1.0, cpl[0]);
+      }
+    }
+    // word w of the rows: the first six, or all eight
+    auto put = [&](int w, double r0, double r1, double r2, double r3, double r4, double r5, double r6, double r7) {
+      TF* o = out + w * 32;
+      if constexpr (sizeof(TF) == 4) {
+        *reinterpret_cast<float4*>(o) = make_float4((float)r0, (float)r1, (float)r2, (float)r3);
+        *reinterpret_cast<float4*>(o + 4) = make_float4((float)r4, (float)r5, (float)r6, (float)r7);
+      } else {
+        *reinterpret_cast<double2*>(o) = make_double2(r0, r1);
+        *reinterpret_cast<double2*>(o + 2) = make_double2(r2, r3);
+        *reinterpret_cast<double2*>(o + 4) = make_double2(r4, r5);
+        if (coupled) *reinterpret_cast<double2*>(o + 6) = make_double2(r6, r7);
+      }
+    };
+    // the link above: this cell's upper block and, for the next element, its lower one
+    const int sign = k + 1 < len ? p.ch_sign[(size_t)ch * p.chain_L + k] : 0;
+    double su[3] = {0.0, 0.0, 0.0}, lu = 0.0, qn[NV3_MAX] = {}, upsa = 0.0, nextsa = 0.0;
+    if (k + 1 < len) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L + k + 1], qn);
+    if (sign != 0) {
+      const int f = p.ch_face[(size_t)ch * p.chain_L + k];
+      int fa, fi, fj, fk;
+      face_of(p, f, fa, fi, fj, fk);
+      face_vector(p, fa, fi, fj, fk, su);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) su[m] *= (double)sign;
+      lu = lam[f];
+      if constexpr (SA) {
+        const double um = -(double)sign * mflux[f], d = dflux[f];
+        upsa = -((um > 0.0 ? um : 0.0) + d) / qn[0];
+        nextsa = -((-um > 0.0 ? -um : 0.0) + d) / q[0];
+        if (coupled) sa_coupling_row(qn, su, 1.0, cpl[1]);
+      }
+    }
+    if constexpr (SA) {
+      if (!coupled) csa = sc = spiv * upsa;
+      lsa = nextsa;
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(b, L[0][b], L[1][b], L[2][b], L[3][b], L[4][b], b == 0 ? slo : (b == 1 ? spiv : 0.0), 0.0, 0.0);
+    // P = T^-1 in place
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const double inv = 1.0 / T[i][i];
+      T[i][i] = 1.0;
+#pragma unroll
+      for (int b = 0; b < 5; ++b) T[i][b] = T[i][b] * inv;
+#pragma unroll
+      for (int a = 0; a < 5; ++a) {
+        if (a == i) continue;
+        const double f = T[a][i];
+        T[a][i] = 0.0;
+#pragma unroll
+        for (int b = 0; b < 5; ++b) T[a][b] = T[a][b] - f * T[i][b];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(5 + b, T[0][b], T[1][b], T[2][b], T[3][b], T[4][b], 0.0, 0.0, 0.0);
+    // C = P upper
+    if (sign != 0) {
+      double B[5][5];
+      coupling5_closed(qn, su[0], su[1], su[2], lu, g, B);
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) {
+          double m = T[a][0] * B[0][b];
+#pragma unroll
+          for (int t = 1; t < 5; ++t) m = m + T[a][t] * B[t][b];
+          C[a][b] = m;
+        }
+    } else {
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) C[a][b] = 0.0;
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(10 + b, C[0][b], C[1][b], C[2][b], C[3][b], C[4][b], b == 0 ? sc : 0.0, cpl[0][b], cpl[1][b]);
+    linked = sign != 0;
+    ll = lu;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) sl[m] = -su[m];
+#pragma unroll
+    for (int v = 0; v < NV3_MAX; ++v) {
+      qb[v] = q[v];
+      q[v] = qn[v];
+    }
+  }
+  if constexpr (SA) {
+    if (!coupled) return;
+    // the SA chain from its far end: 1 / (d_k - upper_k c_{k+1}), c_k = that times lower_k
+    TF* plane = F + line_words(p);
+    double cs = 0.0;
+    for (int k = len - 1; k >= 0; --k) {
+      out -= stride;
+      const size_t at = (size_t)ch * p.chain_L + k;
+      const int c = p.ch_cells[at], up = k + 1 < len ? p.ch_sign[at] : 0, down = k > 0 ? p.ch_sign[at - 1] : 0;
+      double u = 0.0, l = 0.0;
+      if (up != 0) {
+        const int f = p.ch_face[at];
+        const double m = -(double)up * mflux[f];
+        u = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at + 1]];
+      }
+      if (down != 0) {
+        const int f = p.ch_face[at - 1];
+        const double m = (double)down * mflux[f];
+        l = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at - 1]];
+      }
+      const double piv = 1.0 / (dsa[c] - u * cs);
+      cs = piv * l;
+      out[10 * 32 + 5] = (TF)u;
+      out[11 * 32 + 5] = (TF)piv;
+      plane[(size_t)k * groups * LW_CHAINS + ch] = (TF)cs;
+    }
+  }
+}
+
+// z = M^-1 (s r) from the factor, s = *scale (1 where null); with vout the scaled input is also
+// written there (a normalised Krylov vector).  Four chains a warp, eight lanes a chain: lane
+// `row` holds its row's words and the vector's entry, the other rows' entries come by
+// shuffles, and the words of the two elements ahead are in flight.  Bound by the factor's
+// bytes where many chains run, by the sweeps' latency where few do: 61,440 coupled FP32 chains
+// of 64, 638 us (one thread a chain and a copy of the whole vector first: 1.14 ms); 3,072
+// FP64 chains of 16, 21 us (231 us).  The blocks after the chains' copy the cells on no chain.
+constexpr int LA_THREADS = 128, LA_CHAINS = LA_THREADS / 32 * LW_CHAINS;
+
+template <class TF, int NV>
+__global__ void __launch_bounds__(LA_THREADS) k3_line_apply(Plan3Dev p, const TF* __restrict__ F,
+                                                            const double* __restrict__ r, double* __restrict__ z,
+                                                            const double* __restrict__ scale,
+                                                            double* __restrict__ vout, int chain_blocks) {
+  const size_t n = (size_t)p.NI * p.NJ * p.NK;
+  const double s = scale != nullptr ? *scale : 1.0;
+  if ((int)blockIdx.x >= chain_blocks) {
+    const size_t total = (size_t)p.n_offchain * NV, step = (size_t)(gridDim.x - chain_blocks) * LA_THREADS;
+    for (size_t e = (size_t)(blockIdx.x - chain_blocks) * LA_THREADS + threadIdx.x; e < total; e += step) {
+      const size_t at = e / p.n_offchain * n + p.offchain[e % p.n_offchain];
+      const double x = s * r[at];
+      z[at] = x;
+      if (vout != nullptr) vout[at] = x;
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, row = lane & 7, base = lane & 24;
+  const int group = blockIdx.x * (LA_THREADS / 32) + threadIdx.x / 32, groups = line_groups(p), nc = p.n_chains;
+  if (group >= groups) return;   // whole warps
+  const int ch = group * LW_CHAINS + (lane >> 3);
+  const bool mine = ch < nc && row < NV;
+  const int len = ch < nc ? p.ch_len[ch] : 0;
+  int most = len;
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 8));
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+  const bool sa = NV > 5 && row == 5, coupled = NV > 5 && p.line_coupled;
+  const size_t kstride = (size_t)groups * LW_WORDS * 32;
+  const TF* Fw = F + (size_t)group * LW_WORDS * 32 + lane;
+  const size_t ro = (size_t)row * n;
+  constexpr int D = 2;   // elements in flight
+  // 1. down: d_k = P_k (r_k - lower_k d_{k-1}); the uncoupled SA row beside the mean flow's
+  {
+    TF w[D][10];
+    double rv[D];
+    int cell[D];
+    auto fetch = [&](int k, int b) {
+      const bool in = mine && k < len;
+      cell[b] = in ? p.ch_cells[(size_t)ch * p.chain_L + k] : -1;
+      rv[b] = in ? r[ro + cell[b]] : 0.0;
+      const TF* f = Fw + (size_t)k * kstride;
+#pragma unroll
+      for (int t = 0; t < 10; ++t) w[b][t] = in ? f[t * 32] : TF(0);
+    };
+#pragma unroll
+    for (int b = 0; b < D; ++b)
+      if (b < most) fetch(b, b);
+    TF d = TF(0);
+    for (int k0 = 0; k0 < most; k0 += D) {
+#pragma unroll
+      for (int b = 0; b < D; ++b) {
+        const int k = k0 + b;
+        if (k >= most) break;
+        const double x = s * rv[b];
+        const TF mr = TF(x);
+        TF rhs, dn;
+        {
+          TF m = w[b][0] * __shfl_sync(0xffffffffu, d, base);
+#pragma unroll
+          for (int t = 1; t < 5; ++t) m = m + w[b][t] * __shfl_sync(0xffffffffu, d, base + t);
+          rhs = mr - m;
+          dn = w[b][5] * __shfl_sync(0xffffffffu, rhs, base);
+#pragma unroll
+          for (int t = 1; t < 5; ++t) dn = dn + w[b][5 + t] * __shfl_sync(0xffffffffu, rhs, base + t);
+        }
+        if (sa) dn = w[b][1] * (mr - w[b][0] * d);
+        if (cell[b] >= 0) {
+          if (!(coupled && sa)) {   // (the coupled SA row starts on the way back)
+            d = dn;
+            z[ro + cell[b]] = double(dn);
+          }
+          if (vout != nullptr) vout[ro + cell[b]] = x;
+        }
+        if (k + D < most) fetch(k + D, b);
+      }
+    }
+  }
+  // 2. back: x_k = d_k - C_k x_{k+1}.  Coupled, the SA row's right-hand side of element k + 1,
+  // r - (lo x_k + up x_{k+2}), is complete once x_k is, and the SA chain's first sweep,
+  // d_{k+1} = pivot (that - upper d_{k+2}), goes one element behind.
+  {
+    TF w[D][5];
+    double dv[D];
+    int cell[D];
+    auto fetch = [&](int k, int b) {
+      const bool in = ch < nc && k < len, vec = in && row < NV;
+      cell[b] = vec ? p.ch_cells[(size_t)ch * p.chain_L + k] : -1;
+      dv[b] = !vec ? 0.0 : (coupled && sa ? s * r[ro + cell[b]] : z[ro + cell[b]]);
+      const TF* f = Fw + (size_t)k * kstride;
+#pragma unroll
+      for (int t = 0; t < 5; ++t) w[b][t] = in && (row < NV || coupled) ? f[(10 + t) * 32] : TF(0);
+    };
+#pragma unroll
+    for (int b = 0; b < D; ++b)
+      if (most - 1 - b >= 0) fetch(most - 1 - b, b);
+    TF x = TF(0);
+    // of element k + 1: its coupling words (row 6), up x_{k+2} (row 7); the SA lane's r, upper,
+    // pivot and cell
+    TF pw[5] = {}, pup = TF(0), pr = TF(0), pupper = TF(0), ppiv = TF(0);
+    int pcell = -1;
+    auto finish = [&](TF lo) {   // the SA row's element k + 1
+      const TF lo_all = __shfl_sync(0xffffffffu, lo, base + 6), up_all = __shfl_sync(0xffffffffu, pup, base + 7);
+      if (sa && pcell >= 0) {
+        x = ppiv * ((pr - (lo_all + up_all)) - pupper * x);
+        z[ro + pcell] = double(x);
+      }
+    };
+    for (int k0 = most - 1; k0 >= 0; k0 -= D) {
+#pragma unroll
+      for (int b = 0; b < D; ++b) {
+        const int k = k0 - b;
+        if (k < 0) break;
+        TF xt[5];   // the mean flow's x_{k+1}
+#pragma unroll
+        for (int t = 0; t < 5; ++t) xt[t] = __shfl_sync(0xffffffffu, x, base + t);
+        TF m = w[b][0] * (sa ? x : xt[0]);
+        if (!sa)
+#pragma unroll
+          for (int t = 1; t < 5; ++t) m = m + w[b][t] * xt[t];
+        if (cell[b] >= 0 && !(coupled && sa)) {
+          x = TF(dv[b]) - m;
+          z[ro + cell[b]] = double(x);
+        }
+        if (coupled) {
+          TF lo = pw[0] * __shfl_sync(0xffffffffu, x, base);
+#pragma unroll
+          for (int t = 1; t < 5; ++t) lo = lo + pw[t] * __shfl_sync(0xffffffffu, x, base + t);
+          finish(lo);
+          pup = k + 1 < len ? m : TF(0);   // row 7: its words are the coupling above
+#pragma unroll
+          for (int t = 0; t < 5; ++t) pw[t] = w[b][t];
+          pr = TF(dv[b]);
+          pupper = w[b][0];
+          ppiv = w[b][1];
+          pcell = cell[b];
+        }
+        if (k - D >= 0) fetch(k - D, b);
+      }
+    }
+    if (coupled) finish(TF(0));   // element 0 has nothing below
+  }
+  if (!coupled || !sa || ch >= nc) return;
+  // 3. coupled: the SA row forward, x_k = d_k - c_k x_{k-1}
+  {
+    const TF* plane = F + line_words(p) + ch;
+    const size_t pstride = (size_t)groups * LW_CHAINS;
+    constexpr int DS = 4;
+    TF x = TF(0), wc[DS];
+    double dv[DS];
+    int cell[DS];
+    auto fetch = [&](int k, int b) {
+      cell[b] = p.ch_cells[(size_t)ch * p.chain_L + k];
+      dv[b] = z[ro + cell[b]];
+      wc[b] = plane[(size_t)k * pstride];
+    };
+#pragma unroll
+    for (int b = 0; b < DS; ++b)
+      if (b < len) fetch(b, b);
+    for (int k0 = 0; k0 < len; k0 += DS)
+#pragma unroll
+      for (int b = 0; b < DS; ++b) {
+        const int k = k0 + b;
+        if (k >= len) break;
+        x = TF(dv[b]) - wc[b] * x;
+        z[ro + cell[b]] = double(x);
+        if (k + DS < len) fetch(k + DS, b);
+      }
   }
 }
 
@@ -42,33 +399,66 @@ void launch_wave_speeds3(const Plan3Dev& p, const double* U, double* lam, cudaSt
   k3_wave_speeds<<<(total + 127) / 128, 128, 0, st>>>(p, U, lam);
 }
 
-// the line_j factor at (U, cfl) into F: n_chains * chain_L * FACTOR3 words, FP32 where
-// p.line_fp32 (the mixed form), else FP64
-void launch_line_factor3(const Plan3Dev& p, const double* U, double cfl, void* F, cudaStream_t st) {
-  if (p.n_chains == 0) return;
-  counted3();
-  if (p.line_fp32)
-    k3_chain_factor<float><<<(p.n_chains + 63) / 64, 64, 0, st>>>(p, U, cfl, static_cast<float*>(F));
-  else
-    k3_chain_factor<double><<<(p.n_chains + 63) / 64, 64, 0, st>>>(p, U, cfl, static_cast<double*>(F));
+size_t line_factor_words3(const Plan3Dev& p) {
+  return line_words(p) + (size_t)p.chain_L * line_groups(p) * LW_CHAINS;
 }
 
-// z = M^-1 r from the factor F: r copied where no chain runs (ghosts and the canvas gaps)
-void launch_line_apply3(const Plan3Dev& p, const void* F, const double* r, double* z, cudaStream_t st) {
-  const int n = p.nvar * p.NI * p.NJ * p.NK;
-  counted3(p.n_chains > 0 ? 2 : 1);
-  k3_copy_rows<<<(n + 255) / 256, 256, 0, st>>>(n, r, z);
-  if (p.n_chains == 0) return;
-  if (p.line_fp32)
-    k3_chain_apply<float><<<(p.n_chains + 127) / 128, 128, 0, st>>>(p, static_cast<const float*>(F), r, z);
-  else
-    k3_chain_apply<double><<<(p.n_chains + 127) / 128, 128, 0, st>>>(p, static_cast<const double*>(F), r, z);
+template <class TF, bool SA>
+static void factor_chains(const Plan3Dev& p, const double* U, const double* lam, const double* m, const double* d,
+                          const double* dflow, const double* dsa, void* F, cudaStream_t st) {
+  k3_line_factor<TF, SA><<<(p.n_chains + 63) / 64, 64, 0, st>>>(p, U, lam, m, d, dflow, dsa, static_cast<TF*>(F));
+}
+
+// V/dt at (U, cfl) into vdt (may be null) and, where F is given, the line_j factor into F
+// (line_factor_words3 words, FP32 where p.line_fp32, else FP64).  The faces' and cells' terms
+// stay in p.face_buf between the launches (planes of all faces: lambda, the SA mass flux and
+// diffusion, then the cells' two diagonals), which the residual overwrites.
+void launch_line_factor3(const Plan3Dev& p, const double* U, double cfl, void* F, double* vdt, cudaStream_t st) {
+  const int nf = face_count(p, 0) + face_count(p, 1) + face_count(p, 2), n = p.NI * p.NJ * p.NK;
+  double *lam = p.face_buf, *m = lam + nf, *d = m + nf, *dflow = d + nf, *dsa = dflow + nf;
+  const bool sa = p.nvar > 5;
+  counted3(2);
+  if (sa) {
+    k3_line_faces<true><<<(nf + 127) / 128, 128, 0, st>>>(p, U, lam, m, d, nf);
+    k3_line_cells<true><<<(n + 127) / 128, 128, 0, st>>>(p, U, lam, m, d, cfl, dflow, dsa, vdt);
+  } else {
+    k3_line_faces<false><<<(nf + 127) / 128, 128, 0, st>>>(p, U, lam, m, d, nf);
+    k3_line_cells<false><<<(n + 127) / 128, 128, 0, st>>>(p, U, lam, m, d, cfl, dflow, dsa, vdt);
+  }
+  if (F == nullptr || p.n_chains == 0) return;
+  counted3();
+  if (p.line_fp32) {
+    if (sa) factor_chains<float, true>(p, U, lam, m, d, dflow, dsa, F, st);
+    else factor_chains<float, false>(p, U, lam, m, d, dflow, dsa, F, st);
+  } else {
+    if (sa) factor_chains<double, true>(p, U, lam, m, d, dflow, dsa, F, st);
+    else factor_chains<double, false>(p, U, lam, m, d, dflow, dsa, F, st);
+  }
+}
+
+// z = M^-1 (*scale r) from the factor F (scale null: 1), cells on no chain copied; vout (may
+// be null) receives *scale r
+void launch_line_apply3(const Plan3Dev& p, const void* F, const double* r, double* z, const double* scale, double* vout,
+                        cudaStream_t st) {
+  const int chains = (p.n_chains + LA_CHAINS - 1) / LA_CHAINS;
+  const int copies = (int)((size_t)p.n_offchain * p.nvar / 1024 + 1);
+  const unsigned grid = (unsigned)(chains + (copies < 1184 ? copies : 1184));
+  counted3();
+  if (p.line_fp32) {
+    const float* f = static_cast<const float*>(F);
+    if (p.nvar > 5) k3_line_apply<float, 6><<<grid, LA_THREADS, 0, st>>>(p, f, r, z, scale, vout, chains);
+    else k3_line_apply<float, 5><<<grid, LA_THREADS, 0, st>>>(p, f, r, z, scale, vout, chains);
+  } else {
+    const double* f = static_cast<const double*>(F);
+    if (p.nvar > 5) k3_line_apply<double, 6><<<grid, LA_THREADS, 0, st>>>(p, f, r, z, scale, vout, chains);
+    else k3_line_apply<double, 5><<<grid, LA_THREADS, 0, st>>>(p, f, r, z, scale, vout, chains);
+  }
 }
 
 void launch_precondition3(const Plan3Dev& p, const double* U, double cfl, const double* r, double* z, void* F,
                           cudaStream_t st) {
-  launch_line_factor3(p, U, cfl, F, st);
-  launch_line_apply3(p, F, r, z, st);
+  launch_line_factor3(p, U, cfl, F, nullptr, st);
+  launch_line_apply3(p, F, r, z, nullptr, nullptr, st);
 }
 
 }  // namespace jr

@@ -3,8 +3,9 @@
 // face_wave_speeds (src/jaxrans/numerics/residual.py:169-203) and line_j
 // (src/jaxrans/solvers/preconditioners.py:209-306) on a 3D plan -- 5x5 mean-flow chain
 // blocks, the SA row on its own scalar chains -- solved along each chain by the block
-// Thomas algorithm (src/jaxrans/core/linalg.py:80-132).  A first form: one thread walks
-// a chain, its blocks assembled as it goes, the eliminated blocks kept in scratch.
+// Thomas algorithm (src/jaxrans/core/linalg.py:80-132).  chain_factor_* and chain_apply_*
+// walk a chain as a whole, blocks assembled on the way (the form the host checks run); the
+// device's kernels split the same work (below).
 #pragma once
 #include "residual3d.cuh"
 
@@ -379,6 +380,143 @@ inline __host__ __device__ void chain_apply_sa(const Plan3Dev& p, int ch, const 
     nxt = (TF)z[(size_t)5 * n + c] - F[factor_at(p, ch, k, F3_SA + 2)] * nxt;
     z[(size_t)5 * n + c] = (double)nxt;
   }
+}
+
+// ---- the device's form: the same factor and solve split by what can run in parallel.
+// k3_line_faces makes each face's wave speed (and, SA, mass flux and diffusion) once instead
+// of once from either side and again for the link, k3_line_cells each cell's diagonals,
+// k3_line_factor the elimination down a chain, one thread a chain, and k3_line_apply the two
+// sweeps, eight lanes a chain.
+
+// prim_at with the variable count fixed at compile time (no local array)
+template <int NV>
+__host__ __device__ __forceinline__ void prim_at_n(const Plan3Dev& p, const double* U, int c, double q[NV3_MAX]) {
+  const int n = p.NI * p.NJ * p.NK;
+  double u[NV3_MAX];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) u[v] = U[(size_t)v * n + c];
+  to_prim3(u, q, NV, p.P.gamma);
+}
+
+// the line terms of face (a, i, j, k): lambda, and on the SA row the mass flux and diffusion
+template <bool SA>
+__host__ __device__ __forceinline__ void line_face_terms(const Plan3Dev& p, const double* U, int a, int i, int j, int k,
+                                                         double& lam, double& m, double& d) {
+  const Physics3& P = p.P;
+  const double g = P.gamma;
+  constexpr int NV = SA ? 6 : 5;
+  double ql[NV3_MAX], qh[NV3_MAX], qf[NV3_MAX], s[3];
+  const int lo = p.neighbours[cell_index(p, i - (a == 0), j - (a == 1), k - (a == 2))];
+  const int hi = p.neighbours[cell_index(p, i, j, k)];
+  prim_at_n<NV>(p, U, lo, ql);
+  prim_at_n<NV>(p, U, hi, qh);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) qf[v] = 0.5 * (ql[v] + qh[v]);
+  const double vol = 0.5 * (p.volume[lo] + p.volume[hi]);
+  face_vector(p, a, i, j, k, s);
+  const double ss = (s[0] * s[0] + s[1] * s[1]) + s[2] * s[2];
+  const double vn = (qf[1] * s[0] + qf[2] * s[1]) + qf[3] * s[2];
+  lam = (vn >= 0.0 ? vn : -vn) + sqrt(g * qf[4] / qf[0]) * sqrt(ss);
+  if (P.mu_inf > 0.0) {
+    const double mul = viscosity3(P, g * qf[4] / qf[0]);
+    double mu = mul;
+    if constexpr (SA) {
+      mu = mul + eddy_viscosity(P.sa, qf[0], qf[5] * P.mu_inf, mul / qf[0]);
+      m = qf[0] * vn;
+      d = diffusion_coefficient(P.sa, qf[0], qf[5] * P.mu_inf, mul) * ss / vol;
+    }
+    lam = lam + 2.0 * g / PR_LAMINAR * mu * ss / (qf[0] * vol);
+  }
+}
+
+// The diagonals of cell c from its faces' terms: the sum of lambda, and (SA) the SA chain's
+// diagonal (sa_diagonal)
+template <bool SA>
+__host__ __device__ __forceinline__ void line_cell_terms(const Plan3Dev& p, const double* U, const double* lam,
+                                                         const double* mflux, const double* dflux, double cfl, int c,
+                                                         double& sum, double& dsa) {
+  const int i = c / (p.NJ * p.NK), j = (c / p.NK) % p.NJ, k = c % p.NK;
+  int lo[3], hi[3];
+  sum = 0.0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lo[a] = face_flat(p, a, i, j, k);
+    hi[a] = face_flat(p, a, i + (a == 0), j + (a == 1), k + (a == 2));
+    sum = a == 0 ? lam[lo[a]] + lam[hi[a]] : sum + lam[lo[a]] + lam[hi[a]];
+  }
+  if constexpr (SA) {
+    const Physics3& P = p.P;
+    const double g = P.gamma, vol = p.volume[c];
+    double q[NV3_MAX], own[NV3_MAX], diag = 0.0, curl[3] = {0.0, 0.0, 0.0};
+    prim_at_n<6>(p, U, c, q);
+    prim_at_n<6>(p, U, p.neighbours[c], own);   // the cell as its faces' means take it
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double ml = mflux[lo[a]], mh = mflux[hi[a]];
+      const double out_hi = (mh > 0.0 ? mh : 0.0) + dflux[hi[a]], in_lo = (-ml > 0.0 ? -ml : 0.0) + dflux[lo[a]];
+      diag = a == 0 ? out_hi + in_lo : diag + out_hi + in_lo;
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {
+        const int o = side ? 1 : -1;
+        double qn[NV3_MAX], s[3], v[3];
+        prim_at_n<6>(p, U, p.neighbours[cell_index(p, i + (a == 0) * o, j + (a == 1) * o, k + (a == 2) * o)], qn);
+        face_vector(p, a, i + (a == 0) * side, j + (a == 1) * side, k + (a == 2) * side, s);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) v[m] = 0.5 * (own[1 + m] + qn[1 + m]) * o;
+        curl[0] += s[1] * v[2] - s[2] * v[1];
+        curl[1] += s[2] * v[0] - s[0] * v[2];
+        curl[2] += s[0] * v[1] - s[1] * v[0];
+      }
+    }
+    diag = diag / q[0];
+    const double sq = (curl[0] * curl[0] + curl[1] * curl[1]) + curl[2] * curl[2];
+    const double omega = sq > 0.0 ? sqrt(sq) / vol : 0.0;
+    const double nu = viscosity3(P, g * q[4] / q[0]) / q[0], dist = p.distance[c];
+    const double st = s_tilde(P.sa, omega, q[5] * P.mu_inf, nu, dist);
+    const double fw = f_w(P.sa, r_of(P.sa, q[5] * P.mu_inf, st, dist));
+    const double dest = q[5] > 0.0 ? 2.0 * P.sa.c_w1 * fw * P.mu_inf * q[5] / (dist * dist) : 0.0;
+    dsa = diag + dest * vol + sum / cfl;
+  }
+}
+
+// A = d(F . S)/dU (5x5, [row][variable]) of the conservative state whose primitives are q, in
+// closed form, then 1/2 A - 1/2 lam I (coupling5 without its dual-number columns)
+__host__ __device__ __forceinline__ void coupling5_closed(const double* q, double sx, double sy, double sz, double lam,
+                                                          double g, double B[5][5]) {
+  const double S[3] = {sx, sy, sz};
+  const double vn = (q[1] * sx + q[2] * sy) + q[3] * sz;
+  const double vv = (q[1] * q[1] + q[2] * q[2]) + q[3] * q[3];
+  const double phi = 0.5 * (g - 1.0) * vv, H = g / (g - 1.0) * q[4] / q[0] + 0.5 * vv;
+  B[0][0] = -0.5 * lam;
+  B[0][4] = 0.0;
+#pragma unroll
+  for (int b = 0; b < 3; ++b) {
+    B[0][1 + b] = 0.5 * S[b];
+    B[1 + b][0] = 0.5 * (phi * S[b] - q[1 + b] * vn);
+    B[1 + b][4] = 0.5 * ((g - 1.0) * S[b]);
+    B[4][1 + b] = 0.5 * (H * S[b] - (g - 1.0) * q[1 + b] * vn);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      B[1 + b][1 + d] = 0.5 * (q[1 + b] * S[d] - (g - 1.0) * q[1 + d] * S[b]) + (b == d ? 0.5 * (vn - lam) : 0.0);
+  }
+  B[4][0] = 0.5 * ((phi - H) * vn);
+  B[4][4] = 0.5 * (g * vn - lam);
+}
+
+// The factor's layout: four chains a group, eight rows a chain, fifteen words a row and
+// element: word w of row a of chain ch at element k is
+// F[((k * groups + ch / 4) * 15 + w) * 32 + (ch % 4) * 8 + a], so one word of a warp's 4 x 8
+// rows is one aligned segment.  Rows 0 to 4, the mean flow: words 0 to 4 the lower block's
+// row, 5 to 9 the inverse pivot's, 10 to 14 that of C = P upper.  Row 5, the SA chain: its
+// lower scalar, inverse pivot (words 0, 1) and c (word 10).  The coupled form solves the SA
+// chain from its far end down, beside the mean flow's way back: row 5 holds its upper scalar
+// and inverse pivot in words 10, 11 and c = pivot lower in a plane of its own after the
+// layout ([k * 4 groups + ch]); rows 6 and 7 hold in words 10 to 14 the SA row's coupling to
+// the mean flow below and above.
+constexpr int LW_WORDS = 15, LW_ROWS = 8, LW_CHAINS = 4;
+__host__ __device__ __forceinline__ int line_groups(const Plan3Dev& p) { return (p.n_chains + LW_CHAINS - 1) / LW_CHAINS; }
+__host__ __device__ __forceinline__ size_t line_words(const Plan3Dev& p) {
+  return (size_t)p.chain_L * line_groups(p) * LW_WORDS * LW_ROWS * LW_CHAINS;
 }
 
 }  // namespace jr

@@ -13,12 +13,6 @@ namespace jr {
 
 constexpr int RED3_BLOCKS = 296, RED3_THREADS = 256;
 
-__global__ void k3_vdt(Plan3Dev p, const double* __restrict__ U, double cfl, double* __restrict__ vdt) {
-  const int n = p.NI * p.NJ * p.NK;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-    vdt[c] = lambda_sum(p, U, c) / cfl;
-}
-
 __global__ void k3_vdt_add(size_t N, size_t n, const double* __restrict__ vdt, const double* __restrict__ z,
                            double* __restrict__ w) {
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x)
@@ -167,9 +161,7 @@ double DeviceOps3::host_sum(int count, int halves) {
 }
 
 void DeviceOps3::prepare(const double* U, double cfl) {
-  counted3();
-  k3_vdt<<<grid_of(n), 128, 0, st>>>(p, U, cfl, vdt);
-  if (line) launch_line_factor3(p, U, cfl, factor, st);
+  launch_line_factor3(p, U, cfl, line ? factor : nullptr, vdt, st);
   // the tangent map of this step's products; its canvas (A) is the residual's too, which
   // leaves the same values there
   if (lin_face != nullptr) launch_linearize3(p, U, static_cast<double*>(A), lin_face, lin_cell, st);
@@ -189,7 +181,7 @@ void DeviceOps3::matvec(const double* U, double, int src, int out) {
 
 // the factor of this step's (U, cfl), made in prepare
 void DeviceOps3::precondition(const double*, double, int src, int dst) {
-  launch_line_apply3(p, factor, v(src), v(dst), st);
+  launch_line_apply3(p, factor, v(src), v(dst), nullptr, nullptr, st);
 }
 
 void DeviceOps3::mdot(int count, int w, double* h) {
