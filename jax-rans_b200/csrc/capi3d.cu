@@ -30,7 +30,7 @@ struct jr_plan3d {
   double* loads = nullptr;     // 7 per wall face
   std::vector<double> wall_mid;
   double* work = nullptr;      // the Newton step's vectors
-  int* flag = nullptr;
+  Gmres3* scalars = nullptr;
   // the linearised J.v's buffers, made by the first Newton steps (a plan that only evaluates
   // residuals never pays for them)
   double *lin_face = nullptr, *lin_cell = nullptr, *lin_dq = nullptr;
@@ -309,13 +309,14 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   {
     const size_t words = DeviceOps3::work_doubles((size_t)d->nvar * n, n, d->krylov_subspace);
     void *w = nullptr, *f = nullptr;
-    if (cudaMalloc(&w, words * sizeof(double)) != cudaSuccess || (p->allocs.push_back(w), cudaMalloc(&f, sizeof(int))) != cudaSuccess) {
+    if (cudaMalloc(&w, words * sizeof(double)) != cudaSuccess || (p->allocs.push_back(w), cudaMalloc(&f, sizeof(Gmres3))) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
     p->allocs.push_back(f);
     p->work = static_cast<double*>(w);
-    p->flag = static_cast<int*>(f);
+    cudaMemset(f, 0, sizeof(Gmres3));
+    p->scalars = static_cast<Gmres3*>(f);
   }
   if (cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking) != cudaSuccess) {
     jr_plan3d_destroy(p);
@@ -379,7 +380,7 @@ int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, 
   ops.lin_face = plan->lin_face;
   ops.lin_cell = plan->lin_cell;
   ops.lin_dq = plan->lin_dq;
-  ops.bind(plan->work, plan->flag, plan->cfg.restart);
+  ops.bind(plan->work, plan->scalars, plan->cfg.restart);
   double c = *cfl, r = *residual_norm;
   for (int s = 0; s < n_steps; ++s) {
     const double norm = newton_step3_device(ops, U, c, r, plan->cfg);

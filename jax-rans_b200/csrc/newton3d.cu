@@ -1,8 +1,10 @@
 // The 3D Newton step on the device: newton3d.cuh's driver over kernel-backed vector
 // operations (the residual, J.v, wave speeds and line solve of residual3d.cu and
 // linesolve3d.cu; dot products by a fixed-order two-stage reduction, so a step is
-// bitwise reproducible).  The driver synchronises for the scalars it needs: each CGS2
-// pass's dots come back together (k3_mdot_partial), three reads per Arnoldi step.
+// bitwise reproducible).  The device has its own form of the driver's GMRES cycle: the
+// scalars of an Arnoldi step stay on the device (Gmres3), so its six kernels follow one
+// another without a word from the host, which reads H once a cycle for the least squares.
+#include <algorithm>
 #include <cstdio>
 
 #include "linesolve3d.cuh"
@@ -52,29 +54,235 @@ __global__ void k3_dot_partial(size_t N, const double* __restrict__ a, const dou
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
 }
 
-// the dots of basis vectors 0..count-1 with w in one launch: block (x, i) makes exactly
-// the partial sum k3_dot_partial makes for V_i . w
-__global__ void k3_mdot_partial(size_t N, const double* __restrict__ V, const double* __restrict__ w,
-                                double* __restrict__ partial) {
-  const double* a = V + (size_t)blockIdx.y * N;
-  double acc = 0.0;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x)
-    acc = acc + a[e] * w[e];
-  const double t = block_sum(acc);
-  if (threadIdx.x == 0) partial[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+// ---- CGS2 against the basis: three passes, each reading the basis once
+//   0: h1 = V^T w;  1: w -= V h1, then h2 = V^T w;  2: w -= V h2, then |w| and column j of H.
+// A thread holds its elements' entries of every vector in registers, so pass 1 updates w and
+// takes its dots from one read of the basis (the two as separate passes read it twice).  One
+// block of 256 threads an SM: NK entries of E elements (16-byte loads where N is even) and NK
+// sums fill the registers, and 32 x 16 bytes a thread are what the reads need in flight.  On
+// the 3.9M-cell wing (215 MB a vector) bound by HBM: pass 0 against 17 to 30 vectors reads
+// 6.8 TB/s, pass 1 4.9; a step's three passes over 30 vectors 1.9 ms on average where separate
+// dots (w read again for each vector) and updates took 2.8.  The sums are fixed by N alone.
+constexpr int ORTH_THREADS = 256, ORTH_BLOCKS = 148, ORTH_NK = 32;
+
+// The NK sums of every lane over the warp, by a butterfly that halves the sums a lane holds at
+// each exchange: afterwards lane l holds sum l * NK / 32 (NK < 32: every 32 / NK-th lane's) in
+// acc[0].
+template <int NK>
+__device__ __forceinline__ void lane_sums(double (&acc)[NK], int lane) {
+  int held = NK;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    if (held >= 2) {
+      const int half = held / 2;
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int k = 0; k < NK / 2; ++k)
+        if (k < half) {
+          const double send = upper ? acc[k] : acc[k + half], keep = upper ? acc[k + half] : acc[k];
+          acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      held = half;
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+    }
+  }
+}
+
+template <int E> struct Elems {
+  double x[E];
+};
+template <int E> __device__ __forceinline__ Elems<E> load_elems(const double* p) {
+  Elems<E> r;
+  if constexpr (E == 2) {
+    const double2 t = *reinterpret_cast<const double2*>(p);
+    r.x[0] = t.x;
+    r.x[1] = t.y;
+  } else {
+    r.x[0] = *p;
+  }
+  return r;
+}
+template <int E> __device__ __forceinline__ void store_elems(double* p, const Elems<E>& v) {
+  if constexpr (E == 2) *reinterpret_cast<double2*>(p) = make_double2(v.x[0], v.x[1]);
+  else *p = v.x[0];
+}
+
+// sums[NK] of every thread: over the block into partial, and by the last block over the
+// blocks in order; true there, with the totals in total[NK]
+template <int NK>
+__device__ bool finish_sums(double (&sums)[NK], double* partial, unsigned* ticket, double* total) {
+  __shared__ double warps[ORTH_THREADS / 32][NK];
+  __shared__ double groups[ORTH_THREADS];
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  lane_sums<NK>(sums, lane);
+  if (lane % (32 / NK) == 0) warps[warp][lane / (32 / NK)] = sums[0];
+  __syncthreads();
+  if (t < NK) {
+    double s = warps[0][t];
+    for (int w = 1; w < ORTH_THREADS / 32; ++w) s += warps[w][t];
+    partial[(size_t)blockIdx.x * NK + t] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  constexpr int G = ORTH_THREADS / NK;
+  const int k = t % NK, g = t / NK, nb = gridDim.x;
+  double s = 0.0;
+  for (int b = g; b < nb; b += 8 * G) {
+    double x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = b + u * G < nb ? __ldcg(partial + (size_t)(b + u * G) * NK + k) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += x[u];
+  }
+  groups[t] = s;
+  __syncthreads();
+  if (t < NK) {
+    double v = groups[t];
+    for (int q = 1; q < G; ++q) v += groups[q * NK + t];
+    total[t] = v;
+  }
+  if (t == 0) *ticket = 0u;
+  __syncthreads();
+  return true;
+}
+
+// The dots of vectors k0 .. k0 + nk - 1 (nk <= NK) with w, after (UPDATE) w -= sum h V over
+// the same vectors; hin, hout: the scalars of vector k0.
+template <int NK, int E, bool UPDATE>
+__global__ void __launch_bounds__(ORTH_THREADS, 1) k3_orth_dots(size_t N, int nk, const double* __restrict__ V,
+                                                                double* __restrict__ w,
+                                                                const double* __restrict__ hin, double* hout,
+                                                                double* partial, unsigned* ticket) {
+  __shared__ double h[NK], total[NK];
+  if (UPDATE) {
+    if ((int)threadIdx.x < NK) h[threadIdx.x] = (int)threadIdx.x < nk ? hin[threadIdx.x] : 0.0;
+    __syncthreads();
+  }
+  double acc[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) acc[k] = 0.0;
+  const size_t step = (size_t)gridDim.x * ORTH_THREADS * E;
+  for (size_t e = ((size_t)blockIdx.x * ORTH_THREADS + threadIdx.x) * E; e < N; e += step) {
+    Elems<E> we = load_elems<E>(w + e), v[NK];
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk) v[k] = load_elems<E>(V + (size_t)k * N + e);
+    if (UPDATE) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < NK; ++k)
+          if (k < nk) s += h[k] * v[k].x[i];
+        we.x[i] -= s;
+      }
+      store_elems<E>(w + e, we);
+    }
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk)
+#pragma unroll
+        for (int i = 0; i < E; ++i) acc[k] += v[k].x[i] * we.x[i];
+  }
+  if (finish_sums<NK>(acc, partial, ticket, total) && (int)threadIdx.x < nk) hout[threadIdx.x] = total[threadIdx.x];
+}
+
+// w -= sum h V over all nk vectors, and with `column` |w| and column j of H (m + 1 rows,
+// row-major H[i * m + j])
+template <int E>
+__global__ void __launch_bounds__(ORTH_THREADS) k3_orth_update(size_t N, int nk, const double* __restrict__ V,
+                                                               double* __restrict__ w, const double* __restrict__ hin,
+                                                               Gmres3* g, int j, int m, int column, double* partial) {
+  __shared__ double h[MAX_RESTART3 + 1], total[8];
+  if ((int)threadIdx.x < nk) h[threadIdx.x] = hin[threadIdx.x];
+  __syncthreads();
+  double acc[8] = {};
+  const size_t step = (size_t)gridDim.x * ORTH_THREADS * E;
+  for (size_t e = ((size_t)blockIdx.x * ORTH_THREADS + threadIdx.x) * E; e < N; e += step) {
+    Elems<E> we = load_elems<E>(w + e);
+    double s[E] = {};
+    for (int k0 = 0; k0 < nk; k0 += 16) {
+      Elems<E> v[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        if (k0 + k < nk) v[k] = load_elems<E>(V + (size_t)(k0 + k) * N + e);
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        if (k0 + k < nk)
+#pragma unroll
+          for (int i = 0; i < E; ++i) s[i] += h[k0 + k] * v[k].x[i];
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      we.x[i] -= s[i];
+      acc[0] += we.x[i] * we.x[i];
+    }
+    store_elems<E>(w + e, we);
+  }
+  if (!column || !finish_sums<8>(acc, partial, &g->ticket, total)) return;
+  const double nrm = sqrt(total[0]);
+  for (int i = threadIdx.x; i < nk; i += ORTH_THREADS) g->H[i * m + j] = g->h1[i] + g->h2[i];
+  if (threadIdx.x == 0) {
+    g->H[(j + 1) * m + j] = nrm;
+    g->inv = 1.0 / fmax(nrm, 2.2250738585072014e-308);
+  }
+}
+
+__global__ void k3_cycle_begin(Gmres3* g, double inv, int m) {
+  for (int e = threadIdx.x; e < (m + 1) * m; e += blockDim.x) g->H[e] = 0.0;
+  if (threadIdx.x == 0) g->inv = inv;
 }
 
 struct Coeffs3 {
-  double c[MAX_RESTART3 + 1];
+  double y[MAX_RESTART3], hy[MAX_RESTART3 + 1];
 };
 
-// y += c_0 V_0 + c_1 V_1 + ... + c_{count-1} V_{count-1}, term by term in that order (the
-// arithmetic of count axpys, in one pass)
-__global__ void k3_maxpy(size_t N, int count, Coeffs3 cf, const double* __restrict__ V, double* __restrict__ y) {
+// The end of a cycle: t = sum y V, action += sum (H y) V, V_m = w / |w| (one read of the basis)
+__global__ void __launch_bounds__(256) k3_combine(size_t N, int m, Coeffs3 cf, const double* __restrict__ V,
+                                                  const double* __restrict__ w, const Gmres3* __restrict__ g,
+                                                  double* __restrict__ t, double* __restrict__ action) {
+  const double inv = g->inv;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x) {
-    double acc = y[e];
-    for (int i = 0; i < count; ++i) acc = acc + cf.c[i] * V[(size_t)i * N + e];
-    y[e] = acc;
+    double s = 0.0, a = action[e];
+    for (int k0 = 0; k0 < m; k0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = k0 + k < m ? V[(size_t)(k0 + k) * N + e] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < m) {
+          s += cf.y[k0 + k] * v[k];
+          a += cf.hy[k0 + k] * v[k];
+        }
+    }
+    t[e] = s;
+    action[e] = a + cf.hy[m] * (inv * w[e]);
+  }
+}
+
+// x += z; r = b - action
+__global__ void k3_cycle_end(size_t N, const double* __restrict__ z, const double* __restrict__ b,
+                             const double* __restrict__ action, double* __restrict__ x, double* __restrict__ r) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x) {
+    x[e] += z[e];
+    r[e] = b[e] - action[e];
+  }
+}
+
+// z = v = *scale src: the Arnoldi vector without a preconditioner
+__global__ void k3_scale_copy(size_t N, const double* __restrict__ scale, const double* __restrict__ src,
+                              double* __restrict__ v, double* __restrict__ z) {
+  const double s = *scale;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < N; e += (size_t)gridDim.x * blockDim.x) {
+    const double x = s * src[e];
+    v[e] = x;
+    z[e] = x;
   }
 }
 
@@ -184,24 +392,94 @@ void DeviceOps3::precondition(const double*, double, int src, int dst) {
   launch_line_apply3(p, factor, v(src), v(dst), nullptr, nullptr, st);
 }
 
-void DeviceOps3::mdot(int count, int w, double* h) {
+template <int NK, int E>
+static void orth_dots(DeviceOps3& o, bool update, int blocks, int nk, const double* V, double* w, const double* hin,
+                      double* hout) {
   counted3();
-  k3_mdot_partial<<<dim3(RED3_BLOCKS, count), RED3_THREADS, 0, st>>>(N, v(V(0)), v(w), partial);
-  std::vector<double> part((size_t)count * RED3_BLOCKS);
-  cudaMemcpyAsync(part.data(), partial, part.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
-  cudaStreamSynchronize(st);
-  for (int i = 0; i < count; ++i) {
-    double s = 0.0;
-    for (int b = 0; b < RED3_BLOCKS; ++b) s = s + part[(size_t)i * RED3_BLOCKS + b];
-    h[i] = s;
-  }
+  if (update)
+    k3_orth_dots<NK, E, true><<<blocks, ORTH_THREADS, 0, o.st>>>(o.N, nk, V, w, hin, hout, o.partial, &o.gm->ticket);
+  else
+    k3_orth_dots<NK, E, false><<<blocks, ORTH_THREADS, 0, o.st>>>(o.N, nk, V, w, hin, hout, o.partial, &o.gm->ticket);
 }
 
-void DeviceOps3::maxpy(int count, const double* coef, int y) {
-  Coeffs3 cf{};
-  for (int i = 0; i < count; ++i) cf.c[i] = coef[i];
-  counted3();
-  k3_maxpy<<<grid_of(N), 256, 0, st>>>(N, count, cf, v(V(0)), v(y));
+// orthogonalise W_ against V(0) .. V(j) and make column j of H
+template <int E> static void orthogonalise(DeviceOps3& o, int j, int m) {
+  const int nk = j + 1;
+  const size_t per = (size_t)ORTH_THREADS * E;
+  const int blocks = (int)std::min<size_t>(ORTH_BLOCKS, (o.N + per - 1) / per);
+  const double* V = o.v(o.V(0));
+  double* w = o.v(DeviceOps3::W_);
+  Gmres3* g = o.gm;
+  auto dots = [&](bool update, int k0, int count, const double* hin, double* hout) {
+    const double* Vk = V + (size_t)k0 * o.N;
+    // (few vectors: registers for two blocks an SM, which the reads in flight then need)
+    if (count <= 8) orth_dots<8, E>(o, update, blocks * 2, count, Vk, w, hin, hout + k0);
+    else if (count <= 16) orth_dots<16, E>(o, update, blocks, count, Vk, w, hin, hout + k0);
+    else orth_dots<ORTH_NK, E>(o, update, blocks, count, Vk, w, hin, hout + k0);
+  };
+  auto update = [&](const double* h, int column) {
+    counted3();
+    k3_orth_update<E><<<blocks * 2, ORTH_THREADS, 0, o.st>>>(o.N, nk, V, w, h, g, j, m, column, o.partial);
+  };
+  for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(false, k0, std::min(ORTH_NK, nk - k0), nullptr, g->h1);
+  if (nk <= ORTH_NK) {
+    dots(true, 0, nk, g->h1, g->h2);
+  } else {   // more vectors than a thread holds: the update, then the dots in slices
+    update(g->h1, 0);
+    for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(false, k0, std::min(ORTH_NK, nk - k0), nullptr, g->h2);
+  }
+  update(g->h2, 1);
+}
+
+// gmres3 (newton3d.cuh) with an Arnoldi step's scalars on the device
+int gmres3(DeviceOps3& ops, const double* U, double cfl, const Newton3Config& c, int B, int X, int ACTION) {
+  const double tiny = 2.2250738585072014e-308;
+  const double rcond = 2.220446049250313e-16 * (c.restart + 1);
+  const int m = c.restart, grid = grid_of(ops.N);
+  const size_t N = ops.N;
+  const double bn = ops.nrm2(B);
+  ops.zero(X);
+  ops.copy(B, DeviceOps3::R_);
+  ops.zero(ACTION);
+  std::vector<double> H((size_t)(m + 1) * m), y;
+  for (int k = 0; k < c.maxiter; ++k) {
+    const double beta = k == 0 ? bn : ops.nrm2(DeviceOps3::R_);
+    if (!(beta > c.tol * bn)) break;
+    counted3();
+    k3_cycle_begin<<<1, 256, 0, ops.st>>>(ops.gm, 1.0 / std::fmax(beta, tiny), m);
+    for (int j = 0; j < m; ++j) {
+      const double* src = ops.v(j == 0 ? DeviceOps3::R_ : DeviceOps3::W_);
+      double *z = ops.v(DeviceOps3::Z_), *vj = ops.v(ops.V(j));
+      if (c.preconditioner >= 1) {
+        launch_line_apply3(ops.p, ops.factor, src, z, &ops.gm->inv, vj, ops.st);
+      } else {
+        counted3();
+        k3_scale_copy<<<grid, 256, 0, ops.st>>>(N, &ops.gm->inv, src, vj, z);
+      }
+      ops.matvec(U, cfl, DeviceOps3::Z_, DeviceOps3::W_);
+      if (N % 2 == 0) orthogonalise<2>(ops, j, m);
+      else orthogonalise<1>(ops, j, m);
+    }
+    cudaMemcpyAsync(H.data(), ops.gm->H, H.size() * sizeof(double), cudaMemcpyDeviceToHost, ops.st);
+    cudaStreamSynchronize(ops.st);
+    givens_lstsq(H, m, beta, rcond, y);
+    Coeffs3 cf{};
+    for (int i = 0; i <= m; ++i) {
+      double s = 0.0;
+      for (int j = 0; j < m; ++j) s = s + H[(size_t)i * m + j] * y[j];
+      cf.hy[i] = s;
+      if (i < m) cf.y[i] = y[i];
+    }
+    counted3();
+    k3_combine<<<grid, 256, 0, ops.st>>>(N, m, cf, ops.v(ops.V(0)), ops.v(DeviceOps3::W_), ops.gm,
+                                         ops.v(DeviceOps3::T_), ops.v(ACTION));
+    if (c.preconditioner >= 1) ops.precondition(U, cfl, DeviceOps3::T_, DeviceOps3::Z_);
+    else ops.copy(DeviceOps3::T_, DeviceOps3::Z_);
+    counted3();
+    k3_cycle_end<<<grid, 256, 0, ops.st>>>(N, ops.v(DeviceOps3::Z_), ops.v(B), ops.v(ACTION), ops.v(X),
+                                           ops.v(DeviceOps3::R_));
+  }
+  return 0;
 }
 
 double DeviceOps3::dot(int a, int b) {
@@ -255,14 +533,16 @@ void DeviceOps3::add_to_state(double* U, int du) {
 }
 
 size_t DeviceOps3::work_doubles(size_t N, size_t n, int m) {
-  return (size_t)(BASE + m + 1) * N + n + (size_t)(m + 1) * RED3_BLOCKS;
+  // the vectors, V/dt and the reductions' partial sums (and room to keep each 16-byte aligned)
+  return (size_t)(BASE + m + 1) * N + n + 2 + std::max<size_t>((size_t)2 * RED3_BLOCKS, (size_t)4 * ORTH_BLOCKS * ORTH_NK);
 }
 
-void DeviceOps3::bind(double* work, int* flag_word, int m) {
+void DeviceOps3::bind(double* work, Gmres3* scalars, int m) {
   vecs = work;
   vdt = work + (size_t)(BASE + m + 1) * N;
   partial = vdt + n;
-  flag = flag_word;
+  gm = scalars;
+  flag = &scalars->flag;
 }
 
 double newton_step3_device(DeviceOps3& ops, double* U, double& cfl, double& res_prev, const Newton3Config& c) {

@@ -8,6 +8,15 @@
 
 namespace jr {
 
+// The scalars a GMRES cycle keeps on the device: the dots of the two orthogonalisations, the
+// Hessenberg matrix (row-major, m + 1 rows of m), 1 / |w|, the reductions' ticket (0 between
+// kernels) and the physicality flag.
+struct Gmres3 {
+  double h1[MAX_RESTART3 + 1], h2[MAX_RESTART3 + 1], H[(MAX_RESTART3 + 1) * MAX_RESTART3], inv;
+  unsigned ticket;
+  int flag;
+};
+
 struct DeviceOps3 {
   enum { R_ = 0, Z_, W_, T_, RES_, B_, DU_, ACT_, BASE };
   Plan3Dev p;
@@ -21,6 +30,7 @@ struct DeviceOps3 {
   double* vecs = nullptr;
   double* vdt = nullptr;
   double* partial = nullptr;
+  Gmres3* gm = nullptr;
   int* flag = nullptr;
   double last_second = 0.0;
   cudaStream_t st = nullptr;
@@ -33,8 +43,6 @@ struct DeviceOps3 {
   void matvec(const double* U, double cfl, int src, int out);
   void precondition(const double* U, double cfl, int src, int dst);
   double dot(int a, int b);
-  void mdot(int count, int w, double* h);                 // h[i] = V(i) . w, i < count
-  void maxpy(int count, const double* coef, int y);       // y += sum_i coef[i] V(i), in order
   double nrm2(int a) { return sqrt(dot(a, a)); }
   void axpy(double al, int x, int y);
   void scale(double al, int x, int y);
@@ -45,8 +53,11 @@ struct DeviceOps3 {
   bool physical_after(const double* U, int du);
   void add_to_state(double* U, int du);
   static size_t work_doubles(size_t N, size_t n, int m);
-  void bind(double* work, int* flag_word, int m);
+  void bind(double* work, Gmres3* scalars, int m);
 };
+
+// the cycles of gmres3 (newton3d.cuh) on the device's scalars; newton_step3 takes this overload
+int gmres3(DeviceOps3& ops, const double* U, double cfl, const Newton3Config& c, int B, int X, int ACTION);
 
 double newton_step3_device(DeviceOps3& ops, double* U, double& cfl, double& res_prev, const Newton3Config& c);
 
