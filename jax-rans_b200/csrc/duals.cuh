@@ -26,7 +26,6 @@ template <int N> JR_HD Duals<N> duals_cst(double x) {
 template <> JR_HD Duals<2> cst<Duals<2>>(double x) { return duals_cst<2>(x); }
 template <> JR_HD Duals<3> cst<Duals<3>>(double x) { return duals_cst<3>(x); }
 template <> JR_HD Duals<4> cst<Duals<4>>(double x) { return duals_cst<4>(x); }
-template <> JR_HD Duals<5> cst<Duals<5>>(double x) { return duals_cst<5>(x); }
 
 // r.v = VALUE, r.d[k] = TANGENT for every k
 #define JR_DUALS(VALUE, TANGENT)          \

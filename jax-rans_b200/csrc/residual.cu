@@ -9,6 +9,7 @@
 // faces of each cell -- a per-cell reduction with no atomics.  The same source gives
 // R(U) (T = double) and dR1/dU . v (T = Dual, first-order faces).
 #include "device.cuh"
+#include "duals.cuh"
 
 namespace jr {
 
@@ -450,6 +451,58 @@ __device__ __forceinline__ void viscous_tail(const Physics& P, const T* x, doubl
   }
 }
 
+// The derivatives of viscous_tail's outputs without QCR2000, put(r, k, d out[r] / d x[k]) for
+// every (r, k) a dependence allows: the stress is linear in the velocity gradients and the
+// viscosity, so only the viscosities' own derivatives (one in the laminar face temperature,
+// three in the face rho, p, nu_hat) are evaluated as tangents.
+template <int VISC, class PUT>
+__device__ __forceinline__ void viscous_derivatives(const Physics& P, const double* x, double sx, double sy, PUT put) {
+  const double g = P.gamma, kl = 1.0 / (PR_LAM * (g - 1.0)), kt = 1.0 / (PR_TURB * (g - 1.0));
+  const Dual mul = viscosity(P, Dual{x[8], 1.0});
+  double mu = mul.v, k = mul.v / (PR_LAM * (g - 1.0));
+  using D = Duals<3>;   // with respect to the face rho, p, nu_hat
+  D mut = cst<D>(0.0), coef = cst<D>(0.0);
+  if constexpr (VISC == 2) {
+    const D rho{x[11], {1.0, 0.0, 0.0}}, p{x[12], {0.0, 1.0, 0.0}}, nuh{x[13], {0.0, 0.0, 1.0}};
+    const D muf = viscosity(P, g * p / rho);
+    mut = eddy_viscosity(P.sa, rho, nuh * P.mu_inf, muf / rho);
+    coef = diffusion_coefficient(P.sa, rho, nuh * P.mu_inf, muf);
+    mu = mu + mut.v;
+    k = k + mut.v / (PR_TURB * (g - 1.0));
+  }
+  const double ttd = (2.0 / 3.0) * (x[0] + x[3]), shear = x[1] + x[2];
+  const double lx = (2.0 * x[0] - ttd) * sx + shear * sy, ly = shear * sx + (2.0 * x[3] - ttd) * sy;
+  const double gts = x[4] * sx + x[5] * sy;
+  const double third = mu * (4.0 / 3.0), two = mu * (2.0 / 3.0);
+  const double dx[4] = {third * sx, mu * sy, mu * sy, -two * sx}, dy[4] = {-two * sy, mu * sx, mu * sx, third * sy};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    put(0, e, dx[e]);
+    put(1, e, dy[e]);
+    put(2, e, x[6] * dx[e] + x[7] * dy[e]);
+  }
+  put(2, 4, k * sx);
+  put(2, 5, k * sy);
+  put(2, 6, mu * lx);
+  put(2, 7, mu * ly);
+  const double work = x[6] * lx + x[7] * ly;   // per unit viscosity
+  put(0, 8, mul.d * lx);
+  put(1, 8, mul.d * ly);
+  put(2, 8, mul.d * (work + kl * gts));
+  if constexpr (VISC == 2) {
+    const double gn = x[9] * sx + x[10] * sy;
+    put(3, 9, coef.v * sx);
+    put(3, 10, coef.v * sy);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+      put(0, 11 + t, mut.d[t] * lx);
+      put(1, 11 + t, mut.d[t] * ly);
+      put(2, 11 + t, mut.d[t] * (work + kt * gts));
+      put(3, 11 + t, coef.d[t] * gn);
+    }
+  }
+}
+
 // The SA source of one cell times nothing (the caller multiplies by the volume):
 // y = (rho, p, nu_hat, dv/dx, du/dy, dnu_hat/dx, dnu_hat/dy), the gradients by
 // Green-Gauss over face-averaged values (turbulence.py:93-103,138-151).
@@ -679,6 +732,10 @@ int jac_coefficients(int visc) {
 }
 int jac_cell_coefficients(int visc) { return visc == 2 ? JCELL : 0; }
 
+// Columns of the inviscid flux's Jacobian per evaluation (Duals): the flux's divisions and
+// roots are shared by the columns of one evaluation.
+constexpr int LIN_COLUMNS = 4;
+
 // Coefficients of one face at flat face index f (i-faces first, then j-faces); the face
 // lies between staged cells (ai, aj) and the next along `axis` of a double tile.
 template <int NV, int VISC, class TJ>
@@ -695,18 +752,27 @@ __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double
     qb[v] = s.q[v][bi][bj];
   }
   double mass = 0.0;
+  using D = Duals<LIN_COLUMNS>;
 #pragma unroll 1
-  for (int seed = 0; seed < 8; ++seed) {
-    Dual qL[4], qR[4], F[4];
+  for (int s0 = 0; s0 < 8; s0 += LIN_COLUMNS) {
+    D qL[4], qR[4], F[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      qL[v] = Dual{qa[v], seed == v ? 1.0 : 0.0};
-      qR[v] = Dual{qb[v], seed == 4 + v ? 1.0 : 0.0};
+      qL[v].v = qa[v];
+      qR[v].v = qb[v];
+#pragma unroll
+      for (int t = 0; t < LIN_COLUMNS; ++t) {
+        qL[v].d[t] = s0 + t == v ? 1.0 : 0.0;
+        qR[v].d[t] = s0 + t == 4 + v ? 1.0 : 0.0;
+      }
     }
     riemann(P.flux, qL, qR, sx, sy, g, F);
-    const int base = seed < 4 ? seed : 12 + seed;   // AL[r][v] at r * 4 + v, AR[r][v] at 16 + r * 4 + v
 #pragma unroll
-    for (int r = 0; r < 4; ++r) jac[(size_t)(base + 4 * r) * stride + f] = TJ(F[r].d);
+    for (int t = 0; t < LIN_COLUMNS; ++t) {
+      const int seed = s0 + t, base = seed < 4 ? seed : 12 + seed;   // AL[r][v] at r * 4 + v, AR[r][v] at 16 + r * 4 + v
+#pragma unroll
+      for (int r = 0; r < 4; ++r) jac[(size_t)(base + 4 * r) * stride + f] = TJ(F[r].d[t]);
+    }
     mass = F[0].v;
   }
   if constexpr (VISC == 2) {
@@ -728,23 +794,32 @@ __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double
     double x[NX];
     face_intermediates<double, VISC>(q, phi, cxv, cyv, axis, ai, aj, x);
     using S = ViscShape<VISC>;
+    if (VISC < 2 || P.c_cr1 == 0.0) {
+      viscous_derivatives<VISC>(P, x, sx, sy, [&](int r, int k, double d) {
+        jac[(size_t)(J::VBASE + S::slot(r, k)) * stride + f] = TJ(d);
+      });
+    } else {   // QCR2000's stress: one evaluation a direction
 #pragma unroll 1
-    for (int k = 0; k < NX; ++k) {
-      Dual xd[NX], out[NR];
+      for (int k = 0; k < NX; ++k) {
+        Dual xd[NX], out[NR];
 #pragma unroll
-      for (int m = 0; m < NX; ++m) xd[m] = Dual{x[m], m == k ? 1.0 : 0.0};
-      viscous_tail<Dual, VISC>(P, xd, sx, sy, out);
+        for (int m = 0; m < NX; ++m) xd[m] = Dual{x[m], m == k ? 1.0 : 0.0};
+        viscous_tail<Dual, VISC>(P, xd, sx, sy, out);
 #pragma unroll
-      for (int r = 0; r < NR; ++r)
-        if ((S::depends(r) >> k) & 1u) jac[(size_t)(J::VBASE + S::slot(r, k)) * stride + f] = TJ(out[r].d);
+        for (int r = 0; r < NR; ++r)
+          if ((S::depends(r) >> k) & 1u) jac[(size_t)(J::VBASE + S::slot(r, k)) * stride + f] = TJ(out[r].d);
+      }
     }
   }
 }
 
-// Three CTAs per SM (at most 168 registers, some spilled to local memory): a single
-// 385 x 97 case's tiles then run in one wave instead of two; measured 262 against 368 us.
+// Bound by FP64 issue.  Four columns of the flux an evaluation and two CTAs an SM (255
+// registers, some spilled): 79 us on a 385 x 97 SA case, 537 us on nine cases' 442k cells in
+// the mixed form, 31 us on a 257 x 65 Euler case, ghost maps included (one column and one
+// direction of the viscous terms at a time: 209, 2329 and 75 us; two columns and three CTAs:
+// 71, 640 and 39 us).
 template <int NV, int VISC, class TJ>
-__global__ void __launch_bounds__(TILE_THREADS, 3) k_linearize(const CaseDev* __restrict__ cases) {
+__global__ void __launch_bounds__(TILE_THREADS, 2) k_linearize(const CaseDev* __restrict__ cases) {
   __shared__ CaseDev scase;
   if (idle_block(cases[blockIdx.z],
                  (int)blockIdx.x >= cases[blockIdx.z].tiles_x || (int)blockIdx.y >= cases[blockIdx.z].tiles_y, 0))
@@ -825,13 +900,20 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) k_linearize(const CaseDev* __
         const double y[JCELL] = {s.q[0][si][sj], s.q[3][si][sj], s.q[NV == 5 ? 4 : 0][si][sj], gg[0][1], gg[1][0],
                                  gg[0][2], gg[1][2]};
         const double d = c.distance[idx];
-#pragma unroll 1
-        for (int k = 0; k < JCELL; ++k) {
-          Dual yd[JCELL];
+        // the source's tangents in rho, p, nu_hat and |vorticity|; the gradient term's by hand
+        using D = Duals<4>;
+        const D rho{y[0], {1.0, 0.0, 0.0, 0.0}}, p{y[1], {0.0, 1.0, 0.0, 0.0}}, nuh{y[2], {0.0, 0.0, 1.0, 0.0}};
+        const double vort = y[3] - y[4], side = vort >= 0.0 ? 1.0 : -1.0;
+        const D omega{side * vort, {0.0, 0.0, 0.0, 1.0}};
+        const D mu = viscosity(P, P.gamma * p / rho);
+        D Pr, De;
+        sa_source(P.sa, nuh * P.mu_inf, mu / rho, omega, d, Pr, De);
+        const double cb = P.sa.c_b2 / P.sa.sigma * P.mu_inf;
+        const D src = rho * ((Pr - De) / P.mu_inf + cb * (y[5] * y[5] + y[6] * y[6]));
+        const double out[JCELL] = {src.d[0], src.d[1], src.d[2], side * src.d[3], -side * src.d[3],
+                                   2.0 * y[0] * cb * y[5], 2.0 * y[0] * cb * y[6]};
 #pragma unroll
-          for (int m = 0; m < JCELL; ++m) yd[m] = Dual{y[m], m == k ? 1.0 : 0.0};
-          jcell[(size_t)k * N + idx] = sa_cell_source(P, yd, d).d;
-        }
+        for (int k = 0; k < JCELL; ++k) jcell[(size_t)k * N + idx] = out[k];
       }
     }
   }
