@@ -188,7 +188,7 @@ struct BatchDims {
   int n_vec;                // nvar * cells
   int chain_blocks;         // chains + off-chain blocks of the line solve
   int max_L;                // longest chain
-  int cgs_blocks;           // blocks of the basis passes
+  int cgs_blocks;           // blocks of the FP32 basis passes
   int ls_factor_threads;    // threads per chain of the line factor and of the line solve:
   int ls_apply_threads;     // the schedule the plan's autotuner picked (results do not depend on it)
   int ls_apply_stage;       // s >= 1: the line solve stages its factor from level s-1 of the longest chain
@@ -197,7 +197,7 @@ struct BatchDims {
 constexpr int LS_MAX_THREADS = 256;   // the largest line-solve block
 constexpr int APPLY_STAGES = 4;       // staged line-solve forms 1..4 (0: the factor read from global memory)
 
-// The basis passes: a block owns a chunk of cgs_chunk(n) elements of a case of n, set by
+// The FP32 basis passes: a block owns a chunk of cgs_chunk(n) elements of a case of n, set by
 // the case's size alone (so its sums are the same in any batch): small cases (a 385 x 97
 // SA case: 194k unknowns, 380 blocks) take short chunks to keep more blocks per SM,
 // large ones longer chunks.
@@ -206,6 +206,13 @@ __host__ __device__ __forceinline__ int cgs_chunk(int n) {
   return n >= 2 * 148 * 2048 ? 2048 : (n >= 2 * 148 * 1024 ? 1024 : 512);
 }
 __host__ __device__ __forceinline__ int cgs_blocks(int n) { return (n + cgs_chunk(n) - 1) / cgs_chunk(n); }
+
+// The FP64 basis passes: blocks of a case of n unknowns, set by its size alone (so its sums are the
+// same in any batch): one an SM, fewer where that leaves a thread without an element.
+__host__ __device__ __forceinline__ int orth_blocks(int n) {
+  const int b = (n + 255) / 256;
+  return b < 1 ? 1 : (b > 148 ? 148 : b);
+}
 
 // the number of blocks a per-case reduction over n elements uses (<= the grid's x)
 __host__ __device__ __forceinline__ int chunk_blocks(int n) {

@@ -3,12 +3,13 @@
 //
 // Every cycle runs with a fixed launch sequence (so a Newton step can be captured in
 // one CUDA graph): the kernels of a cycle read the case's `active` flag and return at
-// once when the restart loop has already stopped.  CGS2 is three passes over the basis:
+// once when the restart loop has already stopped.  CGS2 is three reads of the basis:
 // the dots; the first update fused with the second dots; the second update fused with
 // the norm.  Reductions are per-block partial sums finished by the last block in a fixed
 // order, so a rerun gives bitwise the same scalars.  TV is the basis type (double;
 // float in the mixed form, with FP64 accumulation).
 #include "device.cuh"
+#include "orth.cuh"
 
 namespace jr {
 
@@ -96,33 +97,6 @@ __device__ bool reduce_last(double (&vals)[W], double* partial, unsigned* ticket
   return true;
 }
 
-// The NK accumulators of every lane summed over the warp by a butterfly that halves the
-// values a lane holds at each of the five exchanges: at the end lane l holds the sums of
-// accumulators l*(NK/32) .. l*(NK/32) + NK/32 - 1 (NK >= 32), or of l / (32/NK) in
-// acc[0] (NK < 32).  The additions follow a fixed tree, so a rerun is bitwise the same.
-template <int NK>
-__device__ __forceinline__ void warp_transpose_sum(double (&acc)[NK], int lane) {
-  int held = NK;
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    if (held >= 2) {
-      const int half = held / 2;
-      const bool upper = (lane & o) != 0;
-#pragma unroll
-      for (int k = 0; k < NK / 2; ++k) {
-        if (k < half) {
-          const double send = upper ? acc[k] : acc[k + half];
-          const double keep = upper ? acc[k + half] : acc[k];
-          acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
-      held = half;
-    } else {
-      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-    }
-  }
-}
-
 // The range of elements block b of nb owns
 __device__ __forceinline__ void chunk(int n, int nb, int& lo, int& hi) {
   int per = (n + nb - 1) / nb;
@@ -206,17 +180,135 @@ __global__ void k_cycle_gate(const CaseDev* __restrict__ cases, int n_cases, cud
   }
 }
 
-// The three passes of CGS2 over the basis, one kernel: MODE 0 h = V^T w; MODE 1
-// w -= V hin, then h = V^T w; MODE 2 w -= V hin, then |w| and column j of H.  A block
-// owns a chunk of cgs_chunk(n) elements.  The update runs thread per element (for an FP64
-// basis the nk loads of an element issued together, up to 32 in flight, before they are
-// added in order); the dot products run warp per basis vector against the block's w held
-// in shared memory, each lane with 32 loads in flight (16 for an FP32 basis).  With one
-// or two blocks per SM the passes are bound by the bytes in flight, hence the batches;
-// the order of every sum is that of one load at a time.  In MODE 1 the second read of
-// the chunk's basis rows is served by L2.
-template <class TV, int NK, int MODE>
-__global__ void __launch_bounds__(RED_THREADS) k_mdot(const CaseDev* __restrict__ cases, int nk, int j) {
+// The three passes of CGS2 over an FP64 basis: h1 = V^T w; w -= V h1, then h2 = V^T w; w -= V h2,
+// then |w| and column j of H.  A block owns a contiguous part of a case (orth_blocks(n) of
+// them, at most one an SM); a thread holds its E elements' entries of every vector in
+// registers, so the second pass updates w and takes its dots from one read of the basis, and
+// NK x E loads a thread are in flight.  On one 385 x 97 case (194k unknowns) a pass is its
+// latency: launch, a few rounds of loads, the sums' two stages; the three over 30 vectors take
+// 39 us, 135 us on a 769 x 193 case (a warp a vector over 512- to 2048-element chunks, the
+// second pass reading the basis twice: 55 and 188 us).
+
+// The dots of the NK vectors from k0 (nk of them) with w, after (UPDATE) w -= sum h V over the
+// same vectors.  second: h1 in, h2 out; else h1 out.
+template <int NK, int E, bool UPDATE>
+__global__ void __launch_bounds__(ORTH_THREADS, NK <= 8 ? 2 : 1)
+    k_orth_dots(const CaseDev* __restrict__ cases, int k0, int nk, int second) {
+  const CaseDev& cd = cases[blockIdx.y];
+  if (!cd.enabled) return;
+  Scalars* sc = cd.sc;
+  if (sc->active == 0) return;
+  const int n = cd.n_vec, nb = orth_blocks(n);
+  if ((int)blockIdx.x >= nb) return;
+  const size_t ldv = (size_t)n;
+  const double* __restrict__ V = (const double*)cd.V + (size_t)k0 * ldv;
+  double* __restrict__ w = cd.w;
+  double* hout = (second ? sc->h2 : sc->h1) + k0;
+  __shared__ double h[NK], total[NK];
+  if (UPDATE) {
+    if ((int)threadIdx.x < NK) h[threadIdx.x] = (int)threadIdx.x < nk ? sc->h1[k0 + threadIdx.x] : 0.0;
+    __syncthreads();
+  }
+  int lo, hi;
+  chunk(n, nb, lo, hi);
+  double acc[NK];
+#pragma unroll
+  for (int k = 0; k < NK; ++k) acc[k] = 0.0;
+  for (int e = lo + threadIdx.x; e < hi; e += E * ORTH_THREADS) {
+    double x[E];
+    double v[E][NK];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int at = e + i * ORTH_THREADS;
+      x[i] = at < hi ? w[at] : 0.0;
+#pragma unroll
+      for (int k = 0; k < NK; ++k) v[i][k] = k < nk && at < hi ? V[k * ldv + at] : 0.0;
+    }
+    if (UPDATE) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) {
+        const int at = e + i * ORTH_THREADS;
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < NK; ++k)
+          if (k < nk) s += h[k] * v[i][k];
+        x[i] -= s;
+        if (at < hi) w[at] = x[i];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+      if (k < nk)
+#pragma unroll
+        for (int i = 0; i < E; ++i) acc[k] += v[i][k] * x[i];
+  }
+  if (finish_sums<NK>(acc, cd.partial, cd.ticket, nb, total) && (int)threadIdx.x < nk)
+    hout[threadIdx.x] = total[threadIdx.x];
+}
+
+// w -= sum h V over all nk vectors (h: h2, or h1 where `first`), and with `column` |w| and
+// column j of H
+__global__ void __launch_bounds__(ORTH_THREADS) k_orth_update(const CaseDev* __restrict__ cases, int nk, int j,
+                                                              int first, int column) {
+  const CaseDev& cd = cases[blockIdx.y];
+  if (!cd.enabled) return;
+  Scalars* sc = cd.sc;
+  if (sc->active == 0) return;
+  const int n = cd.n_vec, m = cd.m, nb = orth_blocks(n);
+  if ((int)blockIdx.x >= nb) return;
+  const size_t ldv = (size_t)n;
+  const double* __restrict__ V = (const double*)cd.V;
+  double* __restrict__ w = cd.w;
+  __shared__ double h[MAX_KRYLOV], total[8];
+  if ((int)threadIdx.x < nk) h[threadIdx.x] = (first ? sc->h1 : sc->h2)[threadIdx.x];
+  __syncthreads();
+  int lo, hi;
+  chunk(n, nb, lo, hi);
+  double acc[8] = {};
+  constexpr int E = 2, KB = 16;
+  for (int e = lo + threadIdx.x; e < hi; e += E * ORTH_THREADS) {
+    double x[E], s[E] = {};
+#pragma unroll
+    for (int i = 0; i < E; ++i) x[i] = e + i * ORTH_THREADS < hi ? w[e + i * ORTH_THREADS] : 0.0;
+    for (int k0 = 0; k0 < nk; k0 += KB) {
+      double v[E][KB];
+#pragma unroll
+      for (int i = 0; i < E; ++i)
+#pragma unroll
+        for (int k = 0; k < KB; ++k)
+          v[i][k] = k0 + k < nk && e + i * ORTH_THREADS < hi ? V[(k0 + k) * ldv + e + i * ORTH_THREADS] : 0.0;
+#pragma unroll
+      for (int k = 0; k < KB; ++k)
+        if (k0 + k < nk)
+#pragma unroll
+          for (int i = 0; i < E; ++i) s[i] += h[k0 + k] * v[i][k];
+    }
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      x[i] -= s[i];
+      acc[0] += x[i] * x[i];
+      if (e + i * ORTH_THREADS < hi) w[e + i * ORTH_THREADS] = x[i];
+    }
+  }
+  if (!column || !finish_sums<8>(acc, cd.partial, cd.ticket, nb, total)) return;
+  const double nrm = sqrt(total[0]);
+  if ((int)threadIdx.x < nk) sc->H[threadIdx.x + (m + 1) * j] = sc->h1[threadIdx.x] + sc->h2[threadIdx.x];
+  if (threadIdx.x == 0) {
+    sc->H[j + 1 + (m + 1) * j] = nrm;
+    sc->nrm = nrm;
+    sc->inv_nrm = 1.0 / fmax(nrm, 2.2250738585072014e-308);
+    if (nrm == 0.0) sc->status |= ST_GMRES_BREAKDOWN;
+  }
+}
+
+// The same passes over an FP32 basis (the mixed form), one kernel: MODE 0, 1, 2.  A block owns a
+// chunk of cgs_chunk(n) elements; the update runs thread per element and the dot products warp
+// per basis vector against the block's w in shared memory, 16 loads in flight a lane, so the
+// FP64 conversions follow whole batches of loads.  Holding the entries in registers as the
+// FP64 passes do is slower here (the loads, each with its conversion, are not issued
+// together): nine cases' 442k cells, three passes over 30 vectors, 324 against 488 us.
+template <int NK, int MODE>
+__global__ void __launch_bounds__(RED_THREADS) k_mdot_fp32(const CaseDev* __restrict__ cases, int nk, int j) {
   const CaseDev& cd = cases[blockIdx.y];
   if (!cd.enabled) return;
   Scalars* sc = cd.sc;
@@ -224,7 +316,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_mdot(const CaseDev* __restrict_
   const int n = cd.n_vec, m = cd.m;
   const int nb = cgs_blocks(n), C = cgs_chunk(n);
   if ((int)blockIdx.x >= nb) return;
-  const TV* __restrict__ V = (const TV*)cd.V;
+  const float* __restrict__ V = (const float*)cd.V;
   const size_t ldv = (size_t)n;
   double* __restrict__ w = cd.w;
   double* __restrict__ partial = cd.partial;
@@ -248,19 +340,10 @@ __global__ void __launch_bounds__(RED_THREADS) k_mdot(const CaseDev* __restrict_
     const int i = i0 + e;
     double wi = w[i];
     if constexpr (MODE != 0) {
-      // an FP64 basis: the element's nk entries loaded together, then added in order (an
-      // FP32 basis keeps one load per entry: measured faster there)
-      constexpr int KB = sizeof(TV) == 4 ? 1 : (NK < 32 ? NK : 32);
       double s = 0.0;
 #pragma unroll
-      for (int k0 = 0; k0 < NK; k0 += KB) {
-        double vk[KB];
-#pragma unroll
-        for (int u = 0; u < KB; ++u) vk[u] = k0 + u < nk ? double(V[(size_t)(k0 + u) * ldv + i]) : 0.0;
-#pragma unroll
-        for (int u = 0; u < KB; ++u)
-          if (k0 + u < nk) s += h[k0 + u] * vk[u];
-      }
+      for (int k = 0; k < NK; ++k)
+        if (k < nk) s += h[k] * double(V[(size_t)k * ldv + i]);
       wi = wi - s;
       w[i] = wi;
     }
@@ -281,18 +364,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_mdot(const CaseDev* __restrict_
     __syncthreads();
     // 2. the dot products, warp per basis vector
     for (int k = warp; k < nk; k += nw) {
-      const TV* __restrict__ vk = V + k * ldv + i0;
+      const float* __restrict__ vk = V + k * ldv + i0;
       double a = 0.0;
       int e = lane;
-      if constexpr (sizeof(TV) == 8) {   // an FP64 basis: 32 loads in flight per lane
-        for (; e + 32 * 31 < cn; e += 32 * 32) {
-          double x[32];
-#pragma unroll
-          for (int u = 0; u < 32; ++u) x[u] = double(vk[e + 32 * u]);
-#pragma unroll
-          for (int u = 0; u < 32; ++u) a += x[u] * ws[e + 32 * u];
-        }
-      }
       for (; e + 32 * 15 < cn; e += 32 * 16) {
         double x[16];
 #pragma unroll
@@ -609,27 +683,47 @@ void launch_cycle_gate(const CaseDev* cases, const BatchDims& d, cudaGraphCondit
   k_cycle_gate<<<1, 256, 0, st>>>(cases, d.n_cases, gate, cycles);
 }
 
-template <class TV, int NK>
-static void arnoldi_nk(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
-  dim3 grid(d.cgs_blocks, d.n_cases);
-  k_mdot<TV, NK, 0><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
-  k_mdot<TV, NK, 1><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
-  k_mdot<TV, NK, 2><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
+static void orth_fp64(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
+  const int nk = j + 1;
+  const dim3 grid(orth_blocks(d.n_vec), d.n_cases);
+  auto dots = [&](int k0, int count, int second) {
+    if (count <= 8) k_orth_dots<8, 4, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
+    else if (count <= 16) k_orth_dots<16, 2, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
+    else k_orth_dots<32, 2, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
+  };
+  for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(k0, min(ORTH_NK, nk - k0), 0);
+  if (nk <= 8) {
+    k_orth_dots<8, 4, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+  } else if (nk <= 16) {
+    k_orth_dots<16, 2, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+  } else if (nk <= ORTH_NK) {
+    k_orth_dots<32, 1, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+  } else {   // more vectors than a thread holds: the update, then the dots in slices
+    k_orth_update<<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, 1, 0);
+    for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(k0, min(ORTH_NK, nk - k0), 1);
+  }
+  k_orth_update<<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, 0, 1);
 }
 
-template <class TV>
-static void arnoldi_t(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
+template <int NK> static void mdot_fp32(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
+  const dim3 grid(d.cgs_blocks, d.n_cases);
+  k_mdot_fp32<NK, 0><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
+  k_mdot_fp32<NK, 1><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
+  k_mdot_fp32<NK, 2><<<grid, RED_THREADS, 0, st>>>(cases, j + 1, j);
+}
+
+static void orth_fp32(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
   const int nk = j + 1;
-  if (nk <= 8) arnoldi_nk<TV, 8>(cases, d, j, st);
-  else if (nk <= 16) arnoldi_nk<TV, 16>(cases, d, j, st);
-  else if (nk <= 32) arnoldi_nk<TV, 32>(cases, d, j, st);
-  else arnoldi_nk<TV, 64>(cases, d, j, st);
+  if (nk <= 8) mdot_fp32<8>(cases, d, j, st);
+  else if (nk <= 16) mdot_fp32<16>(cases, d, j, st);
+  else if (nk <= 32) mdot_fp32<32>(cases, d, j, st);
+  else mdot_fp32<64>(cases, d, j, st);
 }
 
 // orthogonalise w against V_0..V_j (CGS2) and append column j of H
 void launch_arnoldi_orth(const CaseDev* cases, const BatchDims& d, bool fp32, int j, cudaStream_t st) {
-  if (fp32) arnoldi_t<float>(cases, d, j, st);
-  else arnoldi_t<double>(cases, d, j, st);
+  if (fp32) orth_fp32(cases, d, j, st);
+  else orth_fp64(cases, d, j, st);
 }
 
 void launch_lstsq(const CaseDev* cases, const BatchDims& d, cudaStream_t st) {

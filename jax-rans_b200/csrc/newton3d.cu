@@ -10,6 +10,7 @@
 #include "linesolve3d.cuh"
 #include "newton3d.cuh"
 #include "newton3d_ops.cuh"
+#include "orth.cuh"
 
 namespace jr {
 
@@ -63,32 +64,6 @@ __global__ void k3_dot_partial(size_t N, const double* __restrict__ a, const dou
 // the 3.9M-cell wing (215 MB a vector) bound by HBM: pass 0 against 17 to 30 vectors reads
 // 6.8 TB/s, pass 1 4.9; a step's three passes over 30 vectors 1.9 ms on average where separate
 // dots (w read again for each vector) and updates took 2.8.  The sums are fixed by N alone.
-constexpr int ORTH_THREADS = 256, ORTH_BLOCKS = 148, ORTH_NK = 32;
-
-// The NK sums of every lane over the warp, by a butterfly that halves the sums a lane holds at
-// each exchange: afterwards lane l holds sum l * NK / 32 (NK < 32: every 32 / NK-th lane's) in
-// acc[0].
-template <int NK>
-__device__ __forceinline__ void lane_sums(double (&acc)[NK], int lane) {
-  int held = NK;
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    if (held >= 2) {
-      const int half = held / 2;
-      const bool upper = (lane & o) != 0;
-#pragma unroll
-      for (int k = 0; k < NK / 2; ++k)
-        if (k < half) {
-          const double send = upper ? acc[k] : acc[k + half], keep = upper ? acc[k + half] : acc[k];
-          acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      held = half;
-    } else {
-      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
-    }
-  }
-}
-
 template <int E> struct Elems {
   double x[E];
 };
@@ -108,54 +83,10 @@ template <int E> __device__ __forceinline__ void store_elems(double* p, const El
   else *p = v.x[0];
 }
 
-// sums[NK] of every thread: over the block into partial, and by the last block over the
-// blocks in order; true there, with the totals in total[NK]
-template <int NK>
-__device__ bool finish_sums(double (&sums)[NK], double* partial, unsigned* ticket, double* total) {
-  __shared__ double warps[ORTH_THREADS / 32][NK];
-  __shared__ double groups[ORTH_THREADS];
-  __shared__ bool last;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  lane_sums<NK>(sums, lane);
-  if (lane % (32 / NK) == 0) warps[warp][lane / (32 / NK)] = sums[0];
-  __syncthreads();
-  if (t < NK) {
-    double s = warps[0][t];
-    for (int w = 1; w < ORTH_THREADS / 32; ++w) s += warps[w][t];
-    partial[(size_t)blockIdx.x * NK + t] = s;
-  }
-  __threadfence();
-  __syncthreads();
-  if (t == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  constexpr int G = ORTH_THREADS / NK;
-  const int k = t % NK, g = t / NK, nb = gridDim.x;
-  double s = 0.0;
-  for (int b = g; b < nb; b += 8 * G) {
-    double x[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) x[u] = b + u * G < nb ? __ldcg(partial + (size_t)(b + u * G) * NK + k) : 0.0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) s += x[u];
-  }
-  groups[t] = s;
-  __syncthreads();
-  if (t < NK) {
-    double v = groups[t];
-    for (int q = 1; q < G; ++q) v += groups[q * NK + t];
-    total[t] = v;
-  }
-  if (t == 0) *ticket = 0u;
-  __syncthreads();
-  return true;
-}
-
 // The dots of vectors k0 .. k0 + nk - 1 (nk <= NK) with w, after (UPDATE) w -= sum h V over
 // the same vectors; hin, hout: the scalars of vector k0.
 template <int NK, int E, bool UPDATE>
-__global__ void __launch_bounds__(ORTH_THREADS, 1) k3_orth_dots(size_t N, int nk, const double* __restrict__ V,
+__global__ void __launch_bounds__(ORTH_THREADS, NK <= 16 ? 2 : 1) k3_orth_dots(size_t N, int nk, const double* __restrict__ V,
                                                                 double* __restrict__ w,
                                                                 const double* __restrict__ hin, double* hout,
                                                                 double* partial, unsigned* ticket) {
@@ -190,7 +121,7 @@ __global__ void __launch_bounds__(ORTH_THREADS, 1) k3_orth_dots(size_t N, int nk
 #pragma unroll
         for (int i = 0; i < E; ++i) acc[k] += v[k].x[i] * we.x[i];
   }
-  if (finish_sums<NK>(acc, partial, ticket, total) && (int)threadIdx.x < nk) hout[threadIdx.x] = total[threadIdx.x];
+  if (finish_sums<NK>(acc, partial, ticket, gridDim.x, total) && (int)threadIdx.x < nk) hout[threadIdx.x] = total[threadIdx.x];
 }
 
 // w -= sum h V over all nk vectors, and with `column` |w| and column j of H (m + 1 rows,
@@ -225,7 +156,7 @@ __global__ void __launch_bounds__(ORTH_THREADS) k3_orth_update(size_t N, int nk,
     }
     store_elems<E>(w + e, we);
   }
-  if (!column || !finish_sums<8>(acc, partial, &g->ticket, total)) return;
+  if (!column || !finish_sums<8>(acc, partial, &g->ticket, gridDim.x, total)) return;
   const double nrm = sqrt(total[0]);
   for (int i = threadIdx.x; i < nk; i += ORTH_THREADS) g->H[i * m + j] = g->h1[i] + g->h2[i];
   if (threadIdx.x == 0) {
@@ -414,7 +345,7 @@ template <int E> static void orthogonalise(DeviceOps3& o, int j, int m) {
     const double* Vk = V + (size_t)k0 * o.N;
     // (few vectors: registers for two blocks an SM, which the reads in flight then need)
     if (count <= 8) orth_dots<8, E>(o, update, blocks * 2, count, Vk, w, hin, hout + k0);
-    else if (count <= 16) orth_dots<16, E>(o, update, blocks, count, Vk, w, hin, hout + k0);
+    else if (count <= 16) orth_dots<16, E>(o, update, blocks * 2, count, Vk, w, hin, hout + k0);
     else orth_dots<ORTH_NK, E>(o, update, blocks, count, Vk, w, hin, hout + k0);
   };
   auto update = [&](const double* h, int column) {
