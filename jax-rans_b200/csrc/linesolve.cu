@@ -20,24 +20,27 @@ namespace jr {
 
 constexpr int LS_THREADS = 128;
 
-// A = d(F.S)/dU (4x4, [row][col]) by forward-mode tangents of the flux of the
-// conservative state (physics/euler.py:55-71)
+// A = d(F.S)/dU (4x4, [row][col]) of the conservative state whose primitives are q
+// (physics/euler.py:55-71), in closed form
 __device__ __forceinline__ void flux_jacobian(const double* q, double sx, double sy, double g, double A[4][4]) {
-  double U[4];
-  U[0] = q[0];
-  U[1] = q[0] * q[1];
-  U[2] = q[0] * q[2];
-  U[3] = q[3] / (g - 1.0) + 0.5 * q[0] * (q[1] * q[1] + q[2] * q[2]);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    Dual Ud[4], qd[4], F[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) Ud[v] = Dual{U[v], v == k ? 1.0 : 0.0};
-    to_prim(Ud, qd, 4, g);
-    normal_flux(qd, sx, sy, g, F);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) A[r][k] = F[r].d;
-  }
+  const double u = q[1], v = q[2], vn = u * sx + v * sy, vv = u * u + v * v, g1 = g - 1.0;
+  const double phi = 0.5 * g1 * vv, H = g / g1 * q[3] / q[0] + 0.5 * vv;
+  A[0][0] = 0.0;
+  A[0][1] = sx;
+  A[0][2] = sy;
+  A[0][3] = 0.0;
+  A[1][0] = phi * sx - u * vn;
+  A[1][1] = vn + u * sx - g1 * u * sx;
+  A[1][2] = u * sy - g1 * v * sx;
+  A[1][3] = g1 * sx;
+  A[2][0] = phi * sy - v * vn;
+  A[2][1] = v * sx - g1 * u * sy;
+  A[2][2] = vn + v * sy - g1 * v * sy;
+  A[2][3] = g1 * sy;
+  A[3][0] = (phi - H) * vn;
+  A[3][1] = H * sx - g1 * u * vn;
+  A[3][2] = H * sy - g1 * v * vn;
+  A[3][3] = g * vn;
 }
 
 // unpivoted Gauss-Jordan inverse (core/linalg.py:49-77)
@@ -52,9 +55,9 @@ template <class S> __device__ __forceinline__ void invert4(const S M[4][4], S In
     }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    S p = a[k][k];
+    const S p = S(1) / a[k][k];   // one quotient a pivot
 #pragma unroll
-    for (int c = 0; c < 8; ++c) a[k][c] = a[k][c] / p;
+    for (int c = 0; c < 8; ++c) a[k][c] = a[k][c] * p;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (r == k) continue;
@@ -116,8 +119,10 @@ __device__ __forceinline__ void face_vector(const Canvas& cv, int f, double& sx,
 __device__ __forceinline__ void prim_at(const Canvas& cv, const Physics& P, const double* U, int idx, double* q) {
   const int N = cv.ncanvas();
   double u[5];
-  for (int v = 0; v < cv.nvar; ++v) u[v] = U[v * N + idx];
-  to_prim(u, q, cv.nvar, P.gamma);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) u[v] = U[v * N + idx];
+  u[4] = cv.nvar > 4 ? U[4 * N + idx] : 0.0;
+  to_prim(u, q, 5, P.gamma);
 }
 
 // 1/2 A(q_nb, sign S) - 1/2 lambda I, or zero where the link does not exist

@@ -1173,11 +1173,14 @@ __global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__
 // partner from the neighbour map), the SA mass flux and diffusion per face.
 // ------------------------------------------------------------------------------------
 
+// (NV == c.nvar fixed at compile time, so the state stays in registers)
+template <int NV>
 __device__ __forceinline__ void prim_raw(const Canvas& c, const Physics& P, const double* U, int idx, double* q) {
   const int N = c.ncanvas();
   double u[5];
-  for (int v = 0; v < c.nvar; ++v) u[v] = U[v * N + idx];
-  to_prim(u, q, c.nvar, P.gamma);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) u[v] = U[v * N + idx];
+  to_prim(u, q, NV, P.gamma);
 }
 
 template <int VISC>
@@ -1220,9 +1223,11 @@ __global__ void k_faces(const CaseDev* __restrict__ cases) {
     }
     int na = c.neighbours[a], nb = c.neighbours[b];
     double qa[5], qb[5], qf[5];
-    prim_raw(c, P, U, na, qa);
-    prim_raw(c, P, U, nb, qb);
-    for (int v = 0; v < c.nvar; ++v) qf[v] = 0.5 * (qa[v] + qb[v]);
+    constexpr int NV = VISC == 2 ? 5 : 4;
+    prim_raw<NV>(c, P, U, na, qa);
+    prim_raw<NV>(c, P, U, nb, qb);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) qf[v] = 0.5 * (qa[v] + qb[v]);
     double vn = qf[1] * sx + qf[2] * sy;
     double l = fabs(vn) + sqrt(g * qf[3] / qf[0]) * hypot(sx, sy);
     if (VISC > 0) {
@@ -1278,26 +1283,32 @@ __global__ void k_cells(const CaseDev* __restrict__ cases) {
       auto out_f = [&](int f) { return fmax(mflux[f], 0.0) + dflux[f]; };
       auto in_f = [&](int f) { return fmax(-mflux[f], 0.0) + dflux[f]; };
       double q[5];
-      prim_raw(c, P, U, idx, q);
+      prim_raw<5>(c, P, U, idx, q);
       double diag = ((out_f(fh) + in_f(fl)) + out_f(gh)) + in_f(gl);
       diag = diag / q[0];
       // vorticity from face-averaged velocities (neighbour-filled raw states)
       double sxl = c.fi[fl], syl = c.fi[nfi + fl], sxh = c.fi[fh], syh = c.fi[nfi + fh];
       int jl = i * (NJ + 1) + j, jh = jl + 1;
       double txl = c.fj[jl], tyl = c.fj[c.nfj() + jl], txh = c.fj[jh], tyh = c.fj[c.nfj() + jh];
-      auto favg = [&](int a, int b, int v) {
-        double qa[5], qb[5];
-        prim_raw(c, P, U, c.neighbours[a], qa);
-        prim_raw(c, P, U, c.neighbours[b], qb);
-        return 0.5 * (qa[v] + qb[v]);
+      // the velocities of the cell and its four neighbours, each as the faces' means take it
+      auto vel = [&](int a, double* w) {
+        double q5[5];
+        prim_raw<5>(c, P, U, c.neighbours[a], q5);
+        w[0] = q5[1];
+        w[1] = q5[2];
       };
-      int im = max(i - 1, 0) * NJ + j, ip = min(i + 1, NI - 1) * NJ + j;
-      int jm = i * NJ + max(j - 1, 0), jp = i * NJ + min(j + 1, NJ - 1);
+      double own[2], wim[2], wip[2], wjm[2], wjp[2];
+      vel(idx, own);
+      vel(max(i - 1, 0) * NJ + j, wim);
+      vel(min(i + 1, NI - 1) * NJ + j, wip);
+      vel(i * NJ + max(j - 1, 0), wjm);
+      vel(i * NJ + min(j + 1, NJ - 1), wjp);
       double vol = c.volume[idx];
       double gxv[2], gyv[2];
+#pragma unroll
       for (int v = 0; v < 2; ++v) {
-        double pil = favg(im, idx, 1 + v), pih = favg(idx, ip, 1 + v);
-        double pjl = favg(jm, idx, 1 + v), pjh = favg(idx, jp, 1 + v);
+        double pil = 0.5 * (wim[v] + own[v]), pih = 0.5 * (own[v] + wip[v]);
+        double pjl = 0.5 * (wjm[v] + own[v]), pjh = 0.5 * (own[v] + wjp[v]);
         gxv[v] = ((pih * sxh - pil * sxl) + (pjh * txh - pjl * txl)) / vol;
         gyv[v] = ((pih * syh - pil * syl) + (pjh * tyh - pjl * tyl)) / vol;
       }
@@ -1428,17 +1439,17 @@ void launch_ghosts(const CaseDev* cases, const BatchDims& d, int tangent_id, int
 }
 
 void launch_faces(const CaseDev* cases, const BatchDims& d, int visc, cudaStream_t st) {
-  dim3 grid(max(1, min((d.faces + 255) / 256, 148 * 8)), d.n_cases);
-  if (visc == 2) k_faces<2><<<grid, 256, 0, st>>>(cases);
-  else if (visc == 1) k_faces<1><<<grid, 256, 0, st>>>(cases);
-  else k_faces<0><<<grid, 256, 0, st>>>(cases);
+  dim3 grid(max(1, min((d.faces + 127) / 128, 148 * 16)), d.n_cases);
+  if (visc == 2) k_faces<2><<<grid, 128, 0, st>>>(cases);
+  else if (visc == 1) k_faces<1><<<grid, 128, 0, st>>>(cases);
+  else k_faces<0><<<grid, 128, 0, st>>>(cases);
 }
 
 void launch_cells(const CaseDev* cases, const BatchDims& d, int visc, cudaStream_t st) {
-  dim3 grid(max(1, min((d.cells + 255) / 256, 148 * 8)), d.n_cases);
-  if (visc == 2) k_cells<2><<<grid, 256, 0, st>>>(cases);
-  else if (visc == 1) k_cells<1><<<grid, 256, 0, st>>>(cases);
-  else k_cells<0><<<grid, 256, 0, st>>>(cases);
+  dim3 grid(max(1, min((d.cells + 127) / 128, 148 * 16)), d.n_cases);
+  if (visc == 2) k_cells<2><<<grid, 128, 0, st>>>(cases);
+  else if (visc == 1) k_cells<1><<<grid, 128, 0, st>>>(cases);
+  else k_cells<0><<<grid, 128, 0, st>>>(cases);
 }
 
 }  // namespace jr
