@@ -216,7 +216,7 @@ __host__ __device__ __forceinline__ int orth_blocks(int n) {
 
 // the number of blocks a per-case reduction over n elements uses (<= the grid's x)
 __host__ __device__ __forceinline__ int chunk_blocks(int n) {
-  int b = (n + 1023) / 1024;
+  int b = (n + 255) / 256;   // one element a thread until two blocks an SM
   return b < 1 ? 1 : (b > 2 * 148 ? 2 * 148 : b);
 }
 

@@ -31,7 +31,7 @@ __device__ __forceinline__ double warp_max(double x) {
 // In the last block of a reduction: out[k] = the sum (or NaN-propagating max) over the
 // nb rows of partial[b * stride + k], k < W, by all the block's threads in a fixed order
 // -- thread (k, r) takes the rows b = r, r + R, ... (R = blockDim.x / W groups), with its
-// loads issued eight at a time, then thread k adds the R group totals in order.  Loads go
+// loads issued eight at a time, then the R group totals are added by halves.  Loads go
 // to L2 (ld.global.cg), where the other blocks' partials are.
 template <bool MAX>
 __device__ void reduce_rows(const double* partial, int stride, int W, int nb, double* out) {
@@ -53,11 +53,14 @@ __device__ void reduce_rows(const double* partial, int stride, int W, int nb, do
     group[t] = acc;
   }
   __syncthreads();
-  if (t < W) {
-    double v = group[t];
-    for (int g = 1; g < R; ++g) v = MAX ? nmax(v, group[g * W + t]) : v + group[g * W + t];
-    out[t] = v;
+  // the R groups by halving (one after another they are a serial chain of R shared loads)
+  int half = 1;
+  while (2 * half < R) half *= 2;
+  for (; half > 0; half >>= 1) {
+    if (r < half && r + half < R) group[t] = MAX ? nmax(group[t], group[t + half * W]) : group[t] + group[t + half * W];
+    __syncthreads();
   }
+  if (t < W) out[t] = group[t];
   __syncthreads();
 }
 
@@ -136,15 +139,20 @@ __global__ void __launch_bounds__(RED_THREADS) k_gmres_init(const CaseDev* __res
     action[i] = 0.0;
     acc[0] += v * v;
   }
+  if (blockIdx.x == 0) {   // the residual's norm, from its tiles' sums by all the block's threads
+    __shared__ double total;
+    reduce_rows<false>(cd.tile_partial, 1, 1, cd.n_tiles, &total);
+    if (threadIdx.x == 0) {
+      Scalars* sc = cd.sc;
+      const double nrm = sqrt(total / cd.c.volume_sum);
+      sc->norm = nrm;
+      // history: [step][case] over the cases of the batch
+      if (cd.history != nullptr) cd.history[(size_t)sc->hpos * n_cases_hist + cd.slot] = nrm;
+      sc->hpos += 1;
+    }
+  }
   if (reduce_last<1>(acc, cd.partial, cd.ticket, nb)) {
     Scalars* sc = cd.sc;
-    double s = 0.0;
-    for (int t = 0; t < cd.n_tiles; ++t) s += cd.tile_partial[t];
-    double nrm = sqrt(s / cd.c.volume_sum);
-    sc->norm = nrm;
-    // history: [step][case] over the cases of the batch
-    if (cd.history != nullptr) cd.history[(size_t)sc->hpos * n_cases_hist + cd.slot] = nrm;
-    sc->hpos += 1;
     sc->bnorm = sqrt(acc[0]);
     sc->rnorm = sc->bnorm;
     sc->cycle = 0;
@@ -405,72 +413,61 @@ __global__ void __launch_bounds__(RED_THREADS) k_mdot_fp32(const CaseDev* __rest
 }
 
 // argmin |beta e1 - H y| by Givens rotations, pivots below rcond * the largest dropped
-// (krylov.py:100-137); hy = H y.  One CTA per case: rotation j, once formed, is applied
-// to rows j, j+1 of every later column at once -- each entry sees the same rotations in
-// the same order as column-by-column elimination.
-__global__ void __launch_bounds__(64) k_lstsq(const CaseDev* __restrict__ cases) {
+// (krylov.py:100-137); hy = H y.  One warp per case, columns over its lanes: rotation j, once
+// formed by the lane that holds column j, is applied to rows j, j+1 of every later column at
+// once -- each entry sees the same rotations in the same order as column-by-column
+// elimination -- and the back substitution takes column j out of every row above at once.  A
+// serial chain of m roots and quotients: no block barrier lies in it (m = 30: 32 us as two
+// warps with three barriers a rotation, 20 us so; m = 10: 11 -> 7 us).
+__global__ void __launch_bounds__(32) k_lstsq(const CaseDev* __restrict__ cases) {
   const CaseDev& cd = cases[blockIdx.y];
   if (!cd.enabled) return;
   Scalars* sc = cd.sc;
   if (sc->active == 0) return;
-  const int m = cd.m;
+  const int m = cd.m, lane = threadIdx.x;
   __shared__ double h[MAX_KRYLOV + 1][MAX_KRYLOV + 1];
-  __shared__ double g[MAX_KRYLOV + 1], cs[MAX_KRYLOV], sn[MAX_KRYLOV], y[MAX_KRYLOV];
-  __shared__ double largest;
-  const int t = threadIdx.x;
-  for (int e = t; e < (m + 1) * m; e += blockDim.x) {
-    int i = e % (m + 1), jj = e / (m + 1);
-    h[i][jj] = sc->H[e];
-  }
-  if (t <= m) g[t] = t == 0 ? sc->beta : 0.0;
-  __syncthreads();
+  __shared__ double g[MAX_KRYLOV + 1], y[MAX_KRYLOV];
+  for (int e = lane; e < (m + 1) * m; e += 32) h[e % (m + 1)][e / (m + 1)] = sc->H[e];
+  for (int i = lane; i <= m; i += 32) g[i] = i == 0 ? sc->beta : 0.0;
+  __syncwarp();
+  double largest = 0.0;
   for (int j = 0; j < m; ++j) {
-    if (t == 0) {
-      double a = h[j][j], c = h[j + 1][j];
-      double r = sqrt(a * a + c * c);
-      double safe = r > 0.0 ? r : 1.0;
-      double cj = r > 0.0 ? a / safe : 1.0, sj = r > 0.0 ? c / safe : 0.0;
-      cs[j] = cj;
-      sn[j] = sj;
+    // every lane forms the rotation from the same two entries
+    const double a = h[j][j], c = h[j + 1][j];
+    const double r = sqrt(a * a + c * c);
+    const double safe = r > 0.0 ? r : 1.0;
+    const double cj = r > 0.0 ? a / safe : 1.0, sj = r > 0.0 ? c / safe : 0.0;
+    const double gj = g[j];
+    __syncwarp();
+    largest = j == 0 ? r : fmax(largest, r);
+    for (int col = j + 1 + lane; col < m; col += 32) {
+      const double p = h[j][col], q = h[j + 1][col];
+      h[j][col] = cj * p + sj * q;
+      h[j + 1][col] = cj * q - sj * p;
+    }
+    if (lane == 0) {
       h[j][j] = r;
       h[j + 1][j] = 0.0;
-      double gj = g[j];
       g[j] = cj * gj;
       g[j + 1] = -sj * gj;
     }
-    __syncthreads();
-    for (int col = j + 1 + t; col < m; col += blockDim.x) {
-      double a = h[j][col], c = h[j + 1][col];
-      h[j][col] = cs[j] * a + sn[j] * c;
-      h[j + 1][col] = cs[j] * c - sn[j] * a;
-    }
-    __syncthreads();
+    __syncwarp();
   }
-  if (t == 0) {
-    double l = fabs(h[0][0]);
-    for (int jj = 1; jj < m; ++jj) l = fmax(l, fabs(h[jj][jj]));
-    largest = l;
-  }
-  __syncthreads();
   const double rcond = 2.220446049250313e-16 * (m + 1);
   for (int j = m - 1; j >= 0; --j) {
-    if (t < 32) {
-      double s = 0.0;
-      for (int k = j + 1 + t; k < m; k += 32) s += h[j][k] * y[k];
-      s = warp_sum(s);
-      if (t == 0) {
-        double rest = g[j] - s;
-        bool keep = fabs(h[j][j]) > rcond * largest;
-        y[j] = keep ? rest / h[j][j] : 0.0;
-      }
-    }
-    __syncthreads();
+    const double d = h[j][j];
+    const double yj = fabs(d) > rcond * largest ? g[j] / d : 0.0;
+    __syncwarp();
+    for (int i = lane; i < j; i += 32) g[i] -= h[i][j] * yj;
+    if (lane == 0) y[j] = yj;
+    __syncwarp();
   }
-  if (t < m) sc->y[t] = y[t];
-  if (t <= m) {
+  for (int i = lane; i < m; i += 32) sc->y[i] = y[i];
+  for (int i = lane; i <= m; i += 32) {
     double s = 0.0;
-    for (int jj = 0; jj < m; ++jj) s += sc->H[t + (m + 1) * jj] * y[jj];
-    sc->hy[t] = s;
+#pragma unroll 8
+    for (int jj = 0; jj < m; ++jj) s += sc->H[i + (m + 1) * jj] * y[jj];
+    sc->hy[i] = s;
   }
 }
 
@@ -727,7 +724,7 @@ void launch_arnoldi_orth(const CaseDev* cases, const BatchDims& d, bool fp32, in
 }
 
 void launch_lstsq(const CaseDev* cases, const BatchDims& d, cudaStream_t st) {
-  k_lstsq<<<dim3(1, d.n_cases), 64, 0, st>>>(cases);
+  k_lstsq<<<dim3(1, d.n_cases), 32, 0, st>>>(cases);
 }
 
 void launch_combine(const CaseDev* cases, const BatchDims& d, bool fp32, cudaStream_t st) {
