@@ -114,7 +114,7 @@ __host__ __device__ void linearize_face3(const Plan3Dev& p, const double* Q, int
   }
   if constexpr (VISC) {
     double grad[3][5];
-    face_gradient_stored<double, SA ? 5 : 4>(p, Q, a, i, j, k, grad);
+    face_gradient_stored<double, SA ? 5 : 4>(p, ql, qh, a, i, j, k, grad);
     double vel[3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) vel[m] = 0.5 * (ql[1 + m] + qh[1 + m]);

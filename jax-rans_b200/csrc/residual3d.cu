@@ -79,28 +79,35 @@ void launch_face_geometry3(const Plan3Dev& p, double* geo, cudaStream_t st) {
   k3_face_geometry<<<(nf + 127) / 128, 128, 0, st>>>(p, geo, nf);
 }
 
-// (FO 1: the first-order flux, 2: second order; PART 0: the whole flux, 1: its inviscid
-// part, 2: its viscous part added to the stored inviscid part)
+// (FO 1: the first-order flux, 2: second order; PART as face_flux's)
 template <class T, bool VISC, bool SA, int FO, int PART>
 __global__ void __launch_bounds__(128) k3_face_flux(Plan3Dev p, const T* __restrict__ Q, int nf) {
   for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x)
     store_face_flux<T, VISC, SA, FO, PART>(p, Q, FO == 1, f, p.face_buf, (size_t)nf);
 }
 
-// A viscous flux in two launches (inviscid, then viscous added): each holds half the
-// live values of the whole, so neither spills the way the fused face did.  The viscous
-// launch reads its diamond gradient's geometry from the plan (k3_face_geometry) and the
-// node values from this evaluation's node pass (k3_node_phi: each node once, not once
-// for each of the twelve faces round it).
+// A viscous flux reads its diamond gradient's geometry from the plan (k3_face_geometry) and
+// the node values from this evaluation's node pass (k3_node_phi: each node once, not once for
+// each of the twelve faces round it).  A dual-number flux goes in two launches (inviscid, then
+// viscous added): each holds half the live values of the whole, so neither spills.  A flux of
+// plain doubles fits in one once its gradient takes one reciprocal for its nine quotients
+// (490k cells, SA, second order: 267 us for 245 + 144 us as two; the dual's viscous part
+// 567 -> 390 us by the reciprocal alone).  Bound by FP64 issue and by the latency of the
+// scattered node and cell loads.
 template <class T, bool VISC, bool SA, int FO>
 static void face_parts(const Plan3Dev& p, const T* A, int nf, cudaStream_t st) {
   const int fblocks = (nf + 127) / 128;
   if constexpr (VISC) {
-    counted3(2);
+    counted3(1);
     const int nn = node_count(p);
     k3_node_phi<T, SA ? 5 : 4><<<(nn + 127) / 128, 128, 0, st>>>(p, A);
-    k3_face_flux<T, VISC, SA, FO, 1><<<fblocks, 128, 0, st>>>(p, A, nf);
-    k3_face_flux<T, VISC, SA, FO, 2><<<fblocks, 128, 0, st>>>(p, A, nf);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      k3_face_flux<T, VISC, SA, FO, 3><<<fblocks, 128, 0, st>>>(p, A, nf);
+    } else {
+      counted3(1);
+      k3_face_flux<T, VISC, SA, FO, 1><<<fblocks, 128, 0, st>>>(p, A, nf);
+      k3_face_flux<T, VISC, SA, FO, 2><<<fblocks, 128, 0, st>>>(p, A, nf);
+    }
   } else {
     k3_face_flux<T, VISC, SA, FO, 0><<<fblocks, 128, 0, st>>>(p, A, nf);
   }
@@ -108,8 +115,10 @@ static void face_parts(const Plan3Dev& p, const T* A, int nf, cudaStream_t st) {
 
 template <class T, bool VISC, bool SA>
 static void face_phase(const Plan3Dev& p, const T* A, bool first_order, int nf, cudaStream_t st) {
-  if (first_order) face_parts<T, VISC, SA, 1>(p, A, nf, st);
-  else face_parts<T, VISC, SA, 2>(p, A, nf, st);
+  if constexpr (sizeof(T) == sizeof(double)) {
+    if (!first_order) return face_parts<T, VISC, SA, 2>(p, A, nf, st);
+  }
+  face_parts<T, VISC, SA, 1>(p, A, nf, st);   // (the tangent is the first-order flux's)
 }
 
 // phase 2: each cell's sum of its faces' fluxes (and the SA source)

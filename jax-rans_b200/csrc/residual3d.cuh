@@ -313,28 +313,28 @@ __host__ __device__ __forceinline__ int node_flat(const Plan3Dev& p, int I, int 
 }
 __host__ __device__ __forceinline__ int node_count(const Plan3Dev& p) { return (p.NI + 1) * (p.NJ + 1) * (p.NK + 1); }
 
-// face_gradient from the plan's stored face geometry (p.face_geo) and this evaluation's
-// node values (p.node_buf, filled by k3_node_phi): the same values in the same arithmetic
+// face_gradient from the plan's stored face geometry (p.face_geo), the face's two cells ql,
+// qh and this evaluation's node values (p.node_buf, filled by k3_node_phi): one reciprocal of
+// the determinant in place of a quotient a component
 template <class T, int NPHI>
-__host__ __device__ __forceinline__ void face_gradient_stored(const Plan3Dev& p, const T* Q, int a, int fi, int fj,
-                                                              int fk, T grad[3][5]) {
-  // (shifts by selects, not by indexing small arrays with the family: those would live in
-  // local memory)
-  T pl[5], ph[5];
-  grad_vars(p, Q, cell_index(p, fi - (a == 0), fj - (a == 1), fk - (a == 2)), pl);
-  grad_vars(p, Q, cell_index(p, fi, fj, fk), ph);
+__host__ __device__ __forceinline__ void face_gradient_stored(const Plan3Dev& p, const T* ql, const T* qh, int a, int fi,
+                                                              int fj, int fk, T grad[3][5]) {
+  const double g = p.P.gamma;
+  const T p1[5] = {qh[1] - ql[1], qh[2] - ql[2], qh[3] - ql[3], g * qh[4] / qh[0] - g * ql[4] / ql[0],
+                   NPHI > 4 ? qh[5] - ql[5] : cst<T>(0.0)};
   const size_t nf = (size_t)face_count(p, 0) + face_count(p, 1) + face_count(p, 2);
   const size_t f = (size_t)face_flat(p, a, fi, fj, fk);
+  const double inv = 1.0 / p.face_geo[(size_t)9 * nf + f];
   double c23[3], c31[3], c12[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    c23[d] = p.face_geo[(size_t)d * nf + f];
-    c31[d] = p.face_geo[(size_t)(3 + d) * nf + f];
-    c12[d] = p.face_geo[(size_t)(6 + d) * nf + f];
+    c23[d] = p.face_geo[(size_t)d * nf + f] * inv;
+    c31[d] = p.face_geo[(size_t)(3 + d) * nf + f] * inv;
+    c12[d] = p.face_geo[(size_t)(6 + d) * nf + f] * inv;
   }
-  const double det = p.face_geo[(size_t)9 * nf + f];
   const int b1 = a == 0 ? 1 : 0, b2 = a == 2 ? 1 : 2;
-  // node (fi, fj, fk) shifted by s1 along axis b1 and s2 along axis b2
+  // node (fi, fj, fk) shifted by s1 along axis b1 and s2 along axis b2 (shifts by selects, not
+  // by indexing small arrays with the family: those would live in local memory)
   auto node_at = [&](int s1, int s2) {
     return node_flat(p, fi + (b1 == 0) * s1 + (b2 == 0) * s2, fj + (b1 == 1) * s1 + (b2 == 1) * s2,
                      fk + (b1 == 2) * s1 + (b2 == 2) * s2);
@@ -344,10 +344,9 @@ __host__ __device__ __forceinline__ void face_gradient_stored(const Plan3Dev& p,
   const size_t nn = (size_t)node_count(p);
 #pragma unroll
   for (int m = 0; m < NPHI; ++m) {
-    const T f00 = nb[m * nn + i00], f11 = nb[m * nn + i11], f10 = nb[m * nn + i10], f01 = nb[m * nn + i01];
-    T p1 = ph[m] - pl[m], p2 = f11 - f00, p3 = f01 - f10;
+    const T p2 = nb[m * nn + i11] - nb[m * nn + i00], p3 = nb[m * nn + i01] - nb[m * nn + i10];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) grad[d][m] = (p1 * c23[d] + p2 * c31[d] + p3 * c12[d]) / det;
+    for (int d = 0; d < 3; ++d) grad[d][m] = p1[m] * c23[d] + p2 * c31[d] + p3 * c12[d];
   }
 }
 
@@ -397,9 +396,10 @@ __host__ __device__ __forceinline__ void qcr_extra(const T grad[3][5], const T& 
 
 // FO: 1 first order, 2 second order, 0 as `first_order` says (the kernels fix it at
 // compile time, so a first-order flux loads only the two cells either side).  PART: 0 the
-// whole flux; 1 its inviscid part (with the SA row's upwind convection); 2 its viscous
-// part alone, the terms the whole flux subtracts, negated (0 - term), so that part 1 plus
-// part 2 is the whole flux bitwise (a + (0 - b) == a - b).
+// whole flux; 3 the same with its gradient from the plan's stored geometry; 1 its inviscid
+// part (with the SA row's upwind convection); 2 its viscous part alone, the terms the whole
+// flux subtracts, negated (0 - term), so that part 1 plus part 2 is the whole flux bitwise
+// (a + (0 - b) == a - b).
 template <class T, bool VISC, bool SA, int FO = 0, int PART = 0>
 __host__ __device__ void face_flux(const Plan3Dev& p, const T* Q, int a, int fi, int fj, int fk, bool first_order_arg,
                                    T F[NV3_MAX]) {
@@ -452,7 +452,7 @@ __host__ __device__ void face_flux(const Plan3Dev& p, const T* Q, int a, int fi,
   }
   if constexpr (VISC && PART != 1) {
     T grad[3][5];
-    if constexpr (PART == 2) face_gradient_stored<T, SA ? 5 : 4>(p, Q, a, fi, fj, fk, grad);
+    if constexpr (PART >= 2) face_gradient_stored<T, SA ? 5 : 4>(p, qm, qp, a, fi, fj, fk, grad);
     else face_gradient<T, SA ? 5 : 4>(p, Q, a, fi, fj, fk, grad);
     // face means of the two cells either side
     T extra[3][3];
@@ -506,59 +506,47 @@ __host__ __device__ void face_flux(const Plan3Dev& p, const T* Q, int a, int fi,
 
 // The SA row's source at block cell c, times the volume: the production and destruction
 // with |curl V| and the c_b2 gradient term, both from Green-Gauss gradients of the face
-// means of (u, v, w, nu~) (src/jaxrans/numerics/turbulence.py).
+// means of (u, v, w, nu~) (src/jaxrans/numerics/turbulence.py).  The two faces of a family at a
+// time, in registers (with the means of all six kept in local memory the cell pass took 102 us
+// at 490k cells, 175 us on dual numbers; 67 and 93 us so).
 template <class T>
 __host__ __device__ T sa_cell_source(const Plan3Dev& p, const T* __restrict__ Q, int c) {
   const int i = c / (p.NJ * p.NK), j = (c / p.NK) % p.NJ, k = c % p.NK;
-  T lo_s[3][5], hi_s[3][5];   // face means of (u, v, w, nu~) for the cell's Green-Gauss gradients
-  for (int a = 0; a < 3; ++a) {
-    int lo[3] = {i, j, k}, hi[3] = {i, j, k};
-    lo[a] -= 1;
-    hi[a] += 1;
-    T qc[NV3_MAX], ql[NV3_MAX], qh[NV3_MAX];
-    load_cell_n<6>(p, Q, c, qc);
-    load_cell_n<6>(p, Q, cell_index(p, lo[0], lo[1], lo[2]), ql);
-    load_cell_n<6>(p, Q, cell_index(p, hi[0], hi[1], hi[2]), qh);
-    for (int m = 0; m < 3; ++m) {
-      lo_s[a][m] = 0.5 * (ql[1 + m] + qc[1 + m]);
-      hi_s[a][m] = 0.5 * (qc[1 + m] + qh[1 + m]);
-    }
-    lo_s[a][3] = 0.5 * (ql[5] + qc[5]);
-    hi_s[a][3] = 0.5 * (qc[5] + qh[5]);
-  }
   const Physics3& P = p.P;
-  const double vol = p.volume[c];
-  // Green-Gauss: (1/V) sum_families (phi_hi S_hi - phi_lo S_lo)[component]
-  T gv[3][3], gn[3];
-  for (int comp = 0; comp < 3; ++comp) {
-    T tv[3], tn = cst<T>(0.0);
-    for (int m = 0; m < 3; ++m) tv[m] = cst<T>(0.0);
-    for (int a = 0; a < 3; ++a) {
-      int f0[3] = {i, j, k}, f1[3] = {i, j, k};
-      f1[a] += 1;
-      double s0[3], s1[3];
-      face_vector(p, a, f0[0], f0[1], f0[2], s0);
-      face_vector(p, a, f1[0], f1[1], f1[2], s1);
-      for (int m = 0; m < 3; ++m) {
-        T d = hi_s[a][m] * s1[comp] - lo_s[a][m] * s0[comp];
-        tv[m] = a == 0 ? d : tv[m] + d;
+  const double vol = p.volume[c], g = P.gamma;
+  T qc[NV3_MAX], sum[3][4];   // [direction][u, v, w, nu~]: sums over the families of phi_hi S_hi - phi_lo S_lo
+  load_cell_n<6>(p, Q, c, qc);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    T ql[NV3_MAX], qh[NV3_MAX];
+    double s0[3], s1[3];
+    load_cell_n<6>(p, Q, cell_index(p, i - (a == 0), j - (a == 1), k - (a == 2)), ql);
+    load_cell_n<6>(p, Q, cell_index(p, i + (a == 0), j + (a == 1), k + (a == 2)), qh);
+    face_vector(p, a, i, j, k, s0);
+    face_vector(p, a, i + (a == 0), j + (a == 1), k + (a == 2), s1);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int row = m < 3 ? 1 + m : 5;
+      const T lo = 0.5 * (ql[row] + qc[row]), hi = 0.5 * (qc[row] + qh[row]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        if (m == d) continue;   // the curl takes no diagonal term
+        const T t = hi * s1[d] - lo * s0[d];
+        sum[d][m] = a == 0 ? t : sum[d][m] + t;
       }
-      T dn = hi_s[a][3] * s1[comp] - lo_s[a][3] * s0[comp];
-      tn = a == 0 ? dn : tn + dn;
     }
-    for (int m = 0; m < 3; ++m) gv[comp][m] = tv[m] / vol;   // gv[direction][component]
-    gn[comp] = tn / vol;
   }
-  T cx = gv[1][2] - gv[2][1], cy = gv[2][0] - gv[0][2], cz = gv[0][1] - gv[1][0];
-  T sq = (cx * cx + cy * cy) + cz * cz;
-  T omega = val(sq) > 0.0 ? dsqrt(sq) : cst<T>(0.0);
-  T qc[NV3_MAX];
-  load_cell(p, Q, c, qc);
-  const double g = P.gamma;
-  T mu = viscosity3(P, g * qc[4] / qc[0]);
+  // Green-Gauss: those sums over the volume
+  const T cx = sum[1][2] / vol - sum[2][1] / vol, cy = sum[2][0] / vol - sum[0][2] / vol;
+  const T cz = sum[0][1] / vol - sum[1][0] / vol;
+  const T gn[3] = {sum[0][3] / vol, sum[1][3] / vol, sum[2][3] / vol};
+  const T sq = (cx * cx + cy * cy) + cz * cz;
+  const T omega = val(sq) > 0.0 ? dsqrt(sq) : cst<T>(0.0);
+  const T mu = viscosity3(P, g * qc[4] / qc[0]);
   T Pr, Dd;
   sa_source(P.sa, qc[5] * P.mu_inf, mu / qc[0], omega, p.distance[c], Pr, Dd);
-  T src = qc[0] * ((Pr - Dd) / P.mu_inf + P.sa.c_b2 / P.sa.sigma * P.mu_inf * ((gn[0] * gn[0] + gn[1] * gn[1]) + gn[2] * gn[2]));
+  const T src = qc[0] * ((Pr - Dd) / P.mu_inf +
+                         P.sa.c_b2 / P.sa.sigma * P.mu_inf * ((gn[0] * gn[0] + gn[1] * gn[1]) + gn[2] * gn[2]));
   return src * vol;
 }
 
