@@ -17,6 +17,8 @@ static_assert(JR_STATUS_NONFINITE == ST_NONFINITE && JR_STATUS_REJECTED == ST_RE
               "the status bits of the C ABI are the device's");
 // residual.cu
 void launch_residual(const CaseDev*, const BatchDims&, int visc, bool second, int out_id, cudaStream_t);
+void launch_residual_of(const CaseDev*, const BatchDims&, int visc, bool second, const double* U, double* R,
+                        cudaStream_t);
 void launch_jvp(const CaseDev*, const BatchDims&, int visc, bool fp32, int tangent_id, int vdt_id, int out_id,
                 int check_active, int own_ghosts, cudaStream_t);
 void launch_ghosts(const CaseDev*, const BatchDims&, int tangent_id, int check_active, cudaStream_t);
@@ -400,6 +402,7 @@ static int build_buffers(jr_plan* p, const std::vector<size_t>& factor_rows) {
   for (int k = 0; k < nc; ++k) {
     CaseDev& cd = p->host[k];
     const size_t vo = p->vec_off[k], co = p->can_off[k], fo = p->face_off[k];
+    cd.vec_off = vo;
     double** mine[NVEC] = {&cd.U, &cd.qg, &cd.dqg, &cd.R, &cd.b, &cd.x, &cd.action, &cd.r, &cd.w, &cd.z, &cd.tmp};
     for (int v = 0; v < NVEC; ++v) *mine[v] = vec[v] + vo;
     cd.vdt = vdt + co;
@@ -739,12 +742,17 @@ int jr_synchronize(jr_plan* plan) {
 
 int jr_residual(jr_plan* plan, const double* U, double* R, int first_order) {
   if (!plan || !U || !R) return fail(JR_EINVAL, "null argument");
-  Adhoc a(plan);
-  a.vec(&CaseDev::U, U);
-  a.vec(&CaseDev::R, R);
-  const CaseDev* t = a.upload();
-  launch_ghosts(t, plan->dims, -1, 0, plan->st);
-  launch_residual(t, plan->dims, plan->visc, first_order == 0, B_R, plan->st);
+  // One launch on the plan's own table: the tiles evaluate their halos' ghosts.  A case with the
+  // point-vortex far field (its circulation a sum over the wall) has them filled by a launch,
+  // from a table that holds U.
+  bool vortex = false;
+  for (const CaseDev& cd : plan->host) vortex = vortex || cd.P.far_field == 1;
+  if (vortex) {
+    Adhoc a(plan);
+    a.vec(&CaseDev::U, U);
+    launch_ghosts(a.upload(), plan->dims, -1, 0, plan->st);
+  }
+  launch_residual_of(plan->cases, plan->dims, plan->visc, first_order == 0, U, R, plan->st);
   return cuda_check("jr_residual");
 }
 

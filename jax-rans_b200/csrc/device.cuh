@@ -120,6 +120,7 @@ struct CaseDev {
   Canvas c;
   Physics P;
   Config cfg;
+  size_t vec_off;           // where the case's entries start in a vector over the whole batch
   double *U, *qg, *dqg, *R, *b, *x, *action, *r, *w, *z, *tmp, *vdt, *dflow, *dsa, *lam, *mflux, *dflux;
   double *tile_partial, *history, *force_out;
   void* jac;                // the linearisation: per face coefficient planes of jstride values

@@ -176,6 +176,32 @@ __device__ __forceinline__ void eval_record(const Canvas& c, const Physics& P, i
   }
 }
 
+// the state ghost record t gives (a stage-1 index, or n_ghost[0] + a stage-2 index): a stage-2
+// record whose source is a stage-1 ghost (a corner) evaluates that record itself
+template <class T>
+__device__ __forceinline__ void ghost_state(const Canvas& c, const Physics& P, int t, const double* U,
+                                            const double* V, const double* qg, const double* dqg, T circ, T* out) {
+  const int n0 = c.n_ghost[0];
+  const int s = t < n0 ? 0 : 1, r = t < n0 ? t : t - n0;
+  T q[5];
+  const int r1 = s == 1 ? c.g_src_rec[r] : -1;
+  if (r1 >= 0) {
+    T q1[5];
+    load_prim<T>(c, P, c.g_source[0][r1], U, V, qg, dqg, q1);
+    eval_record<T>(c, P, 0, r1, q1, circ, q);
+  } else {
+    load_prim<T>(c, P, c.g_source[s][r], U, V, qg, dqg, q);
+  }
+  eval_record<T>(c, P, s, r, q, circ, out);
+}
+
+// the same for a tile's halo, out of line: a few threads of the boundary tiles call it, and
+// inlined it would set the tile kernel's registers
+__device__ __noinline__ void tile_ghost(const Canvas& c, const Physics& P, int t, const double* U, const double* qg,
+                                        double* out) {
+  ghost_state<double>(c, P, t, U, nullptr, qg, nullptr, 0.0, out);
+}
+
 // Both stages in one launch: a stage-2 record whose source is a stage-1 ghost (a
 // corner) evaluates that stage-1 record itself rather than reading it, so no record
 // waits on another and every CTA works independently.
@@ -264,16 +290,8 @@ __global__ void __launch_bounds__(GHOST_THREADS) k_ghosts(const CaseDev* __restr
   const int n0 = c.n_ghost[0], total = n0 + c.n_ghost[1];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     const int s = t < n0 ? 0 : 1, r = t < n0 ? t : t - n0;
-    T q[5], out[5];
-    const int r1 = s == 1 ? c.g_src_rec[r] : -1;
-    if (r1 >= 0) {
-      T q1[5];
-      load_prim<T>(c, P, c.g_source[0][r1], U, V, qg, dqg, q1);
-      eval_record<T>(c, P, 0, r1, q1, circ, q);
-    } else {
-      load_prim<T>(c, P, c.g_source[s][r], U, V, qg, dqg, q);
-    }
-    eval_record<T>(c, P, s, r, q, circ, out);
+    T out[5];
+    ghost_state<T>(c, P, t, U, V, qg, dqg, circ, out);
     const int ghost = c.g_ghost[s][r];
     for (int v = 0; v < c.nvar; ++v) {
       if constexpr (sizeof(T) == sizeof(Dual)) {
@@ -583,7 +601,8 @@ template <> __device__ __forceinline__ double tangent_or_value<Dual>(const Dual&
 // scalar (double).
 template <class T, int NV, bool SECOND, int VISC>
 __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
-    k_residual(const CaseDev* __restrict__ cases, int out_id, int with_partial, int check_active) {
+    k_residual(const CaseDev* __restrict__ cases, const double* U_batch, double* R_batch, int out_id, int with_partial,
+               int check_active) {
   __shared__ CaseDev scase;
   if (idle_block(cases[blockIdx.z],
                  (int)blockIdx.x >= cases[blockIdx.z].tiles_x || (int)blockIdx.y >= cases[blockIdx.z].tiles_y,
@@ -594,22 +613,37 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
   if ((int)blockIdx.x >= cd.tiles_x || (int)blockIdx.y >= cd.tiles_y) return;
   const Canvas& c = cd.c;
   const Physics& P = cd.P;
-  const double* __restrict__ U = cd.U;
+  const double* __restrict__ U = U_batch != nullptr ? U_batch + cd.vec_off : cd.U;
   const double* __restrict__ qg = cd.qg;
-  double* __restrict__ out = buf(cd, out_id);
+  double* __restrict__ out = R_batch != nullptr ? R_batch + cd.vec_off : buf(cd, out_id);
   double* __restrict__ partial = with_partial ? cd.tile_partial : nullptr;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TileSmem<T, NV>& s = *reinterpret_cast<TileSmem<T, NV>*>(smem_raw);
   const int NI = c.NI, NJ = c.NJ, N = c.ncanvas();
   const int i0 = blockIdx.y * TILE_I, j0 = blockIdx.x * TILE_J;
   const int tid = threadIdx.x;
+  // The tile's own ghosts, listed by the staging and then evaluated a thread each: in place they
+  // would be two long chains one after the other (a condition's loads, roots and quotients).  A
+  // call on a batch-long U is one launch so, without a ghost fill or a table of its own: 47.8 ->
+  // 44.4 us a call on a 65 x 17 Euler grid, 59.8 -> 55.0 us on a 385 x 97 SA grid, most of it the
+  // host's; in the Newton step the linearisation needs the filled ghosts anyway.
+  const bool own = U_batch != nullptr && P.far_field != 1;
+  __shared__ int n_own, own_list[HI * HJ];
+  if (tid == 0) n_own = 0;
+  if (own) __syncthreads();
   // 1. stage the primitive state of the tile and its halo
   for (int e = tid; e < HI * HJ; e += TILE_THREADS) {
     int li = e / HJ, lj = e % HJ;
     int i = i0 - 2 + li, j = j0 - 2 + lj;
     T q[5];
     if (i >= 0 && i < NI && j >= 0 && j < NJ) {
-      load_prim_n<NV, T>(c, P, i * NJ + j, U, nullptr, qg, nullptr, q);
+      const int idx = i * NJ + j;
+      const int rec = own && !c.interior[idx] ? c.ghost_rec[idx] : -1;
+      if (rec >= 0) {
+        own_list[atomicAdd(&n_own, 1)] = rec * 256 + e;
+        continue;
+      }
+      load_prim_n<NV, T>(c, P, idx, U, nullptr, qg, nullptr, q);
     } else {
       for (int v = 0; v < NV; ++v) q[v] = cst<T>(1.0);
     }
@@ -623,6 +657,15 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
       int ci = min(max(i + 1, 0), CI - 1), cj = min(max(j + 1, 0), CJ - 1);
       s.cx[li][lj] = c.centres[ci * CJ + cj];
       s.cy[li][lj] = c.centres[CI * CJ + ci * CJ + cj];
+    }
+  }
+  if (own) {
+    __syncthreads();
+    for (int t = tid; t < n_own; t += TILE_THREADS) {
+      const int rec = own_list[t] / 256, e = own_list[t] % 256;
+      double q[5];
+      tile_ghost(c, P, rec, U, qg, q);
+      for (int v = 0; v < NV; ++v) s.q[v][e / HJ][e % HJ] = q[v];
     }
   }
   __syncthreads();
@@ -1402,25 +1445,38 @@ void configure_kernels() {
 // One launch over every case of a batch: grid z = the case, x/y = the tiles (a case
 // with fewer tiles returns at once from the excess ones).
 template <class T, int NV, bool SECOND, int VISC>
-static void launch_tile(const CaseDev* cases, const BatchDims& d, int out_id, int with_partial, int check_active,
-                        cudaStream_t st) {
+static void launch_tile(const CaseDev* cases, const BatchDims& d, const double* U, double* R, int out_id,
+                        int with_partial, int check_active, cudaStream_t st) {
   dim3 grid(d.tiles_x, d.tiles_y, d.n_cases);
-  k_residual<T, NV, SECOND, VISC><<<grid, TILE_THREADS, sizeof(TileSmem<T, NV>), st>>>(cases, out_id, with_partial,
-                                                                                     check_active);
+  k_residual<T, NV, SECOND, VISC><<<grid, TILE_THREADS, sizeof(TileSmem<T, NV>), st>>>(cases, U, R, out_id,
+                                                                                     with_partial, check_active);
+}
+
+static void residual_of(const CaseDev* cases, const BatchDims& d, int visc, bool second, const double* U, double* R,
+                        int out_id, cudaStream_t st) {
+  if (visc == 2) {
+    if (second) launch_tile<double, 5, true, 2>(cases, d, U, R, out_id, 1, 0, st);
+    else launch_tile<double, 5, false, 2>(cases, d, U, R, out_id, 1, 0, st);
+  } else if (visc == 1) {
+    if (second) launch_tile<double, 4, true, 1>(cases, d, U, R, out_id, 1, 0, st);
+    else launch_tile<double, 4, false, 1>(cases, d, U, R, out_id, 1, 0, st);
+  } else {
+    if (second) launch_tile<double, 4, true, 0>(cases, d, U, R, out_id, 1, 0, st);
+    else launch_tile<double, 4, false, 0>(cases, d, U, R, out_id, 1, 0, st);
+  }
 }
 
 // R(U) of every case into `out_id` (second or first order), with the norm partials
 void launch_residual(const CaseDev* cases, const BatchDims& d, int visc, bool second, int out_id, cudaStream_t st) {
-  if (visc == 2) {
-    if (second) launch_tile<double, 5, true, 2>(cases, d, out_id, 1, 0, st);
-    else launch_tile<double, 5, false, 2>(cases, d, out_id, 1, 0, st);
-  } else if (visc == 1) {
-    if (second) launch_tile<double, 4, true, 1>(cases, d, out_id, 1, 0, st);
-    else launch_tile<double, 4, false, 1>(cases, d, out_id, 1, 0, st);
-  } else {
-    if (second) launch_tile<double, 4, true, 0>(cases, d, out_id, 1, 0, st);
-    else launch_tile<double, 4, false, 0>(cases, d, out_id, 1, 0, st);
-  }
+  residual_of(cases, d, visc, second, nullptr, nullptr, out_id, st);
+}
+
+// the same at U, into R: vectors over the whole batch in place of the table's own.  The tiles
+// evaluate their halos' ghosts, so none need have been filled, but for a case with the
+// point-vortex far field.
+void launch_residual_of(const CaseDev* cases, const BatchDims& d, int visc, bool second, const double* U, double* R,
+                        cudaStream_t st) {
+  residual_of(cases, d, visc, second, U, R, B_NONE, st);
 }
 
 // The linearisation of every case's first-order residual at its U (ghosts of U filled);
