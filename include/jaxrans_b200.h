@@ -349,8 +349,10 @@ int jr_precondition3d(jr_plan3d* plan, const double* U, double cfl, const double
  * n_steps) receives |R| before each step.  GMRES(krylov_subspace) with krylov_restarts
  * cycles, CGS2, Givens least squares, the relaxation, acceptance test and CFL ramp of
  * src/jaxrans/solvers/implicit.py:54-168, driven from the host over device kernels (it
- * synchronises for the scalars: three times per Arnoldi step).  Replaces make_newton_step run as the
- * driver's block on a 3D atlas. */
+ * synchronises once per Krylov cycle and for the step's own scalars).  The products use one
+ * linearisation per step, whose factors (about 2 KB a cell with SA) the plan's first step
+ * allocates; without the memory for them, jr_jvp3d's kernels.  Replaces make_newton_step run
+ * as the driver's block on a 3D atlas. */
 int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, double* residual_norm,
                       double* history);
 /* Force coefficients of a 3D case at U (device): out (host, 4) = cl, cd, cm, cd_friction
