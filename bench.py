@@ -50,7 +50,7 @@ METRIC = "converged RANS solves/hr"
 # Newton steps of one converged solve of each workload from the freestream (FP64): the
 # device path's own count (the bench line's config.newton_steps_per_solve, which it
 # measures every run); the CPU samples, a few Newton steps each, are scaled by it.
-STEPS_PER_SOLVE = {"c_sa_385": 680, "o_euler_257": 3840}
+STEPS_PER_SOLVE = {"c_sa_385": 620, "o_euler_257": 3840}
 # coefficients of the linearisation the J.v tile reads per face and per cell (the
 # kernel's JacShape and JCELL): inviscid 4 x 4 per side, the SA convection's 3, the
 # viscous tail's derivatives its dependences allow (19 laminar, 33 SA)
