@@ -159,7 +159,6 @@ __global__ void k3_wall_loads(Plan3Dev p, const double* __restrict__ Q, double* 
 
 // the loads on every wall face (7 each) at U: the primitive canvas ghost-filled first
 void launch_wall_loads3(const Plan3Dev& p, const double* U, double* loads, void* A, cudaStream_t st) {
-  const int n = p.NI * p.NJ * p.NK;
   counted3(p.n_walls > 0);
   canvas3<double>(p, U, nullptr, (double*)A, st);
   if (p.n_walls > 0) k3_wall_loads<<<(p.n_walls + 127) / 128, 128, 0, st>>>(p, (const double*)A, loads);
