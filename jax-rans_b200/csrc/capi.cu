@@ -456,6 +456,7 @@ static BatchDims dims_of(const std::vector<CaseDev>& cases, int n_slots) {
     const Canvas& c = cd.c;
     d.tiles_x = std::max(d.tiles_x, cd.tiles_x);
     d.tiles_y = std::max(d.tiles_y, cd.tiles_y);
+    d.tiles += cd.n_tiles;
     d.ghost_records = std::max(d.ghost_records, c.n_ghost[0] + c.n_ghost[1]);
     d.faces = std::max(d.faces, (c.NI + 1) * c.NJ + c.NI * (c.NJ + 1));
     d.cells = std::max(d.cells, c.NI * c.NJ);

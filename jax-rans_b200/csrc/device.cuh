@@ -184,6 +184,7 @@ struct BatchDims {
   int n_cases;              // cases in the launch's table
   int n_slots;              // cases of the plan (the history's row length)
   int tiles_x, tiles_y;     // residual tiles
+  int tiles;                // ... of all the cases together
   int ghost_records;        // both stages
   int faces, cells;         // canvas faces, canvas cells
   int n_vec;                // nvar * cells

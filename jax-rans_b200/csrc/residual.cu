@@ -1027,9 +1027,8 @@ __device__ __forceinline__ void load_inviscid_ahead(const double* jf, size_t str
   for (int k = 0; k < 32; ++k) asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(A[k]) : "l"(jf + k * stride));
 }
 
-template <int NV, class TJ>
-__device__ __forceinline__ void jv_inviscid(const JvSmem<NV>& s, int axis, int ai, int aj, const TJ (&A)[32],
-                                            double* dF) {
+template <int NV, class COEF>
+__device__ __forceinline__ void jv_inviscid(const JvSmem<NV>& s, int axis, int ai, int aj, COEF coef, double* dF) {
   const int bi = ai + (axis == 0 ? 1 : 0), bj = aj + (axis == 0 ? 0 : 1);
   double a[4], b[4];
 #pragma unroll
@@ -1041,9 +1040,9 @@ __device__ __forceinline__ void jv_inviscid(const JvSmem<NV>& s, int axis, int a
   for (int r = 0; r < 4; ++r) {
     double acc = 0.0;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc += double(A[4 * r + v]) * a[v];
+    for (int v = 0; v < 4; ++v) acc += coef(4 * r + v) * a[v];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) acc += double(A[16 + 4 * r + v]) * b[v];
+    for (int v = 0; v < 4; ++v) acc += coef(16 + 4 * r + v) * b[v];
     dF[r] = acc;
   }
 }
@@ -1085,9 +1084,9 @@ __device__ __forceinline__ void jv_viscous(const JvSmem<NV>& s, int axis, int ai
 // out = vdt * v + dR1/dU . v with v = buffer `tangent_id` (vdt_id < 0: the bare J.v),
 // from the case's linearisation; own_ghosts: the tile evaluates its halo's tangent
 // ghosts (no tangent ghost fill needed)
-template <int NV, int VISC, class TJ>
-__global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__ cases, int out_id, int tangent_id,
-                                                     int vdt_id, int check_active, int own_ghosts) {
+template <int NV, int VISC, class TJ, bool AHEAD>
+__device__ __forceinline__ void jv_tile(const CaseDev* __restrict__ cases, int out_id, int tangent_id, int vdt_id,
+                                        int check_active, int own_ghosts) {
   __shared__ CaseDev scase;
   if (idle_block(cases[blockIdx.z],
                  (int)blockIdx.x >= cases[blockIdx.z].tiles_x || (int)blockIdx.y >= cases[blockIdx.z].tiles_y,
@@ -1111,12 +1110,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__
   const int i0 = blockIdx.y * TILE_I, j0 = blockIdx.x * TILE_J;
   const int tid = threadIdx.x;
   const int nfi = c.nfi();
-  // This thread's i-face (8 x 16 of them) and j-face (7 x 17).  FP64 coefficients are loaded ahead:
-  // the i-face's while the tile is staged, the j-face's while the i-face's viscous part is summed,
-  // so each face waits for one round of loads less.  On a 385 x 97 case in the Newton step's graph
-  // 23.2 -> 20.0 us (back to back, its coefficients in L2: 18.6 both ways).  FP32 coefficients are
-  // not: with the registers for it a block an SM fewer is resident (769 x 193: 59 -> 67 us).
-  constexpr bool AHEAD = sizeof(TJ) == sizeof(double);
+  // This thread's i-face (8 x 16 of them) and j-face (7 x 17).  AHEAD: the i-face's coefficients are
+  // loaded while the tile is staged, the j-face's while the i-face's viscous part is summed.
   static_assert((TILE_I + 1) * TILE_J == TILE_THREADS && TILE_I * (TILE_J + 1) <= TILE_THREADS, "a face a thread");
   const int fi_i = tid / TILE_J, fi_j = tid % TILE_J, fj_i = tid / (TILE_J + 1), fj_j = tid % (TILE_J + 1);
   const bool live_i = j0 + fi_j < NJ && (interior_at(c, i0 + fi_i - 1, j0 + fi_j) || interior_at(c, i0 + fi_i, j0 + fi_j));
@@ -1179,8 +1174,12 @@ __global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__
 #pragma unroll
   for (int v = 0; v < NV; ++v) dF[v] = 0.0;
   if (live_i) {
-    if constexpr (!AHEAD) load_inviscid(jac_i, stride, A);
-    jv_inviscid<NV, TJ>(s, 0, fi_i, fi_j + 1, A, dF);
+    if constexpr (AHEAD || sizeof(TJ) == 4) {
+      if constexpr (!AHEAD) load_inviscid(jac_i, stride, A);
+      jv_inviscid<NV>(s, 0, fi_i, fi_j + 1, [&](int k) { return double(A[k]); }, dF);
+    } else {
+      jv_inviscid<NV>(s, 0, fi_i, fi_j + 1, [&](int k) { return double(jac_i[k * stride]); }, dF);
+    }
   }
   if constexpr (AHEAD)
     if (live_j) load_inviscid_ahead(jac_j, stride, A);
@@ -1192,8 +1191,12 @@ __global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__
 #pragma unroll
     for (int v = 0; v < NV; ++v) dF[v] = 0.0;
     if (live_j) {
-      if constexpr (!AHEAD) load_inviscid(jac_j, stride, A);
-      jv_inviscid<NV, TJ>(s, 1, fj_i + 1, fj_j, A, dF);
+      if constexpr (AHEAD || sizeof(TJ) == 4) {
+        if constexpr (!AHEAD) load_inviscid(jac_j, stride, A);
+        jv_inviscid<NV>(s, 1, fj_i + 1, fj_j, [&](int k) { return double(A[k]); }, dF);
+      } else {
+        jv_inviscid<NV>(s, 1, fj_i + 1, fj_j, [&](int k) { return double(jac_j[k * stride]); }, dF);
+      }
       jv_viscous<NV, VISC, TJ>(s, 1, fj_i + 1, fj_j, jac_j, stride, dF);
     }
 #pragma unroll
@@ -1246,6 +1249,23 @@ __global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__
     }
   }
 }
+
+// FP32 coefficients, and FP64 ones loaded ahead (no viscous SA terms)
+template <int NV, int VISC, class TJ>
+__global__ void __launch_bounds__(TILE_THREADS) k_jv(const CaseDev* __restrict__ cases, int out_id, int tangent_id,
+                                                     int vdt_id, int check_active, int own_ghosts) {
+  jv_tile<NV, VISC, TJ, sizeof(TJ) == sizeof(double)>(cases, out_id, tangent_id, vdt_id, check_active, own_ghosts);
+}
+
+// FP64 coefficients loaded where they are used, at as many blocks an SM as that leaves registers for
+constexpr int jv_blocks(int visc) { return visc == 2 ? 4 : (visc == 1 ? 5 : 6); }
+template <int NV, int VISC>
+__global__ void __launch_bounds__(TILE_THREADS, jv_blocks(VISC))
+    k_jv_full(const CaseDev* __restrict__ cases, int out_id, int tangent_id, int vdt_id, int check_active,
+              int own_ghosts) {
+  jv_tile<NV, VISC, double, false>(cases, out_id, tangent_id, vdt_id, check_active, own_ghosts);
+}
+
 // ------------------------------------------------------------------------------------
 // Wave speeds and the per-face terms of the preconditioner (residual.py:169-203,
 // preconditioners.py:557-563): lambda from face-averaged states (a block face's
@@ -1422,13 +1442,17 @@ template <class TJ> static void configure_lin() {
                        (int)sizeof(TileSmem<double, 4>));
   cudaFuncSetAttribute(k_linearize<4, 0, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(TileSmem<double, 4>));
-  cudaFuncSetAttribute(k_jv<5, 2, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<5>));
+  if constexpr (sizeof(TJ) == sizeof(float))
+    cudaFuncSetAttribute(k_jv<5, 2, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<5>));
   cudaFuncSetAttribute(k_jv<4, 1, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
   cudaFuncSetAttribute(k_jv<4, 0, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
 }
 
 // the tile kernels' dynamic shared memory limits, set once before any launch or capture
 void configure_kernels() {
+  cudaFuncSetAttribute(k_jv_full<5, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<5>));
+  cudaFuncSetAttribute(k_jv_full<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
+  cudaFuncSetAttribute(k_jv_full<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
   static bool done = false;
   if (done) return;
   configure_one<double, 5, true, 2>();
@@ -1502,19 +1526,38 @@ void launch_linearize(const CaseDev* cases, const BatchDims& d, int visc, bool f
 // every product and sum in double); own_ghosts: the tiles map their halo's tangent ghosts
 // through the linearisation's ghost maps, but in a case with the point-vortex far field,
 // whose tangent ghosts a ghost fill (launch_ghosts) must provide
+// FP64 coefficients: the two forms give the same bits.  Loading ahead saves a face one wait, and
+// costs registers (152 and 158, three blocks an SM; 80 and 96 without, six and five): it pays while
+// every tile of the launch is resident at three blocks an SM.  A Newton step of GMRES(10), ahead
+// and not: a 257 x 65 Euler case (190 tiles) 896 and 925 us, two of them 1.07 and 1.09 ms, four 1.88
+// and 1.78 ms, a 513 x 129 one (666 tiles) 1.55 and 1.48 ms; a 137 x 38 laminar case (GMRES(15)) 702 and
+// 707 us, eight 2.22 and 2.12 ms.  With the SA terms it never does (168 registers against 128, four
+// blocks): GMRES(30) on 385 x 97 2.51 and 2.48 ms, eight of them 14.8 and 14.2 ms, 769 x 193 7.25 and
+// 6.88 ms.
+constexpr int JV_AHEAD_TILES = 3 * 148;
+
+template <int NV, int VISC, class TJ>
+static void jvp_of(const CaseDev* cases, const BatchDims& d, int tangent_id, int vdt_id, int out_id, int check_active,
+                   int own_ghosts, cudaStream_t st) {
+  const dim3 grid(d.tiles_x, d.tiles_y, d.n_cases);
+  if constexpr (sizeof(TJ) == sizeof(double)) {
+    if (VISC == 2 || d.tiles > JV_AHEAD_TILES) {
+      k_jv_full<NV, VISC><<<grid, TILE_THREADS, sizeof(JvSmem<NV>), st>>>(cases, out_id, tangent_id, vdt_id,
+                                                                          check_active, own_ghosts);
+      return;
+    }
+  }
+  if constexpr (sizeof(TJ) == sizeof(float) || VISC < 2)
+    k_jv<NV, VISC, TJ><<<grid, TILE_THREADS, sizeof(JvSmem<NV>), st>>>(cases, out_id, tangent_id, vdt_id, check_active,
+                                                                       own_ghosts);
+}
+
 template <class TJ>
 static void jvp_t(const CaseDev* cases, const BatchDims& d, int visc, int tangent_id, int vdt_id, int out_id,
                   int check_active, int own_ghosts, cudaStream_t st) {
-  dim3 grid(d.tiles_x, d.tiles_y, d.n_cases);
-  if (visc == 2)
-    k_jv<5, 2, TJ><<<grid, TILE_THREADS, sizeof(JvSmem<5>), st>>>(cases, out_id, tangent_id, vdt_id, check_active,
-                                                                  own_ghosts);
-  else if (visc == 1)
-    k_jv<4, 1, TJ><<<grid, TILE_THREADS, sizeof(JvSmem<4>), st>>>(cases, out_id, tangent_id, vdt_id, check_active,
-                                                                  own_ghosts);
-  else
-    k_jv<4, 0, TJ><<<grid, TILE_THREADS, sizeof(JvSmem<4>), st>>>(cases, out_id, tangent_id, vdt_id, check_active,
-                                                                  own_ghosts);
+  if (visc == 2) jvp_of<5, 2, TJ>(cases, d, tangent_id, vdt_id, out_id, check_active, own_ghosts, st);
+  else if (visc == 1) jvp_of<4, 1, TJ>(cases, d, tangent_id, vdt_id, out_id, check_active, own_ghosts, st);
+  else jvp_of<4, 0, TJ>(cases, d, tangent_id, vdt_id, out_id, check_active, own_ghosts, st);
 }
 
 void launch_jvp(const CaseDev* cases, const BatchDims& d, int visc, bool fp32, int tangent_id, int vdt_id,

@@ -1,0 +1,47 @@
+"""The FP64 kernels that take one of two forms by how many cases a launch holds: the J.v tile
+(coefficients loaded ahead while every tile is resident, or where they are used).  A case's
+history and state are bitwise the same whichever form its launch took, for each model's
+instances and on grids whose edges cut the tiles."""
+
+from __future__ import annotations
+
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from jaxrans_b200.case import parse_case
+from jaxrans_b200.solver import freestream_state
+
+pytestmark = pytest.mark.gpu
+
+CASES = 6   # 6 x 76 tiles of the J.v: more than are resident at once; alone they all are
+
+
+@pytest.mark.parametrize("model,subspace", [("euler", 10), ("laminar", 10), ("sa", 10)])
+def test_a_batch_past_the_rule_is_bitwise_the_cases_alone(cuda, model, subspace):
+    from jaxrans_b200.native import DevicePlan
+    euler = model == "euler"
+    case = parse_case({"general": {"case_name": "forms"},
+                       "domain": {"grid": "o_grid", "airfoil": "naca0012", "cells_airfoil": 126, "cells_normal": 46,
+                                  "wall_spacing": 1e-3, "far_field": 20.0},
+                       "boundary_conditions": {"wall": {"type": "slip_wall" if euler else "no_slip_wall"},
+                                               "farfield": {"type": "far_field"}},
+                       "freestream": {"mach": 0.5, "alpha_deg": 2.0, **({} if euler else {"reynolds": 1e5})},
+                       **({"turbulence": {"model": "sa_noft2"}} if model == "sa" else {})},
+                      {"convective_fluxes": {"riemann_solver": "hllc", "limiter": "van_albada"},
+                       "time_integration": {"solver": "implicit"},
+                       "implicit": {"krylov_subspace": subspace, "krylov_restarts": 1, "max_relative_update": 0.2}})
+    plan = case.grid()
+    flows = [replace(case.flow, alpha_deg=float(a)) for a in np.linspace(-2.0, 4.0, CASES)]
+    states = [freestream_state(replace(case, flow=f), plan) for f in flows]
+    batch = DevicePlan.batch(plan, flows, case.numerics, case.implicit)
+    batch.set_state(np.concatenate([u.ravel() for u in states]), 5.0)
+    hist = batch.newton_steps(4)
+    for k in (0, 2, CASES - 1):
+        one = DevicePlan(plan, flows[k], case.numerics, case.implicit)
+        one.set_state(states[k], 5.0)
+        assert np.array_equal(hist[:, k], one.newton_steps(4))
+        assert np.array_equal(batch.case_state(k)[0], one.get_state()[0])
+        one.close()
+    batch.close()
