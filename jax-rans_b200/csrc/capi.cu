@@ -464,6 +464,8 @@ static BatchDims dims_of(const std::vector<CaseDev>& cases, int n_slots) {
     d.chain_blocks = std::max(d.chain_blocks, chain_grid_blocks(c.n_chains, c.n_offchain));
     d.max_L = std::max(d.max_L, c.L);
     d.cgs_blocks = std::max(d.cgs_blocks, cgs_blocks(cd.n_vec));
+    d.orth_total += orth_blocks(cd.n_vec);
+    d.orth_chunk = std::max(d.orth_chunk, orth_chunk(cd.n_vec));
   }
   d.chain_blocks = std::max(d.chain_blocks, 1);
   d.ls_factor_threads = 128;

@@ -191,6 +191,8 @@ struct BatchDims {
   int chain_blocks;         // chains + off-chain blocks of the line solve
   int max_L;                // longest chain
   int cgs_blocks;           // blocks of the FP32 basis passes
+  int orth_total;           // blocks of the FP64 basis passes, of all the cases together
+  int orth_chunk;           // ... and the longest of the cases' chunks
   int ls_factor_threads;    // threads per chain of the line factor and of the line solve:
   int ls_apply_threads;     // the schedule the plan's autotuner picked (results do not depend on it)
   int ls_apply_stage;       // s >= 1: the line solve stages its factor from level s-1 of the longest chain
@@ -210,10 +212,17 @@ __host__ __device__ __forceinline__ int cgs_chunk(int n) {
 __host__ __device__ __forceinline__ int cgs_blocks(int n) { return (n + cgs_chunk(n) - 1) / cgs_chunk(n); }
 
 // The FP64 basis passes: blocks of a case of n unknowns, set by its size alone (so its sums are the
-// same in any batch): one an SM, fewer where that leaves a thread without an element.
+// same in any batch): one an SM, fewer where that leaves a block fewer than 512 elements (at 256,
+// twice the blocks for the same sums: eight 137 x 38 laminar cases, GMRES(15), 37 against 31 us; one
+// 105 x 31 case gains a microsecond of 26 by it).
 __host__ __device__ __forceinline__ int orth_blocks(int n) {
-  const int b = (n + 255) / 256;
+  const int b = (n + 511) / 512;
   return b < 1 ? 1 : (b > 148 ? 148 : b);
+}
+// the elements a block owns, in whole rounds of ORTH_ROUND (orth.cuh)
+__host__ __device__ __forceinline__ int orth_chunk(int n) {
+  const int per = (n + orth_blocks(n) - 1) / orth_blocks(n);
+  return (per + 511) / 512 * 512;
 }
 
 // the number of blocks a per-case reduction over n elements uses (<= the grid's x)

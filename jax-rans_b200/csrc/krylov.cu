@@ -190,12 +190,17 @@ __global__ void k_cycle_gate(const CaseDev* __restrict__ cases, int n_cases, cud
 
 // The three passes of CGS2 over an FP64 basis: h1 = V^T w; w -= V h1, then h2 = V^T w; w -= V h2,
 // then |w| and column j of H.  A block owns a contiguous part of a case (orth_blocks(n) of
-// them, at most one an SM); a thread holds its E elements' entries of every vector in
-// registers, so the second pass updates w and takes its dots from one read of the basis, and
-// NK x E loads a thread are in flight.  On one 385 x 97 case (194k unknowns) a pass is its
-// latency: launch, a few rounds of loads, the sums' two stages; the three over 30 vectors take
-// 39 us, 135 us on a 769 x 193 case (a warp a vector over 512- to 2048-element chunks, the
-// second pass reading the basis twice: 55 and 188 us).
+// them, at most one an SM).  Two forms of the first two passes give the same bits: every dot
+// product is a thread's elements in order, its warp's lanes by halves, the block's eight warps and
+// the blocks in order.
+//
+// Few blocks (k_orth_dots): a thread holds its E elements' entries of every vector in registers,
+// so the second pass updates w and takes its dots from one read of the basis, and NK x E loads a
+// thread are in flight.  On one 385 x 97 case (194k unknowns) a pass is its latency: launch, a few
+// rounds of loads, the sums' two stages; the three over 8, 15 and 30 vectors take 25, 29 and 37 us, on a
+// 769 x 193 case 35, 58 and 134 us (a warp a vector, the second pass reading the basis twice: 29, 38 and
+// 54 us; 45, 76 and 189 us).  E by those two cases: at one element a thread the 769 x 193 case takes 37
+// and 65 us over 8 and 15 vectors, over 30 the same (and two would spill).
 
 // The dots of the NK vectors from k0 (nk of them) with w, after (UPDATE) w -= sum h V over the
 // same vectors.  second: h1 in, h2 out; else h1 out.
@@ -254,10 +259,85 @@ __global__ void __launch_bounds__(ORTH_THREADS, NK <= 8 ? 2 : 1)
     hout[threadIdx.x] = total[threadIdx.x];
 }
 
+// Many blocks, each with few elements (k_orth_dots_dense): in the form above one block is all an
+// SM holds, so the blocks' loads and sums follow one another, and of a thread's work on two elements
+// the sums over its warp are most.  Here w (updated, for UPDATE, from a first read of the
+// block's part of the basis, which its dots then find in L1 or L2) lies in shared memory, and a warp
+// takes a vector, its lanes the elements of all eight warps of the form above, a sum each: 9
+// shuffles a vector in place of 31 for 32 sums in each of eight warps.  Four blocks an SM.
+template <int NK, bool UPDATE>
+__global__ void __launch_bounds__(ORTH_THREADS, 4)
+    k_orth_dots_dense(const CaseDev* __restrict__ cases, int k0, int nk, int second) {
+  const CaseDev& cd = cases[blockIdx.y];
+  if (!cd.enabled) return;
+  Scalars* sc = cd.sc;
+  if (sc->active == 0) return;
+  const int n = cd.n_vec, nb = orth_blocks(n);
+  if ((int)blockIdx.x >= nb) return;
+  const size_t ldv = (size_t)n;
+  const double* __restrict__ V = (const double*)cd.V + (size_t)k0 * ldv;
+  double* __restrict__ w = cd.w;
+  double* hout = (second ? sc->h2 : sc->h1) + k0;
+  extern __shared__ double ws[];   // the block's part of w, zeros to a whole round
+  __shared__ double h[NK], total[NK];
+  if (UPDATE) {
+    if ((int)threadIdx.x < NK) h[threadIdx.x] = (int)threadIdx.x < nk ? sc->h1[k0 + threadIdx.x] : 0.0;
+    __syncthreads();
+  }
+  int lo, hi;
+  chunk(n, nb, lo, hi);
+  const int len = hi - lo, padded = (len + ORTH_ROUND - 1) / ORTH_ROUND * ORTH_ROUND;
+  for (int e = threadIdx.x; e < padded; e += ORTH_THREADS) {
+    double x = 0.0;
+    if (e < len) {
+      x = w[lo + e];
+      if (UPDATE) {
+        constexpr int KB = 8;
+        double s = 0.0;
+#pragma unroll
+        for (int b = 0; b < NK; b += KB) {
+          double v[KB];
+#pragma unroll
+          for (int k = 0; k < KB; ++k) v[k] = V[(size_t)min(b + k, nk - 1) * ldv + lo + e];   // (no branch: all in flight)
+#pragma unroll
+          for (int k = 0; k < KB; ++k)
+            if (b + k < nk) s += h[b + k] * v[k];
+        }
+        x -= s;
+        w[lo + e] = x;
+      }
+    }
+    ws[e] = x;
+  }
+  __syncthreads();
+  constexpr int NW = ORTH_THREADS / 32, NV = ORTH_ROUND / 32;
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < nk; k += NW) {
+    const double* __restrict__ vk = V + k * ldv + lo;
+    double a[NW] = {};
+    for (int e = lane; e < padded; e += ORTH_ROUND) {
+      double v[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) v[q] = e + 32 * q < len ? vk[e + 32 * q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < NV; ++q) a[q % NW] += v[q] * ws[e + 32 * q];
+    }
+    lane_sums<NW>(a, lane);
+    double s = __shfl_sync(0xffffffffu, a[0], 0);
+#pragma unroll
+    for (int q = 1; q < NW; ++q) s += __shfl_sync(0xffffffffu, a[0], q * (32 / NW));
+    if (lane == 0) cd.partial[(size_t)blockIdx.x * NK + k] = s;
+  }
+  if (finish_blocks<NK>(cd.partial, cd.ticket, nb, total) && (int)threadIdx.x < nk)
+    hout[threadIdx.x] = total[threadIdx.x];
+}
+
 // w -= sum h V over all nk vectors (h: h2, or h1 where `first`), and with `column` |w| and
-// column j of H
-__global__ void __launch_bounds__(ORTH_THREADS) k_orth_update(const CaseDev* __restrict__ cases, int nk, int j,
-                                                              int first, int column) {
+// column j of H.  Two elements a thread and 32 loads in flight where the blocks are few; DENSE: one
+// element, eight loads, four blocks an SM (the same bits).
+template <bool DENSE>
+__global__ void __launch_bounds__(ORTH_THREADS, DENSE ? 4 : 2)
+    k_orth_update(const CaseDev* __restrict__ cases, int nk, int j, int first, int column) {
   const CaseDev& cd = cases[blockIdx.y];
   if (!cd.enabled) return;
   Scalars* sc = cd.sc;
@@ -273,7 +353,7 @@ __global__ void __launch_bounds__(ORTH_THREADS) k_orth_update(const CaseDev* __r
   int lo, hi;
   chunk(n, nb, lo, hi);
   double acc[8] = {};
-  constexpr int E = 2, KB = 16;
+  constexpr int E = DENSE ? 1 : 2, KB = DENSE ? 8 : 16;
   for (int e = lo + threadIdx.x; e < hi; e += E * ORTH_THREADS) {
     double x[E], s[E] = {};
 #pragma unroll
@@ -283,8 +363,8 @@ __global__ void __launch_bounds__(ORTH_THREADS) k_orth_update(const CaseDev* __r
 #pragma unroll
       for (int i = 0; i < E; ++i)
 #pragma unroll
-        for (int k = 0; k < KB; ++k)
-          v[i][k] = k0 + k < nk && e + i * ORTH_THREADS < hi ? V[(k0 + k) * ldv + e + i * ORTH_THREADS] : 0.0;
+        for (int k = 0; k < KB; ++k)   // (no branch: all in flight)
+          v[i][k] = V[(size_t)min(k0 + k, nk - 1) * ldv + min(e + i * ORTH_THREADS, hi - 1)];
 #pragma unroll
       for (int k = 0; k < KB; ++k)
         if (k0 + k < nk)
@@ -293,9 +373,10 @@ __global__ void __launch_bounds__(ORTH_THREADS) k_orth_update(const CaseDev* __r
     }
 #pragma unroll
     for (int i = 0; i < E; ++i) {
+      if (e + i * ORTH_THREADS >= hi) break;
       x[i] -= s[i];
       acc[0] += x[i] * x[i];
-      if (e + i * ORTH_THREADS < hi) w[e + i * ORTH_THREADS] = x[i];
+      w[e + i * ORTH_THREADS] = x[i];
     }
   }
   if (!column || !finish_sums<8>(acc, cd.partial, cd.ticket, nb, total)) return;
@@ -680,26 +761,52 @@ void launch_cycle_gate(const CaseDev* cases, const BatchDims& d, cudaGraphCondit
   k_cycle_gate<<<1, 256, 0, st>>>(cases, d.n_cases, gate, cycles);
 }
 
+// The dense form where the launch has more blocks than SMs and they are short: at most 768
+// elements for each block an SM is given, and 2560.  The three passes, registers and dense: two
+// 385 x 97 SA cases (1311 elements a block) over 30 vectors 70 and 64 us, eight over 8, 15 and 30
+// vectors 111 and 86, 191 and 151, 301 and 275 us; two 257 x 65 Euler cases (478) over 10 vectors 31 and 28 us,
+// 32 of them 317 and 198 us; four 513 x 129 SA cases (2300) over 10 and 30 vectors 122 and 84, 239 and 232 us,
+// but two over 30 vectors 125 and 144 us; four 769 x 193 cases (5110) over 30 vectors 448 and 500 us,
+// eight 385 x 97 cases with one of those 410 and 516 us.  A case alone has at most a block an SM.
+constexpr int ORTH_DENSE_EACH = 768, ORTH_DENSE_LONGEST = 2560;
+static bool orth_dense(const BatchDims& d) {
+  return d.orth_total > 148 && d.orth_chunk <= ORTH_DENSE_LONGEST &&
+         148LL * d.orth_chunk <= (long long)ORTH_DENSE_EACH * d.orth_total;
+}
+
+template <int NK, int E, bool UPDATE>
+static void orth_dots(const CaseDev* cases, const BatchDims& d, int k0, int count, int second, cudaStream_t st) {
+  const dim3 grid(orth_blocks(d.n_vec), d.n_cases);
+  if (orth_dense(d))
+    k_orth_dots_dense<NK, UPDATE><<<grid, ORTH_THREADS, d.orth_chunk * sizeof(double), st>>>(cases, k0, count, second);
+  else
+    k_orth_dots<NK, E, UPDATE><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
+}
+
 static void orth_fp64(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {
   const int nk = j + 1;
   const dim3 grid(orth_blocks(d.n_vec), d.n_cases);
   auto dots = [&](int k0, int count, int second) {
-    if (count <= 8) k_orth_dots<8, 4, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
-    else if (count <= 16) k_orth_dots<16, 2, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
-    else k_orth_dots<32, 2, false><<<grid, ORTH_THREADS, 0, st>>>(cases, k0, count, second);
+    if (count <= 8) orth_dots<8, 4, false>(cases, d, k0, count, second, st);
+    else if (count <= 16) orth_dots<16, 2, false>(cases, d, k0, count, second, st);
+    else orth_dots<32, 1, false>(cases, d, k0, count, second, st);
+  };
+  auto update = [&](int first, int column) {
+    if (orth_dense(d)) k_orth_update<true><<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, first, column);
+    else k_orth_update<false><<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, first, column);
   };
   for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(k0, min(ORTH_NK, nk - k0), 0);
   if (nk <= 8) {
-    k_orth_dots<8, 4, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+    orth_dots<8, 4, true>(cases, d, 0, nk, 1, st);
   } else if (nk <= 16) {
-    k_orth_dots<16, 2, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+    orth_dots<16, 2, true>(cases, d, 0, nk, 1, st);
   } else if (nk <= ORTH_NK) {
-    k_orth_dots<32, 1, true><<<grid, ORTH_THREADS, 0, st>>>(cases, 0, nk, 1);
+    orth_dots<32, 1, true>(cases, d, 0, nk, 1, st);
   } else {   // more vectors than a thread holds: the update, then the dots in slices
-    k_orth_update<<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, 1, 0);
+    update(1, 0);
     for (int k0 = 0; k0 < nk; k0 += ORTH_NK) dots(k0, min(ORTH_NK, nk - k0), 1);
   }
-  k_orth_update<<<grid, ORTH_THREADS, 0, st>>>(cases, nk, j, 0, 1);
+  update(0, 1);
 }
 
 template <int NK> static void mdot_fp32(const CaseDev* cases, const BatchDims& d, int j, cudaStream_t st) {

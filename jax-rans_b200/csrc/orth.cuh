@@ -7,6 +7,8 @@ namespace jr {
 
 // One block an SM: its threads' registers hold the basis entries in flight.
 constexpr int ORTH_THREADS = 256, ORTH_BLOCKS = 148, ORTH_NK = 32;
+// The elements a warp takes at a time where a warp takes a vector
+constexpr int ORTH_ROUND = 2 * ORTH_THREADS;
 
 // The NK sums of every lane over the warp, by a butterfly that halves the sums a lane holds at
 // each exchange: afterwards lane l holds sum l * NK / 32 (NK < 32: every 32 / NK-th lane's) in
@@ -32,23 +34,14 @@ __device__ __forceinline__ void lane_sums(double (&acc)[NK], int lane) {
   }
 }
 
-// sums[NK] of every thread of the nb blocks (blockIdx.x, ORTH_THREADS each): over the block
-// into partial, and by the last block to finish over the blocks in order; true there, with the
-// totals in total[NK]
+// The sums of the nb blocks (blockIdx.x, ORTH_THREADS each; a block's in partial[b * NK + k], stored
+// by any of its threads) in order, by the last block to finish; true there, with the totals in
+// total[NK]
 template <int NK>
-__device__ bool finish_sums(double (&sums)[NK], double* partial, unsigned* ticket, int nb, double* total) {
-  __shared__ double warps[ORTH_THREADS / 32][NK];
+__device__ bool finish_blocks(const double* partial, unsigned* ticket, int nb, double* total) {
   __shared__ double groups[ORTH_THREADS];
   __shared__ bool last;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  lane_sums<NK>(sums, lane);
-  if (lane % (32 / NK) == 0) warps[warp][lane / (32 / NK)] = sums[0];
-  __syncthreads();
-  if (t < NK) {
-    double s = warps[0][t];
-    for (int w = 1; w < ORTH_THREADS / 32; ++w) s += warps[w][t];
-    partial[(size_t)blockIdx.x * NK + t] = s;
-  }
+  const int t = threadIdx.x;
   __threadfence();
   __syncthreads();
   if (t == 0) last = atomicAdd(ticket, 1u) == (unsigned)nb - 1;
@@ -75,6 +68,23 @@ __device__ bool finish_sums(double (&sums)[NK], double* partial, unsigned* ticke
   if (t == 0) *ticket = 0u;
   __syncthreads();
   return true;
+}
+
+// The same of sums[NK] of every thread: over the warp, then the block's warps in order, then the
+// blocks
+template <int NK>
+__device__ bool finish_sums(double (&sums)[NK], double* partial, unsigned* ticket, int nb, double* total) {
+  __shared__ double warps[ORTH_THREADS / 32][NK];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  lane_sums<NK>(sums, lane);
+  if (lane % (32 / NK) == 0) warps[warp][lane / (32 / NK)] = sums[0];
+  __syncthreads();
+  if (t < NK) {
+    double s = warps[0][t];
+    for (int w = 1; w < ORTH_THREADS / 32; ++w) s += warps[w][t];
+    partial[(size_t)blockIdx.x * NK + t] = s;
+  }
+  return finish_blocks<NK>(partial, ticket, nb, total);
 }
 
 }  // namespace jr

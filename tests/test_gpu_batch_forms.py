@@ -1,7 +1,9 @@
 """The FP64 kernels that take one of two forms by how many cases a launch holds: the J.v tile
-(coefficients loaded ahead while every tile is resident, or where they are used).  A case's
-history and state are bitwise the same whichever form its launch took, for each model's
-instances and on grids whose edges cut the tiles."""
+(coefficients loaded ahead while every tile is resident, or where they are used) and the
+orthogonalisation (a thread's vectors in registers, or a warp a vector).  A case's history and
+state are bitwise the same whichever form its launch took, for each model's instances, on grids
+whose edges cut the tiles and the blocks' parts, and for every number of vectors a form has its
+own kernel for."""
 
 from __future__ import annotations
 
@@ -15,10 +17,10 @@ from jaxrans_b200.solver import freestream_state
 
 pytestmark = pytest.mark.gpu
 
-CASES = 6   # 6 x 76 tiles of the J.v: more than are resident at once; alone they all are
+CASES = 6   # 6 x 76 tiles of the J.v and 6 x 53 blocks of the basis: more than are resident at once
 
 
-@pytest.mark.parametrize("model,subspace", [("euler", 10), ("laminar", 10), ("sa", 10)])
+@pytest.mark.parametrize("model,subspace", [("euler", 8), ("euler", 10), ("euler", 33), ("laminar", 10), ("sa", 20)])
 def test_a_batch_past_the_rule_is_bitwise_the_cases_alone(cuda, model, subspace):
     from jaxrans_b200.native import DevicePlan
     euler = model == "euler"
