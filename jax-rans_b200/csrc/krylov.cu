@@ -430,9 +430,26 @@ __global__ void __launch_bounds__(RED_THREADS) k_mdot_fp32(const CaseDev* __rest
     double wi = w[i];
     if constexpr (MODE != 0) {
       double s = 0.0;
+      // The 16-vector kernels load under the count's branch, the others select what they loaded:
+      // the same sums, but ptxas schedules the loads so differently that the branch takes the three
+      // passes over 8 vectors 46 -> 50 us on a 769 x 193 case and over 30 vectors 106 -> 120, eight
+      // 385 x 97 cases 219 -> 230, yet over 15 vectors 61 -> 57 and 138 -> 125.
+      if constexpr (NK == 16) {
 #pragma unroll
-      for (int k = 0; k < NK; ++k)
-        if (k < nk) s += h[k] * double(V[(size_t)k * ldv + i]);
+        for (int k = 0; k < NK; ++k)
+          if (k < nk) s += h[k] * double(V[(size_t)k * ldv + i]);
+      } else {
+        constexpr int KB = 1;
+#pragma unroll
+        for (int k0 = 0; k0 < NK; k0 += KB) {
+          double vk[KB];
+#pragma unroll
+          for (int u = 0; u < KB; ++u) vk[u] = k0 + u < nk ? double(V[(size_t)(k0 + u) * ldv + i]) : 0.0;
+#pragma unroll
+          for (int u = 0; u < KB; ++u)
+            if (k0 + u < nk) s += h[k0 + u] * vk[u];
+        }
+      }
       wi = wi - s;
       w[i] = wi;
     }
