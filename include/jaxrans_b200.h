@@ -350,11 +350,24 @@ int jr_precondition3d(jr_plan3d* plan, const double* U, double cfl, const double
  * cycles, CGS2, Givens least squares, the relaxation, acceptance test and CFL ramp of
  * src/jaxrans/solvers/implicit.py:54-168, driven from the host over device kernels (it
  * synchronises once per Krylov cycle and for the step's own scalars).  The products use one
- * linearisation per step, whose factors (about 2 KB a cell with SA) the plan's first step
- * allocates; without the memory for them, jr_jvp3d's kernels.  Replaces make_newton_step run
- * as the driver's block on a 3D atlas. */
+ * linearisation per step, whose factors (about 2 KB a cell with SA) the plan's first steps
+ * allocate and the plan keeps; without the memory for them, jr_jvp3d's kernels, slower and equal to
+ * rounding.  A march is repeatable bit for bit while its steps use one of the two (jr_product3d
+ * tells).  Another plan's creation that the device would refuse for lack of memory takes the
+ * factors of plans not stepping back; a call that has none tries for them again.  Replaces
+ * make_newton_step run as the driver's block on a 3D atlas. */
 int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, double* residual_norm,
                       double* history);
+/* The most bytes the stored factors of jr_newton_steps3d's products may take (negative, the default:
+ * any that the device has): 0 keeps every step on jr_jvp3d's kernels, and frees what the plan holds
+ * beyond the limit.  No counterpart in the reference. */
+int jr_product_limit3d(jr_plan3d* plan, int64_t bytes);
+/* The product the plan's last jr_newton_steps3d used, and the bytes its stored factors take
+ * (either pointer may be null).  No counterpart in the reference. */
+#define JR_PRODUCT_NONE 0        /* no step yet */
+#define JR_PRODUCT_LINEARISED 1  /* one linearisation per step, its factors stored */
+#define JR_PRODUCT_DUAL 2        /* jr_jvp3d's kernels for every product */
+int jr_product3d(jr_plan3d* plan, int32_t* form, int64_t* bytes);
 /* Force coefficients of a 3D case at U (device): out (host, 4) = cl, cd, cm, cd_friction
  * -- lift and drag in the plane of incidence (x-z) per q_inf * area, the pitching moment
  * of pressure and friction about centre (3 values) per q_inf * area * length; the

@@ -118,6 +118,8 @@ static int fail(int code, const std::string& msg) {
 }
 
 namespace jr {
+// cudaMalloc that takes back what 3D plans can do without before it gives up (capi3d.cu)
+cudaError_t device_malloc(void** out, size_t bytes);
 // shared with the 3D entry points (capi3d.cu)
 int report_error(int code, const std::string& msg) { return fail(code, msg); }
 
@@ -132,7 +134,7 @@ static int cuda_check(const char* where) {
 template <class T> static int dev_copy(jr_plan* p, T** dst, const T* src, size_t n) {
   *dst = nullptr;
   if (n == 0) return JR_OK;
-  if (cudaMalloc((void**)dst, n * sizeof(T)) != cudaSuccess) return fail(JR_ENOMEM, "cudaMalloc failed");
+  if (device_malloc((void**)dst, n * sizeof(T)) != cudaSuccess) return fail(JR_ENOMEM, "cudaMalloc failed");
   p->allocs.push_back(*dst);
   if (src != nullptr && cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess)
     return fail(JR_ECUDA, "cudaMemcpy to the device failed");
@@ -143,7 +145,7 @@ template <class T> static int dev_copy(jr_plan* p, T** dst, const T* src, size_t
 static int dev_alloc(jr_plan* p, void** dst, size_t bytes) {
   *dst = nullptr;
   if (bytes == 0) bytes = 16;
-  if (cudaMalloc(dst, bytes) != cudaSuccess) return fail(JR_ENOMEM, "cudaMalloc failed");
+  if (device_malloc(dst, bytes) != cudaSuccess) return fail(JR_ENOMEM, "cudaMalloc failed");
   p->allocs.push_back(*dst);
   cudaMemset(*dst, 0, bytes);
   return JR_OK;

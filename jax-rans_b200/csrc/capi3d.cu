@@ -2,6 +2,7 @@
 // and ghost records, two work buffers, a stream), its residual and its J.v.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -11,6 +12,7 @@
 
 namespace jr {
 int report_error(int code, const std::string& msg);
+cudaError_t device_malloc(void** out, size_t bytes);
 }  // namespace jr
 
 using namespace jr;
@@ -32,9 +34,12 @@ struct jr_plan3d {
   double* work = nullptr;      // the Newton step's vectors
   Gmres3* scalars = nullptr;
   // the linearised J.v's buffers, made by the first Newton steps (a plan that only evaluates
-  // residuals never pays for them)
+  // residuals never pays for them) unless they exceed lin_limit; one allocation, lin_face its start
   double *lin_face = nullptr, *lin_cell = nullptr, *lin_dq = nullptr;
-  bool lin_made = false;
+  int64_t lin_limit = -1;      // bytes; < 0: none
+  int form = 0;                // the product the last Newton steps used (JR_PRODUCT_*)
+  std::mutex stepping;         // held while Newton steps run: the buffers stay
+  int device = 0;
   cudaStream_t st = nullptr;
 };
 
@@ -48,7 +53,7 @@ template <class T> static int copy3(jr_plan3d* p, const T** dst, const T* src, s
   *dst = nullptr;
   if (n == 0 || src == nullptr) return JR_OK;
   void* d = nullptr;
-  if (cudaMalloc(&d, n * sizeof(T)) != cudaSuccess) return report_error(JR_ENOMEM, "cudaMalloc failed");
+  if (device_malloc(&d, n * sizeof(T)) != cudaSuccess) return report_error(JR_ENOMEM, "cudaMalloc failed");
   p->allocs.push_back(d);
   if (cudaMemcpy(d, src, n * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess)
     return report_error(JR_ECUDA, "cudaMemcpy to the device failed");
@@ -56,22 +61,61 @@ template <class T> static int copy3(jr_plan3d* p, const T** dst, const T* src, s
   return JR_OK;
 }
 
-// The linearised J.v's buffers.  Where they do not fit, the plan keeps its Newton steps on
-// the dual-number J.v, which needs none.
-static void make_lin(jr_plan3d* p) {
-  if (p->lin_made) return;
-  p->lin_made = true;
+// ---- the linearised J.v's buffers: memory a plan can do without (its products are then the
+// dual-number J.v's).  The plans that hold any are listed, so that an allocation that nothing can
+// do without (a plan's own) takes them back where it would otherwise fail: what fitted on the
+// device beside a plan before its first Newton step still fits after it.
+static std::mutex lin_mutex;
+static std::vector<jr_plan3d*> lin_holders;
+
+static size_t lin_bytes(const jr_plan3d* p) {
   size_t face, cell, tangents;
   lin3_sizes(p->dev, face, cell, tangents);
+  return (face + cell + tangents) * sizeof(double);
+}
+
+// (lin_mutex held, no Newton steps of p running)
+static void free_lin(jr_plan3d* p) {
+  cudaFree(p->lin_face);
+  p->lin_face = p->lin_cell = p->lin_dq = nullptr;
+  lin_holders.erase(std::remove(lin_holders.begin(), lin_holders.end(), p), lin_holders.end());
+}
+
+cudaError_t jr::device_malloc(void** out, size_t bytes) {
+  cudaError_t e = cudaMalloc(out, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  int device = 0;
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> hold(lin_mutex);
+  const std::vector<jr_plan3d*> holders = lin_holders;
+  for (jr_plan3d* p : holders) {
+    if (p->device != device || !p->stepping.try_lock()) continue;
+    free_lin(p);
+    p->stepping.unlock();
+    e = cudaMalloc(out, bytes);
+    if (e == cudaSuccess) break;
+    cudaGetLastError();
+  }
+  return e;
+}
+
+// (p->stepping held)  Tried by every call that has none: memory may have become free.
+static void make_lin(jr_plan3d* p) {
+  size_t face, cell, tangents;
+  lin3_sizes(p->dev, face, cell, tangents);
+  const size_t bytes = (face + cell + tangents) * sizeof(double);
+  if (p->lin_face != nullptr || (p->lin_limit >= 0 && bytes > (size_t)p->lin_limit)) return;
   void* mem = nullptr;
-  if (cudaMalloc(&mem, (face + cell + tangents) * sizeof(double)) != cudaSuccess) {
+  if (cudaMalloc(&mem, bytes) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
-  p->allocs.push_back(mem);
   p->lin_face = static_cast<double*>(mem);
   p->lin_cell = p->lin_face + face;
   p->lin_dq = p->lin_cell + cell;
+  std::lock_guard<std::mutex> hold(lin_mutex);
+  lin_holders.push_back(p);
 }
 
 // Every ghost's program (Plan3Dev::ghost_of): the record that writes it last, back through
@@ -121,6 +165,10 @@ extern "C" {
 
 int jr_plan3d_destroy(jr_plan3d* plan) {
   if (!plan) return JR_OK;
+  {
+    std::lock_guard<std::mutex> hold(lin_mutex);
+    free_lin(plan);
+  }
   for (void* a : plan->allocs) cudaFree(a);
   if (plan->st) cudaStreamDestroy(plan->st);
   delete plan;
@@ -173,6 +221,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   }
   jr_plan3d* p = new jr_plan3d();
   p->n_canvas = n;
+  cudaGetDevice(&p->device);
   Plan3Dev& dv = p->dev;
   dv.NI = d->NI;
   dv.NJ = d->NJ;
@@ -244,7 +293,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   p->wall_mid.assign(d->wall_mid, d->wall_mid + 3 * (size_t)d->n_walls);
   if (d->n_walls > 0) {
     void* l = nullptr;
-    if (cudaMalloc(&l, (size_t)d->n_walls * 7 * sizeof(double)) != cudaSuccess) {
+    if (device_malloc(&l, (size_t)d->n_walls * 7 * sizeof(double)) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
@@ -260,7 +309,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   dv.line_coupled = d->preconditioner == 2;
   if (n_links > 0) {
     void* sc = nullptr;
-    if (cudaMalloc(&sc, line_factor_words3(dv) * (dv.line_fp32 ? sizeof(float) : sizeof(double))) != cudaSuccess) {
+    if (device_malloc(&sc, line_factor_words3(dv) * (dv.line_fp32 ? sizeof(float) : sizeof(double))) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
@@ -271,7 +320,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
     const size_t nf = (size_t)(d->NI + 1) * d->NJ * d->NK + (size_t)d->NI * (d->NJ + 1) * d->NK +
                       (size_t)d->NI * d->NJ * (d->NK + 1);
     void* fb = nullptr;
-    if (cudaMalloc(&fb, nf * d->nvar * sizeof(double)) != cudaSuccess) {
+    if (device_malloc(&fb, nf * d->nvar * sizeof(double)) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
@@ -283,8 +332,8 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
                       (size_t)d->NI * d->NJ * (d->NK + 1);
     const size_t nn = (size_t)(d->NI + 1) * (d->NJ + 1) * (d->NK + 1);
     void *geo = nullptr, *nb = nullptr;
-    if (cudaMalloc(&geo, nf * 10 * sizeof(double)) != cudaSuccess ||
-        (p->allocs.push_back(geo), cudaMalloc(&nb, nn * 5 * sizeof(Dual))) != cudaSuccess) {
+    if (device_malloc(&geo, nf * 10 * sizeof(double)) != cudaSuccess ||
+        (p->allocs.push_back(geo), device_malloc(&nb, nn * 5 * sizeof(Dual))) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
@@ -293,7 +342,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
     dv.node_buf = nb;
   }
   const size_t work = (size_t)d->nvar * n * sizeof(Dual);
-  if (cudaMalloc(&p->A, work) != cudaSuccess) {
+  if (device_malloc(&p->A, work) != cudaSuccess) {
     jr_plan3d_destroy(p);
     return report_error(JR_ENOMEM, "cudaMalloc failed");
   }
@@ -309,7 +358,7 @@ int jr_plan3d_create(const jr_plan3d_desc* d, jr_plan3d** out) {
   {
     const size_t words = DeviceOps3::work_doubles((size_t)d->nvar * n, n, d->krylov_subspace);
     void *w = nullptr, *f = nullptr;
-    if (cudaMalloc(&w, words * sizeof(double)) != cudaSuccess || (p->allocs.push_back(w), cudaMalloc(&f, sizeof(Gmres3))) != cudaSuccess) {
+    if (device_malloc(&w, words * sizeof(double)) != cudaSuccess || (p->allocs.push_back(w), device_malloc(&f, sizeof(Gmres3))) != cudaSuccess) {
       jr_plan3d_destroy(p);
       return report_error(JR_ENOMEM, "cudaMalloc failed");
     }
@@ -376,7 +425,11 @@ int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, 
   ops.factor = plan->factor;
   ops.line = plan->cfg.preconditioner >= 1;
   ops.st = plan->st;
-  make_lin(plan);
+  std::lock_guard<std::mutex> hold(plan->stepping);
+  if (n_steps > 0) {
+    make_lin(plan);
+    plan->form = plan->lin_face != nullptr ? JR_PRODUCT_LINEARISED : JR_PRODUCT_DUAL;
+  }
   ops.lin_face = plan->lin_face;
   ops.lin_cell = plan->lin_cell;
   ops.lin_dq = plan->lin_dq;
@@ -392,6 +445,22 @@ int jr_newton_steps3d(jr_plan3d* plan, double* U, int32_t n_steps, double* cfl, 
   *cfl = c;
   *residual_norm = r;
   return check3("jr_newton_steps3d");
+}
+
+int jr_product_limit3d(jr_plan3d* plan, int64_t bytes) {
+  if (!plan) return report_error(JR_EINVAL, "null argument");
+  std::lock_guard<std::mutex> steps(plan->stepping);
+  std::lock_guard<std::mutex> hold(lin_mutex);
+  plan->lin_limit = bytes;
+  if (bytes >= 0 && lin_bytes(plan) > (size_t)bytes) free_lin(plan);
+  return check3("jr_product_limit3d");
+}
+
+int jr_product3d(jr_plan3d* plan, int32_t* form, int64_t* bytes) {
+  if (!plan) return report_error(JR_EINVAL, "null argument");
+  if (form) *form = plan->form;
+  if (bytes) *bytes = (int64_t)lin_bytes(plan);
+  return JR_OK;
 }
 
 int jr_forces3d(jr_plan3d* plan, const double* U, double area, double length, const double* centre, double* out) {
@@ -425,7 +494,8 @@ int jr_time_kernels3d(jr_plan3d* plan, const double* U, int32_t reps, double* ms
   if (!plan || !U || !ms || reps < 1) return report_error(JR_EINVAL, "bad argument");
   const size_t N = (size_t)plan->dev.nvar * plan->n_canvas;
   double *v = nullptr, *out = nullptr;
-  if (cudaMalloc(&v, N * sizeof(double)) != cudaSuccess || cudaMalloc(&out, N * sizeof(double)) != cudaSuccess) {
+  if (device_malloc((void**)&v, N * sizeof(double)) != cudaSuccess ||
+      device_malloc((void**)&out, N * sizeof(double)) != cudaSuccess) {
     cudaFree(v);
     return report_error(JR_ENOMEM, "cudaMalloc failed");
   }
@@ -466,7 +536,7 @@ int jr_wall_distance3d(const double* points, int64_t n_points, const double* fac
   if ((n_points > 0 && (!points || !out)) || (n_faces > 0 && !faces)) return report_error(JR_EINVAL, "null argument");
   if (n_points == 0) return JR_OK;
   double* spheres = nullptr;
-  if (n_faces > 0 && cudaMalloc(&spheres, (size_t)n_faces * 4 * sizeof(double)) != cudaSuccess)
+  if (n_faces > 0 && device_malloc((void**)&spheres, (size_t)n_faces * 4 * sizeof(double)) != cudaSuccess)
     return report_error(JR_ENOMEM, "cudaMalloc failed");
   cudaStream_t st;
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) {

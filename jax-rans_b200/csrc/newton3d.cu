@@ -1,7 +1,8 @@
 // The 3D Newton step on the device: newton3d.cuh's driver over kernel-backed vector
 // operations (the residual, J.v, wave speeds and line solve of residual3d.cu and
 // linesolve3d.cu; dot products by a fixed-order two-stage reduction, so a step is
-// bitwise reproducible).  The device has its own form of the driver's GMRES cycle: the
+// bitwise reproducible while its products take the same of their two forms: matvec below).
+// The device has its own form of the driver's GMRES cycle: the
 // scalars of an Arnoldi step stay on the device (Gmres3), so its six kernels follow one
 // another without a word from the host, which reads H once a cycle for the least squares.
 #include <algorithm>

@@ -66,7 +66,7 @@ EXPORTS = ("jr_plan_create", "jr_plan_destroy", "jr_last_error", "jr_plan_sizes"
            "jr_plan3d_create", "jr_plan3d_destroy", "jr_residual3d", "jr_jvp3d", "jr_wave_speeds3d",
            "jr_precondition3d", "jr_newton_steps3d", "jr_forces3d", "jr_wall_distance3d",
            "jr_launches3d", "jr_wall_loads3d", "jr_monitor_set", "jr_monitor_blocks", "jr_monitor_get", "jr_norm",
-           "jr_time_kernels3d")
+           "jr_time_kernels3d", "jr_product_limit3d", "jr_product3d")
 
 TIMED_KERNELS = ("residual_tile", "jvp_tile", "ghosts_tangent", "line_apply", "line_factor", "cgs2_full_basis",
                  "linearize")
@@ -76,6 +76,7 @@ _LIB = None
 
 # return codes and status bits of the C ABI (include/jaxrans_b200.h)
 JR_OK, JR_EINVAL, JR_ENOMEM, JR_ECUDA, JR_EMISMATCH, JR_ETIMEOUT = 0, 1, 2, 3, 4, 5
+JR_PRODUCT_NONE, JR_PRODUCT_LINEARISED, JR_PRODUCT_DUAL = 0, 1, 2
 JR_STATUS_NONFINITE, JR_STATUS_REJECTED, JR_STATUS_GMRES_BREAKDOWN, JR_STATUS_WAIT_LIMIT = 1, 2, 4, 8
 
 
@@ -135,6 +136,8 @@ def load_library(path: Path | None = None) -> C.CDLL:
         "jr_wave_speeds3d": (C.c_int, [vp, vp, vp]),
         "jr_precondition3d": (C.c_int, [vp, vp, C.c_double, vp, vp]),
         "jr_newton_steps3d": (C.c_int, [vp, vp, C.c_int32, C.POINTER(C.c_double), C.POINTER(C.c_double), vp]),
+        "jr_product_limit3d": (C.c_int, [vp, C.c_int64]),
+        "jr_product3d": (C.c_int, [vp, C.POINTER(C.c_int32), C.POINTER(C.c_int64)]),
         "jr_forces3d": (C.c_int, [vp, vp, C.c_double, C.c_double, vp, vp]),
         "jr_wall_distance3d": (C.c_int, [vp, C.c_int64, vp, C.c_int32, vp]),
         "jr_launches3d": (C.c_int, [vp]),

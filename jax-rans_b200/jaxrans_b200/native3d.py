@@ -11,11 +11,13 @@ writes (a later write of the same ghost wins, as in the gather form).
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 from dataclasses import dataclass
 
 import numpy as np
 
-from .native import FLUX_CODES, LIMITER_CODES, NativeError, _check, _f64p, _i32p, _u8p, load_library
+from .native import (FLUX_CODES, JR_PRODUCT_DUAL, LIMITER_CODES, NativeError, _check, _f64p, _i32p, _u8p,
+                     load_library)
 from .grid3d import KINDS_3D
 from .plan3d import Plan3
 
@@ -184,6 +186,7 @@ class DevicePlan3:
         handle = C.c_void_p()
         _check(self.lib, self.lib.jr_plan3d_create(C.byref(d), C.byref(handle)), "jr_plan3d_create")
         self.handle = handle
+        self._limited = self._warned = False
 
     def close(self) -> None:
         if getattr(self, "handle", None):
@@ -231,9 +234,31 @@ class DevicePlan3:
         (u,), _ = self._run("jr_newton_steps3d", U)
         c, r = C.c_double(cfl), C.c_double(residual_norm)
         hist = np.zeros(n_steps)
+        self._steps(u, n_steps, c, r, hist)
+        return u.cpu().numpy(), c.value, r.value, hist
+
+    def _steps(self, u, n_steps, c, r, hist):
         _check(self.lib, self.lib.jr_newton_steps3d(self.handle, u.data_ptr(), int(n_steps), C.byref(c), C.byref(r),
                                                      hist.ctypes.data), "jr_newton_steps3d")
-        return u.cpu().numpy(), c.value, r.value, hist
+        if not (self._limited or self._warned):
+            form, size = self.product()
+            if form == JR_PRODUCT_DUAL:
+                self._warned = True
+                warnings.warn(f"no {size} bytes of device memory for the Newton step's factors: its products take "
+                              "the slower dual-number form (the next call tries again)", RuntimeWarning, stacklevel=3)
+
+    def product(self):
+        """``(form, bytes)``: the matrix-vector product of the last Newton steps
+        (``JR_PRODUCT_*``) and the bytes its stored factors take (``jr_product3d``)."""
+        form, size = C.c_int32(), C.c_int64()
+        _check(self.lib, self.lib.jr_product3d(self.handle, C.byref(form), C.byref(size)), "jr_product3d")
+        return form.value, size.value
+
+    def product_limit(self, size: int | None) -> None:
+        """The most bytes those factors may take (None: any; 0: the dual-number product)."""
+        _check(self.lib, self.lib.jr_product_limit3d(self.handle, -1 if size is None else int(size)),
+               "jr_product_limit3d")
+        self._limited = size is not None
 
     def time_kernels(self, U, reps: int = 5) -> dict:
         """Average ms per call at ``U`` (``jr_time_kernels3d``, CUDA events on the plan's
@@ -260,8 +285,7 @@ class DevicePlan3:
         u, cfl, res = self._state
         c, r = C.c_double(cfl), C.c_double(res)
         hist = np.zeros(n_steps)
-        _check(self.lib, self.lib.jr_newton_steps3d(self.handle, u.data_ptr(), int(n_steps), C.byref(c), C.byref(r),
-                                                     hist.ctypes.data), "jr_newton_steps3d")
+        self._steps(u, n_steps, c, r, hist)
         self._state = [u, c.value, r.value]
         return hist
 
