@@ -120,55 +120,6 @@ static void make_lin(jr_plan3d* p) {
   lin_holders.push_back(p);
 }
 
-// Every ghost's program (Plan3Dev::ghost_of): the record that writes it last, back through
-// the records that had filled each source before its stage, to a cell of its own state.
-static void ghost_programs(const jr_plan3d_desc* d, size_t n, std::vector<int>& ghost_of, std::vector<int>& root,
-                           std::vector<int>& off, std::vector<int>& rec) {
-  std::vector<int> last(n, -1), parent;
-  int at = 0, total = 0;
-  for (int s = 0; s < d->n_stages; ++s) total += d->stage_records[s];
-  parent.reserve(total);
-  for (int s = 0; s < d->n_stages; ++s) {
-    const int end = at + d->stage_records[s];
-    for (int r = at; r < end; ++r) parent.push_back(last[d->source[r]]);
-    for (int r = at; r < end; ++r) last[d->ghost[r]] = r;
-    at = end;
-  }
-  ghost_of.assign(n, -1);
-  off.assign(1, 0);
-  off.reserve((size_t)total + 1);
-  root.reserve(total);
-  std::vector<int> chain;
-  for (int w = 0; w < total; ++w) {
-    if (last[d->ghost[w]] != w) continue;   // written again by a later record
-    ghost_of[d->ghost[w]] = (int)root.size();
-    chain.clear();
-    int r = w;
-    for (;; r = parent[r]) {
-      if (d->kind[r] != 0) chain.push_back(r);
-      if (parent[r] < 0) break;
-    }
-    root.push_back(d->source[r]);
-    rec.insert(rec.end(), chain.rbegin(), chain.rend());
-    off.push_back((int)rec.size());
-  }
-}
-
-// each chain's length (to its first -1) and the cells on none
-static void chain_tables(const jr_plan3d_desc* d, size_t n, std::vector<int>& len, std::vector<int>& offchain) {
-  std::vector<char> on(n, 0);
-  len.resize(d->n_chains);
-  for (int c = 0; c < d->n_chains; ++c) {
-    const int* cells = d->chain_cells + (size_t)c * d->chain_L;
-    int k = 0;
-    for (; k < d->chain_L && cells[k] >= 0; ++k) on[cells[k]] = 1;
-    len[c] = k;
-  }
-  offchain.reserve(n - std::min(n, (size_t)d->n_chains * d->chain_L));
-  for (size_t c = 0; c < n; ++c)
-    if (!on[c]) offchain.push_back((int)c);
-}
-
 static void discard(jr_plan3d*& p) {
   jr_plan3d_destroy(p);
   p = nullptr;
@@ -247,9 +198,6 @@ static int create_plan3(const jr_plan3d_desc* d, jr_plan3d** out, jr_plan3d*& p)
   }
   TRY3(copy3(p, &dv.centres, d->centres, 3 * (size_t)(d->NI + 2) * (d->NJ + 2) * (d->NK + 2)));
   TRY3(copy3(p, &dv.distance, d->nvar == 6 ? d->distance : nullptr, n));
-  dv.n_stages = d->n_stages;
-  dv.stage_off[0] = 0;
-  for (int s = 0; s < d->n_stages; ++s) dv.stage_off[s + 1] = dv.stage_off[s] + d->stage_records[s];
   programs.get();
   TRY3(copy3(p, &dv.ghost_of, ghost_of.data(), ghost_of.size()));
   TRY3(copy3(p, &dv.gp_root, root.data(), root.size()));

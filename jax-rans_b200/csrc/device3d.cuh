@@ -35,10 +35,7 @@ struct Plan3Dev {
   const double* faces[3];      // family a: 3 planes of (NI + (a==0)) (NJ + (a==1)) (NK + (a==2))
   const double* centres;       // 3 planes of (NI+2)(NJ+2)(NK+2): one ring beyond the canvas
   const double* distance;      // canvas (SA) or null
-  int n_stages;
-  int stage_off[MAX_STAGES3 + 1];   // records of stage s: [stage_off[s], stage_off[s+1])
-  const int* g_ghost;
-  const int* g_source;
+  // the ghost records of every stage, one after another
   const int* g_kind;           // 0 copy, 1 slip wall, 2 no-slip wall, 3 symmetry, 4 far field
   const double* g_normal;      // 3 per record: the outward unit normal of the face
   const int* neighbours;       // canvas: the partner across a block face, or the cell itself
@@ -270,9 +267,6 @@ void launch_line_apply3(const Plan3Dev& p, const void* F, const double* r, doubl
                         cudaStream_t st);
 void launch_precondition3(const Plan3Dev& p, const double* U, double cfl, const double* r, double* z, void* F,
                           cudaStream_t st);
-// words per chain element of the host form's line factor (linesolve3d.cuh): three 5x5 blocks, three
-// SA scalars and the SA row's two coupling rows to the mean flow (the coupled form)
-constexpr int FACTOR3 = 88;
 
 // Kernels the 3D path has launched since the library was loaded (counted on the host at
 // each launch site; the benchmark's launch figure).

@@ -46,8 +46,7 @@ __global__ void __launch_bounds__(128) k3_line_cells(Plan3Dev p, const double* _
   }
 }
 
-// The elimination down a chain: T = D - lower C_{k-1}, P = T^-1 (Gauss-Jordan, one
-// reciprocal a pivot), C = P upper, and the SA row's scalars.  One thread a chain: a step is
+// line_factor_chain, one thread a chain: a step is
 // a serial chain of five pivots, so its neighbours' chains are what hides it; its rows leave
 // eight at a time, a sector a chain and word.  61,440 chains of 64: 1.1 ms, and the faces' and
 // cells' terms 1.0 ms (assembling the blocks, every wave speed of a cell twice among them,
@@ -59,159 +58,7 @@ __global__ void __launch_bounds__(64) k3_line_factor(Plan3Dev p, const double* _
                                                      const double* __restrict__ dflow,
                                                      const double* __restrict__ dsa, TF* __restrict__ F) {
   const int ch = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ch >= p.n_chains) return;
-  const double g = p.P.gamma;
-  const int groups = line_groups(p), len = p.ch_len[ch];
-  TF* out = F + ((size_t)(ch / LW_CHAINS) * LW_WORDS) * 32 + (ch % LW_CHAINS) * LW_ROWS;
-  const size_t stride = (size_t)groups * LW_WORDS * 32;
-  const bool coupled = SA && p.line_coupled;
-  double C[5][5] = {}, q[NV3_MAX] = {}, qb[NV3_MAX] = {};   // this cell's state, the one below's
-  double sl[3] = {0.0, 0.0, 0.0}, ll = 0.0, csa = 0.0, lsa = 0.0;   // the link below, outward from this cell
-  bool linked = false;
-  if (len > 0) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L], q);
-  for (int k = 0; k < len; ++k, out += stride) {
-    const int c = p.ch_cells[(size_t)ch * p.chain_L + k];
-    double T[5][5], L[5][5];
-    if (linked) coupling5_closed(qb, sl[0], sl[1], sl[2], ll, g, L);
-    else
-#pragma unroll
-      for (int a = 0; a < 5; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) L[a][b] = 0.0;
-    const double dg = dflow[c];
-#pragma unroll
-    for (int a = 0; a < 5; ++a)
-#pragma unroll
-      for (int b = 0; b < 5; ++b) {
-        double m = L[a][0] * C[0][b];
-#pragma unroll
-        for (int t = 1; t < 5; ++t) m = m + L[a][t] * C[t][b];
-        T[a][b] = (a == b ? dg : 0.0) - m;
-      }
-    // the SA row's scalars beside the mean flow's blocks, and the coupled form's rows
-    double slo = 0.0, spiv = 0.0, sc = 0.0, cpl[2][5] = {};
-    if constexpr (SA) {
-      if (!coupled) {
-        slo = lsa;
-        spiv = 1.0 / (dsa[c] - lsa * csa);
-      } else if (linked) {
-        sa_coupling_row(qb, sl, 1.0, cpl[0]);
-      }
-    }
-    // word w of the rows: the first six, or all eight
-    auto put = [&](int w, double r0, double r1, double r2, double r3, double r4, double r5, double r6, double r7) {
-      TF* o = out + w * 32;
-      if constexpr (sizeof(TF) == 4) {
-        *reinterpret_cast<float4*>(o) = make_float4((float)r0, (float)r1, (float)r2, (float)r3);
-        *reinterpret_cast<float4*>(o + 4) = make_float4((float)r4, (float)r5, (float)r6, (float)r7);
-      } else {
-        *reinterpret_cast<double2*>(o) = make_double2(r0, r1);
-        *reinterpret_cast<double2*>(o + 2) = make_double2(r2, r3);
-        *reinterpret_cast<double2*>(o + 4) = make_double2(r4, r5);
-        if (coupled) *reinterpret_cast<double2*>(o + 6) = make_double2(r6, r7);
-      }
-    };
-    // the link above: this cell's upper block and, for the next element, its lower one
-    const int sign = k + 1 < len ? p.ch_sign[(size_t)ch * p.chain_L + k] : 0;
-    double su[3] = {0.0, 0.0, 0.0}, lu = 0.0, qn[NV3_MAX] = {}, upsa = 0.0, nextsa = 0.0;
-    if (k + 1 < len) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L + k + 1], qn);
-    if (sign != 0) {
-      const int f = p.ch_face[(size_t)ch * p.chain_L + k];
-      int fa, fi, fj, fk;
-      face_of(p, f, fa, fi, fj, fk);
-      face_vector(p, fa, fi, fj, fk, su);
-#pragma unroll
-      for (int m = 0; m < 3; ++m) su[m] *= (double)sign;
-      lu = lam[f];
-      if constexpr (SA) {
-        const double um = -(double)sign * mflux[f], d = dflux[f];
-        upsa = -((um > 0.0 ? um : 0.0) + d) / qn[0];
-        nextsa = -((-um > 0.0 ? -um : 0.0) + d) / q[0];
-        if (coupled) sa_coupling_row(qn, su, 1.0, cpl[1]);
-      }
-    }
-    if constexpr (SA) {
-      if (!coupled) csa = sc = spiv * upsa;
-      lsa = nextsa;
-    }
-#pragma unroll
-    for (int b = 0; b < 5; ++b) put(b, L[0][b], L[1][b], L[2][b], L[3][b], L[4][b], b == 0 ? slo : (b == 1 ? spiv : 0.0), 0.0, 0.0);
-    // P = T^-1 in place
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      const double inv = 1.0 / T[i][i];
-      T[i][i] = 1.0;
-#pragma unroll
-      for (int b = 0; b < 5; ++b) T[i][b] = T[i][b] * inv;
-#pragma unroll
-      for (int a = 0; a < 5; ++a) {
-        if (a == i) continue;
-        const double f = T[a][i];
-        T[a][i] = 0.0;
-#pragma unroll
-        for (int b = 0; b < 5; ++b) T[a][b] = T[a][b] - f * T[i][b];
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < 5; ++b) put(5 + b, T[0][b], T[1][b], T[2][b], T[3][b], T[4][b], 0.0, 0.0, 0.0);
-    // C = P upper
-    if (sign != 0) {
-      double B[5][5];
-      coupling5_closed(qn, su[0], su[1], su[2], lu, g, B);
-#pragma unroll
-      for (int a = 0; a < 5; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) {
-          double m = T[a][0] * B[0][b];
-#pragma unroll
-          for (int t = 1; t < 5; ++t) m = m + T[a][t] * B[t][b];
-          C[a][b] = m;
-        }
-    } else {
-#pragma unroll
-      for (int a = 0; a < 5; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) C[a][b] = 0.0;
-    }
-#pragma unroll
-    for (int b = 0; b < 5; ++b) put(10 + b, C[0][b], C[1][b], C[2][b], C[3][b], C[4][b], b == 0 ? sc : 0.0, cpl[0][b], cpl[1][b]);
-    linked = sign != 0;
-    ll = lu;
-#pragma unroll
-    for (int m = 0; m < 3; ++m) sl[m] = -su[m];
-#pragma unroll
-    for (int v = 0; v < NV3_MAX; ++v) {
-      qb[v] = q[v];
-      q[v] = qn[v];
-    }
-  }
-  if constexpr (SA) {
-    if (!coupled) return;
-    // the SA chain from its far end: 1 / (d_k - upper_k c_{k+1}), c_k = that times lower_k
-    TF* plane = F + line_words(p);
-    double cs = 0.0;
-    for (int k = len - 1; k >= 0; --k) {
-      out -= stride;
-      const size_t at = (size_t)ch * p.chain_L + k;
-      const int c = p.ch_cells[at], up = k + 1 < len ? p.ch_sign[at] : 0, down = k > 0 ? p.ch_sign[at - 1] : 0;
-      double u = 0.0, l = 0.0;
-      if (up != 0) {
-        const int f = p.ch_face[at];
-        const double m = -(double)up * mflux[f];
-        u = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at + 1]];
-      }
-      if (down != 0) {
-        const int f = p.ch_face[at - 1];
-        const double m = (double)down * mflux[f];
-        l = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at - 1]];
-      }
-      const double piv = 1.0 / (dsa[c] - u * cs);
-      cs = piv * l;
-      out[10 * 32 + 5] = (TF)u;
-      out[11 * 32 + 5] = (TF)piv;
-      plane[(size_t)k * groups * LW_CHAINS + ch] = (TF)cs;
-    }
-  }
+  if (ch < p.n_chains) line_factor_chain<TF, SA>(p, U, lam, mflux, dflux, dflow, dsa, F, ch);
 }
 
 // z = M^-1 (s r) from the factor, s = *scale (1 where null); with vout the scaled input is also

@@ -1,11 +1,9 @@
-// The 3D wave speeds and line preconditioner, per-face and per-chain bodies (host and
-// device code; linesolve3d.cu launches them, one thread each): the reference's
+// The 3D wave speeds and line preconditioner, per-face, per-cell and per-chain bodies (host
+// and device code; linesolve3d.cu launches them, one thread each): the reference's
 // face_wave_speeds (src/jaxrans/numerics/residual.py:169-203) and line_j
 // (src/jaxrans/solvers/preconditioners.py:209-306) on a 3D plan -- 5x5 mean-flow chain
 // blocks, the SA row on its own scalar chains -- solved along each chain by the block
-// Thomas algorithm (src/jaxrans/core/linalg.py:80-132).  chain_factor_* and chain_apply_*
-// walk a chain as a whole, blocks assembled on the way (the form the host checks run); the
-// device's kernels split the same work (below).
+// Thomas algorithm (src/jaxrans/core/linalg.py:80-132).
 #pragma once
 #include "residual3d.cuh"
 
@@ -59,86 +57,6 @@ __host__ __device__ __forceinline__ double wave_speed(const Plan3Dev& p, const d
   return lam;
 }
 
-// sum over the cell's six faces of lambda (the order of cell_wave_speed_sum)
-__host__ __device__ __forceinline__ double lambda_sum(const Plan3Dev& p, const double* U, int c) {
-  const int i = c / (p.NJ * p.NK), j = (c / p.NK) % p.NJ, k = c % p.NK;
-  double total = 0.0;
-  for (int a = 0; a < 3; ++a) {
-    int h[3] = {i, j, k};
-    h[a] += 1;
-    const double lo = wave_speed(p, U, a, i, j, k), hi = wave_speed(p, U, a, h[0], h[1], h[2]);
-    total = a == 0 ? lo + hi : total + lo + hi;
-  }
-  return total;
-}
-
-// A = d(F . S)/dU (5x5, [row][variable]) by forward-mode tangents of the flux of the
-// conservative state (src/jaxrans/physics/euler.py:55-71)
-__host__ __device__ __forceinline__ void flux_jacobian3(const double* q, const double* s, double g, double A[5][5]) {
-  double U[5];
-  U[0] = q[0];
-  U[1] = q[0] * q[1];
-  U[2] = q[0] * q[2];
-  U[3] = q[0] * q[3];
-  U[4] = q[4] / (g - 1.0) + 0.5 * q[0] * ((q[1] * q[1] + q[2] * q[2]) + q[3] * q[3]);
-  for (int col = 0; col < 5; ++col) {
-    Dual Ud[5], qd[5], F[5];
-    for (int v = 0; v < 5; ++v) Ud[v] = Dual{U[v], v == col ? 1.0 : 0.0};
-    to_prim3(Ud, qd, 5, g);
-    normal_flux3(qd, s, g, F);
-    for (int r = 0; r < 5; ++r) A[r][col] = F[r].d;
-  }
-}
-
-// unpivoted Gauss-Jordan inverse (src/jaxrans/core/linalg.py:49-77)
-template <int M> __host__ __device__ __forceinline__ void invert_n(const double Mx[M][M], double Inv[M][M]) {
-  double a[M][2 * M];
-  for (int r = 0; r < M; ++r)
-    for (int c = 0; c < M; ++c) {
-      a[r][c] = Mx[r][c];
-      a[r][M + c] = r == c ? 1.0 : 0.0;
-    }
-  for (int k = 0; k < M; ++k) {
-    const double piv = a[k][k];
-    for (int c = 0; c < 2 * M; ++c) a[k][c] = a[k][c] / piv;
-    for (int r = 0; r < M; ++r) {
-      if (r == k) continue;
-      const double f = a[r][k];
-      for (int c = 0; c < 2 * M; ++c) a[r][c] = a[r][c] - f * a[k][c];
-    }
-  }
-  for (int r = 0; r < M; ++r)
-    for (int c = 0; c < M; ++c) Inv[r][c] = a[r][M + c];
-}
-
-// the link k -> k+1 of a chain: its face vector (outward from cell k) and lambda there
-__host__ __device__ __forceinline__ void link_face(const Plan3Dev& p, const double* U, int flat, double s[3],
-                                                   double& lam) {
-  int a, i, j, k;
-  face_of(p, flat, a, i, j, k);
-  face_vector(p, a, i, j, k, s);
-  lam = wave_speed(p, U, a, i, j, k);
-}
-
-// 1/2 A(q_nb, sign S) - 1/2 lambda I
-__host__ __device__ __forceinline__ void coupling5(const double* qnb, const double* s, double sign, double lam,
-                                                   double g, double B[5][5]) {
-  const double ss[3] = {sign * s[0], sign * s[1], sign * s[2]};
-  double A[5][5];
-  flux_jacobian3(qnb, ss, g, A);
-  for (int r = 0; r < 5; ++r)
-    for (int c = 0; c < 5; ++c) B[r][c] = 0.5 * A[r][c] - (r == c ? 0.5 * lam : 0.0);
-}
-
-// The line_j factor of one chain (block Thomas, src/jaxrans/core/linalg.py:80-132, and the
-// scalar SA chain): for element k of the chain, the block toward k-1 (lower_k), the
-// inverse pivot P_k = (D_k - lower_k C_{k-1})^-1 and C_k = P_k upper_k -- 75 entries -- and
-// on the SA row the same three scalars.  Entry e of element k of chain ch is stored at
-// F[(k * FACTOR3 + e) * n_chains + ch]: neighbouring chains' threads read neighbouring
-// words.  The apply is then z_k = P_k (r_k - lower_k d_{k-1}) down the chain and
-// x_k = d_k - C_k x_{k+1} back up, the factor computed once per Newton step.
-constexpr int F3_LOWER = 0, F3_PIV = 25, F3_CHAT = 50, F3_SA = 75, F3_CPL_LO = 78, F3_CPL_UP = 83;
-
 // the SA row's coupling to a neighbour's mean flow: half the Jacobian of rho nu_hat V.S'
 // with respect to its (rho, rho u, rho v, rho w, rho E) at its state qnb, S' = sign S:
 // [-nu_hat vn, nu_hat S'x, nu_hat S'y, nu_hat S'z, 0]
@@ -154,235 +72,7 @@ __host__ __device__ __forceinline__ void sa_coupling_row(const double* qnb, cons
   row[4] = 0.5 * 0.0;
 }
 
-__host__ __device__ __forceinline__ size_t factor_at(const Plan3Dev& p, int ch, int k, int e) {
-  return ((size_t)k * FACTOR3 + e) * p.n_chains + ch;
-}
-
-__host__ __device__ __forceinline__ int chain_length(const Plan3Dev& p, int ch) {
-  const int* cells = p.ch_cells + (size_t)ch * p.chain_L;
-  int len = 0;
-  while (len < p.chain_L && cells[len] >= 0) ++len;
-  return len;
-}
-
-template <class TF>
-inline __host__ __device__ void chain_factor_flow(const Plan3Dev& p, const double* U, double cfl, int ch, TF* F) {
-  const int L = p.chain_L;
-  const double g = p.P.gamma;
-  const int* cells = p.ch_cells + (size_t)ch * L;
-  const int len = chain_length(p, ch);
-  double cprev[5][5] = {};
-  double lower[5][5] = {};   // row k's block toward cell k-1
-  double cpl_lower[5] = {};  // the coupled form: the SA row k's coupling to cell k-1's mean flow
-  for (int k = 0; k < len; ++k) {
-    const int c = cells[k];
-    const double dg = lambda_sum(p, U, c) * (1.0 / cfl + 0.5);
-    double upper[5][5] = {}, lower_next[5][5] = {};
-    double cpl_upper[5] = {}, cpl_lower_next[5] = {};
-    const int sign = k + 1 < len ? p.ch_sign[(size_t)ch * L + k] : 0;
-    if (sign != 0) {
-      double s[3], lam, qn[NV3_MAX], qc[NV3_MAX];
-      link_face(p, U, p.ch_face[(size_t)ch * L + k], s, lam);
-      prim_at(p, U, cells[k + 1], qn);
-      prim_at(p, U, c, qc);
-      coupling5(qn, s, (double)sign, lam, g, upper);
-      coupling5(qc, s, (double)-sign, lam, g, lower_next);
-      if (p.line_coupled && p.nvar > 5) {
-        sa_coupling_row(qn, s, (double)sign, cpl_upper);
-        sa_coupling_row(qc, s, (double)-sign, cpl_lower_next);
-      }
-    }
-    if (p.line_coupled && p.nvar > 5)
-      for (int t = 0; t < 5; ++t) {
-        F[factor_at(p, ch, k, F3_CPL_LO + t)] = (TF)cpl_lower[t];
-        F[factor_at(p, ch, k, F3_CPL_UP + t)] = (TF)cpl_upper[t];
-        cpl_lower[t] = cpl_lower_next[t];
-      }
-    // P = inv(D - lower c_prev); chat = P upper
-    double T[5][5], piv[5][5];
-    for (int a = 0; a < 5; ++a)
-      for (int b = 0; b < 5; ++b) {
-        double m = lower[a][0] * cprev[0][b];
-        for (int t = 1; t < 5; ++t) m = m + lower[a][t] * cprev[t][b];
-        T[a][b] = (a == b ? dg : 0.0) - m;
-      }
-    invert_n<5>(T, piv);
-    for (int a = 0; a < 5; ++a)
-      for (int b = 0; b < 5; ++b) {
-        double m = piv[a][0] * upper[0][b];
-        for (int t = 1; t < 5; ++t) m = m + piv[a][t] * upper[t][b];
-        cprev[a][b] = m;
-        F[factor_at(p, ch, k, F3_LOWER + a * 5 + b)] = (TF)lower[a][b];
-        F[factor_at(p, ch, k, F3_PIV + a * 5 + b)] = (TF)piv[a][b];
-        F[factor_at(p, ch, k, F3_CHAT + a * 5 + b)] = (TF)m;
-      }
-    for (int a = 0; a < 5; ++a)
-      for (int b = 0; b < 5; ++b) lower[a][b] = lower_next[a][b];
-  }
-}
-
-// z = M^-1 r on the mean-flow rows of chain ch from its factor; d_k is kept in z between
-// the two sweeps
-template <class TF>
-inline __host__ __device__ void chain_apply_flow(const Plan3Dev& p, int ch, const TF* F, const double* r, double* z) {
-  const int n = p.NI * p.NJ * p.NK;
-  const int* cells = p.ch_cells + (size_t)ch * p.chain_L;
-  const int len = chain_length(p, ch);
-  TF dprev[5] = {};
-  for (int k = 0; k < len; ++k) {
-    const int c = cells[k];
-    TF rhs[5];
-    for (int a = 0; a < 5; ++a) {
-      TF m = F[factor_at(p, ch, k, F3_LOWER + a * 5)] * dprev[0];
-      for (int t = 1; t < 5; ++t) m = m + F[factor_at(p, ch, k, F3_LOWER + a * 5 + t)] * dprev[t];
-      rhs[a] = (TF)r[(size_t)a * n + c] - m;
-    }
-    for (int a = 0; a < 5; ++a) {
-      TF m = F[factor_at(p, ch, k, F3_PIV + a * 5)] * rhs[0];
-      for (int t = 1; t < 5; ++t) m = m + F[factor_at(p, ch, k, F3_PIV + a * 5 + t)] * rhs[t];
-      dprev[a] = m;
-      z[(size_t)a * n + c] = (double)m;
-    }
-  }
-  TF nxt[5] = {};
-  for (int k = len - 1; k >= 0; --k) {
-    const int c = cells[k];
-    TF x[5];
-    for (int a = 0; a < 5; ++a) {
-      TF m = F[factor_at(p, ch, k, F3_CHAT + a * 5)] * nxt[0];
-      for (int t = 1; t < 5; ++t) m = m + F[factor_at(p, ch, k, F3_CHAT + a * 5 + t)] * nxt[t];
-      x[a] = (TF)z[(size_t)a * n + c] - m;
-    }
-    for (int a = 0; a < 5; ++a) {
-      nxt[a] = x[a];
-      z[(size_t)a * n + c] = (double)x[a];
-    }
-  }
-}
-
-// the SA row's face terms at face (a, i, j, k): mass flux rho V.S and diffusion kappa |S|^2 / V
-__host__ __device__ __forceinline__ void sa_face_terms(const Plan3Dev& p, const double* U, int a, int i, int j, int k,
-                                                       double& m, double& d) {
-  const Physics3& P = p.P;
-  double qf[NV3_MAX], vol, s[3];
-  face_average(p, U, a, i, j, k, qf, vol);
-  face_vector(p, a, i, j, k, s);
-  const double mu = viscosity3(P, P.gamma * qf[4] / qf[0]);
-  const double kap = diffusion_coefficient(P.sa, qf[0], qf[5] * P.mu_inf, mu);
-  m = qf[0] * ((qf[1] * s[0] + qf[2] * s[1]) + qf[3] * s[2]);
-  d = kap * ((s[0] * s[0] + s[1] * s[1]) + s[2] * s[2]) / vol;
-}
-
-// the SA chain diagonal of cell c (src/jaxrans/solvers/preconditioners.py:235-270)
-inline __host__ __device__ double sa_diagonal(const Plan3Dev& p, const double* U, double cfl, int c) {
-  const Physics3& P = p.P;
-  const double g = P.gamma;
-  const int i = c / (p.NJ * p.NK), j = (c / p.NK) % p.NJ, k = c % p.NK;
-  double diag = 0.0;
-  double gv[3][3];   // Green-Gauss of face-averaged velocity: gv[direction][component]
-  for (int dir = 0; dir < 3; ++dir)
-    for (int m = 0; m < 3; ++m) gv[dir][m] = 0.0;
-  double vsum[3][3][3];   // per family: hi*S_hi - lo*S_lo, [family][direction][component]
-  for (int a = 0; a < 3; ++a) {
-    int h[3] = {i, j, k};
-    h[a] += 1;
-    double mlo, dlo, mhi, dhi;
-    sa_face_terms(p, U, a, i, j, k, mlo, dlo);
-    sa_face_terms(p, U, a, h[0], h[1], h[2], mhi, dhi);
-    const double out_hi = (mhi > 0.0 ? mhi : 0.0) + dhi;
-    const double in_lo = (-mlo > 0.0 ? -mlo : 0.0) + dlo;
-    diag = a == 0 ? out_hi + in_lo : diag + out_hi + in_lo;
-    double ql[NV3_MAX], qh[NV3_MAX], vl, vh, sl[3], sh[3];
-    face_average(p, U, a, i, j, k, ql, vl);
-    face_average(p, U, a, h[0], h[1], h[2], qh, vh);
-    face_vector(p, a, i, j, k, sl);
-    face_vector(p, a, h[0], h[1], h[2], sh);
-    for (int dir = 0; dir < 3; ++dir)
-      for (int m = 0; m < 3; ++m) vsum[a][dir][m] = qh[1 + m] * sh[dir] - ql[1 + m] * sl[dir];
-  }
-  const double vol = p.volume[c];
-  for (int dir = 0; dir < 3; ++dir)
-    for (int m = 0; m < 3; ++m) gv[dir][m] = ((vsum[0][dir][m] + vsum[1][dir][m]) + vsum[2][dir][m]) / vol;
-  double q[NV3_MAX];
-  prim_at(p, U, c, q);
-  diag = diag / q[0];
-  const double cx = gv[1][2] - gv[2][1], cy = gv[2][0] - gv[0][2], cz = gv[0][1] - gv[1][0];
-  const double sq = (cx * cx + cy * cy) + cz * cz;
-  const double omega = sq > 0.0 ? sqrt(sq) : 0.0;
-  const double nu = viscosity3(P, g * q[4] / q[0]) / q[0];
-  const double dist = p.distance[c];
-  const double st = s_tilde(P.sa, omega, q[5] * P.mu_inf, nu, dist);
-  const double fw = f_w(P.sa, r_of(P.sa, q[5] * P.mu_inf, st, dist));
-  const double dest = q[5] > 0.0 ? 2.0 * P.sa.c_w1 * fw * P.mu_inf * q[5] / (dist * dist) : 0.0;
-  return diag + dest * vol + lambda_sum(p, U, c) / cfl;
-}
-
-// the SA row's factor of chain ch (scalar Thomas): lower_k, 1 / (d_k - lower_k c_{k-1}), c_k
-template <class TF>
-inline __host__ __device__ void chain_factor_sa(const Plan3Dev& p, const double* U, double cfl, int ch, TF* F) {
-  const int L = p.chain_L;
-  const int* cells = p.ch_cells + (size_t)ch * L;
-  const int len = chain_length(p, ch);
-  double cprev = 0.0, lower = 0.0;
-  for (int k = 0; k < len; ++k) {
-    const int c = cells[k];
-    const double dg = sa_diagonal(p, U, cfl, c);
-    double upper = 0.0, lower_next = 0.0;
-    const int sign = k + 1 < len ? p.ch_sign[(size_t)ch * L + k] : 0;
-    if (sign != 0) {
-      int a, i, j, kk;
-      face_of(p, p.ch_face[(size_t)ch * L + k], a, i, j, kk);
-      double m, d;
-      sa_face_terms(p, U, a, i, j, kk, m, d);
-      const double rho_up = U[cells[k + 1]], rho_c = U[c];
-      const double up_m = -(double)sign * m, down_m = (double)sign * m;
-      upper = -((up_m > 0.0 ? up_m : 0.0) + d) / rho_up;
-      lower_next = -((down_m > 0.0 ? down_m : 0.0) + d) / rho_c;
-    }
-    const double piv = 1.0 / (dg - lower * cprev);
-    cprev = piv * upper;
-    F[factor_at(p, ch, k, F3_SA)] = (TF)lower;
-    F[factor_at(p, ch, k, F3_SA + 1)] = (TF)piv;
-    F[factor_at(p, ch, k, F3_SA + 2)] = (TF)cprev;
-    lower = lower_next;
-  }
-}
-
-// z = M^-1 r on the SA row of chain ch; in the coupled form after the mean flow's apply,
-// the right-hand side less the coupling to the neighbours' z (block forward substitution)
-template <class TF>
-inline __host__ __device__ void chain_apply_sa(const Plan3Dev& p, int ch, const TF* F, const double* r, double* z) {
-  const int n = p.NI * p.NJ * p.NK;
-  const int* cells = p.ch_cells + (size_t)ch * p.chain_L;
-  const int len = chain_length(p, ch);
-  TF dprev = 0;
-  for (int k = 0; k < len; ++k) {
-    const int c = cells[k];
-    TF rhs = (TF)r[(size_t)5 * n + c];
-    if (p.line_coupled) {
-      TF lo = 0, up = 0;
-      if (k > 0) {
-        lo = F[factor_at(p, ch, k, F3_CPL_LO)] * (TF)z[cells[k - 1]];
-        for (int t = 1; t < 5; ++t) lo = lo + F[factor_at(p, ch, k, F3_CPL_LO + t)] * (TF)z[(size_t)t * n + cells[k - 1]];
-      }
-      if (k + 1 < len) {
-        up = F[factor_at(p, ch, k, F3_CPL_UP)] * (TF)z[cells[k + 1]];
-        for (int t = 1; t < 5; ++t) up = up + F[factor_at(p, ch, k, F3_CPL_UP + t)] * (TF)z[(size_t)t * n + cells[k + 1]];
-      }
-      rhs = rhs - (lo + up);
-    }
-    dprev = F[factor_at(p, ch, k, F3_SA + 1)] * (rhs - F[factor_at(p, ch, k, F3_SA)] * dprev);
-    z[(size_t)5 * n + c] = (double)dprev;
-  }
-  TF nxt = 0;
-  for (int k = len - 1; k >= 0; --k) {
-    const int c = cells[k];
-    nxt = (TF)z[(size_t)5 * n + c] - F[factor_at(p, ch, k, F3_SA + 2)] * nxt;
-    z[(size_t)5 * n + c] = (double)nxt;
-  }
-}
-
-// ---- the device's form: the same factor and solve split by what can run in parallel.
+// ---- the factor and the solve, split by what can run in parallel.
 // k3_line_faces makes each face's wave speed (and, SA, mass flux and diffusion) once instead
 // of once from either side and again for the link, k3_line_cells each cell's diagonals,
 // k3_line_factor the elimination down a chain, one thread a chain, and k3_line_apply the two
@@ -430,7 +120,7 @@ __host__ __device__ __forceinline__ void line_face_terms(const Plan3Dev& p, cons
 }
 
 // The diagonals of cell c from its faces' terms: the sum of lambda, and (SA) the SA chain's
-// diagonal (sa_diagonal)
+// diagonal (src/jaxrans/solvers/preconditioners.py:235-270)
 template <bool SA>
 __host__ __device__ __forceinline__ void line_cell_terms(const Plan3Dev& p, const double* U, const double* lam,
                                                          const double* mflux, const double* dflux, double cfl, int c,
@@ -480,7 +170,7 @@ __host__ __device__ __forceinline__ void line_cell_terms(const Plan3Dev& p, cons
 }
 
 // A = d(F . S)/dU (5x5, [row][variable]) of the conservative state whose primitives are q, in
-// closed form, then 1/2 A - 1/2 lam I (coupling5 without its dual-number columns)
+// closed form (src/jaxrans/physics/euler.py:55-71), then 1/2 A - 1/2 lam I
 __host__ __device__ __forceinline__ void coupling5_closed(const double* q, double sx, double sy, double sz, double lam,
                                                           double g, double B[5][5]) {
   const double S[3] = {sx, sy, sz};
@@ -517,6 +207,170 @@ constexpr int LW_WORDS = 15, LW_ROWS = 8, LW_CHAINS = 4;
 __host__ __device__ __forceinline__ int line_groups(const Plan3Dev& p) { return (p.n_chains + LW_CHAINS - 1) / LW_CHAINS; }
 __host__ __device__ __forceinline__ size_t line_words(const Plan3Dev& p) {
   return (size_t)p.chain_L * line_groups(p) * LW_WORDS * LW_ROWS * LW_CHAINS;
+}
+
+// The elimination down chain ch: T = D - lower C_{k-1}, P = T^-1 (Gauss-Jordan, one reciprocal a
+// pivot), C = P upper, and the SA row's scalars, from the faces' terms (lam, mflux, dflux) and the
+// cells' diagonals (dflow, dsa); its rows leave eight at a time.
+template <class TF, bool SA>
+__host__ __device__ __forceinline__ void line_factor_chain(const Plan3Dev& p, const double* __restrict__ U,
+                                                           const double* __restrict__ lam,
+                                                           const double* __restrict__ mflux,
+                                                           const double* __restrict__ dflux,
+                                                           const double* __restrict__ dflow,
+                                                           const double* __restrict__ dsa, TF* __restrict__ F, int ch) {
+  const double g = p.P.gamma;
+  const int groups = line_groups(p), len = p.ch_len[ch];
+  TF* out = F + ((size_t)(ch / LW_CHAINS) * LW_WORDS) * 32 + (ch % LW_CHAINS) * LW_ROWS;
+  const size_t stride = (size_t)groups * LW_WORDS * 32;
+  const bool coupled = SA && p.line_coupled;
+  double C[5][5] = {}, q[NV3_MAX] = {}, qb[NV3_MAX] = {};   // this cell's state, the one below's
+  double sl[3] = {0.0, 0.0, 0.0}, ll = 0.0, csa = 0.0, lsa = 0.0;   // the link below, outward from this cell
+  bool linked = false;
+  if (len > 0) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L], q);
+  for (int k = 0; k < len; ++k, out += stride) {
+    const int c = p.ch_cells[(size_t)ch * p.chain_L + k];
+    double T[5][5], L[5][5];
+    if (linked) coupling5_closed(qb, sl[0], sl[1], sl[2], ll, g, L);
+    else
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) L[a][b] = 0.0;
+    const double dg = dflow[c];
+#pragma unroll
+    for (int a = 0; a < 5; ++a)
+#pragma unroll
+      for (int b = 0; b < 5; ++b) {
+        double m = L[a][0] * C[0][b];
+#pragma unroll
+        for (int t = 1; t < 5; ++t) m = m + L[a][t] * C[t][b];
+        T[a][b] = (a == b ? dg : 0.0) - m;
+      }
+    // the SA row's scalars beside the mean flow's blocks, and the coupled form's rows
+    double slo = 0.0, spiv = 0.0, sc = 0.0, cpl[2][5] = {};
+    if constexpr (SA) {
+      if (!coupled) {
+        slo = lsa;
+        spiv = 1.0 / (dsa[c] - lsa * csa);
+      } else if (linked) {
+        sa_coupling_row(qb, sl, 1.0, cpl[0]);
+      }
+    }
+    // word w of the rows: the first six, or all eight
+    auto put = [&](int w, double r0, double r1, double r2, double r3, double r4, double r5, double r6, double r7) {
+      TF* o = out + w * 32;
+      if constexpr (sizeof(TF) == 4) {
+        *reinterpret_cast<float4*>(o) = make_float4((float)r0, (float)r1, (float)r2, (float)r3);
+        *reinterpret_cast<float4*>(o + 4) = make_float4((float)r4, (float)r5, (float)r6, (float)r7);
+      } else {
+        *reinterpret_cast<double2*>(o) = make_double2(r0, r1);
+        *reinterpret_cast<double2*>(o + 2) = make_double2(r2, r3);
+        *reinterpret_cast<double2*>(o + 4) = make_double2(r4, r5);
+        if (coupled) *reinterpret_cast<double2*>(o + 6) = make_double2(r6, r7);
+      }
+    };
+    // the link above: this cell's upper block and, for the next element, its lower one
+    const int sign = k + 1 < len ? p.ch_sign[(size_t)ch * p.chain_L + k] : 0;
+    double su[3] = {0.0, 0.0, 0.0}, lu = 0.0, qn[NV3_MAX] = {}, upsa = 0.0, nextsa = 0.0;
+    if (k + 1 < len) prim_at_n<SA ? 6 : 5>(p, U, p.ch_cells[(size_t)ch * p.chain_L + k + 1], qn);
+    if (sign != 0) {
+      const int f = p.ch_face[(size_t)ch * p.chain_L + k];
+      int fa, fi, fj, fk;
+      face_of(p, f, fa, fi, fj, fk);
+      face_vector(p, fa, fi, fj, fk, su);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) su[m] *= (double)sign;
+      lu = lam[f];
+      if constexpr (SA) {
+        const double um = -(double)sign * mflux[f], d = dflux[f];
+        upsa = -((um > 0.0 ? um : 0.0) + d) / qn[0];
+        nextsa = -((-um > 0.0 ? -um : 0.0) + d) / q[0];
+        if (coupled) sa_coupling_row(qn, su, 1.0, cpl[1]);
+      }
+    }
+    if constexpr (SA) {
+      if (!coupled) csa = sc = spiv * upsa;
+      lsa = nextsa;
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(b, L[0][b], L[1][b], L[2][b], L[3][b], L[4][b], b == 0 ? slo : (b == 1 ? spiv : 0.0), 0.0, 0.0);
+    // P = T^-1 in place
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const double inv = 1.0 / T[i][i];
+      T[i][i] = 1.0;
+#pragma unroll
+      for (int b = 0; b < 5; ++b) T[i][b] = T[i][b] * inv;
+#pragma unroll
+      for (int a = 0; a < 5; ++a) {
+        if (a == i) continue;
+        const double f = T[a][i];
+        T[a][i] = 0.0;
+#pragma unroll
+        for (int b = 0; b < 5; ++b) T[a][b] = T[a][b] - f * T[i][b];
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(5 + b, T[0][b], T[1][b], T[2][b], T[3][b], T[4][b], 0.0, 0.0, 0.0);
+    // C = P upper
+    if (sign != 0) {
+      double B[5][5];
+      coupling5_closed(qn, su[0], su[1], su[2], lu, g, B);
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) {
+          double m = T[a][0] * B[0][b];
+#pragma unroll
+          for (int t = 1; t < 5; ++t) m = m + T[a][t] * B[t][b];
+          C[a][b] = m;
+        }
+    } else {
+#pragma unroll
+      for (int a = 0; a < 5; ++a)
+#pragma unroll
+        for (int b = 0; b < 5; ++b) C[a][b] = 0.0;
+    }
+#pragma unroll
+    for (int b = 0; b < 5; ++b) put(10 + b, C[0][b], C[1][b], C[2][b], C[3][b], C[4][b], b == 0 ? sc : 0.0, cpl[0][b], cpl[1][b]);
+    linked = sign != 0;
+    ll = lu;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) sl[m] = -su[m];
+#pragma unroll
+    for (int v = 0; v < NV3_MAX; ++v) {
+      qb[v] = q[v];
+      q[v] = qn[v];
+    }
+  }
+  if constexpr (SA) {
+    if (!coupled) return;
+    // the SA chain from its far end: 1 / (d_k - upper_k c_{k+1}), c_k = that times lower_k
+    TF* plane = F + line_words(p);
+    double cs = 0.0;
+    for (int k = len - 1; k >= 0; --k) {
+      out -= stride;
+      const size_t at = (size_t)ch * p.chain_L + k;
+      const int c = p.ch_cells[at], up = k + 1 < len ? p.ch_sign[at] : 0, down = k > 0 ? p.ch_sign[at - 1] : 0;
+      double u = 0.0, l = 0.0;
+      if (up != 0) {
+        const int f = p.ch_face[at];
+        const double m = -(double)up * mflux[f];
+        u = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at + 1]];
+      }
+      if (down != 0) {
+        const int f = p.ch_face[at - 1];
+        const double m = (double)down * mflux[f];
+        l = -((m > 0.0 ? m : 0.0) + dflux[f]) / U[p.ch_cells[at - 1]];
+      }
+      const double piv = 1.0 / (dsa[c] - u * cs);
+      cs = piv * l;
+      out[10 * 32 + 5] = (TF)u;
+      out[11 * 32 + 5] = (TF)piv;
+      plane[(size_t)k * groups * LW_CHAINS + ch] = (TF)cs;
+    }
+  }
 }
 
 }  // namespace jr

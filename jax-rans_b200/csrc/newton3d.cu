@@ -363,7 +363,8 @@ template <int E> static void orthogonalise(DeviceOps3& o, int j, int m) {
   update(g->h2, 1);
 }
 
-// gmres3 (newton3d.cuh) with an Arnoldi step's scalars on the device
+// Right-preconditioned restarted GMRES (src/jaxrans/solvers/krylov.py:34-97), an Arnoldi step's scalars
+// on the device: (V/dt + J) X = B, ACTION = A X
 int gmres3(DeviceOps3& ops, const double* U, double cfl, const Newton3Config& c, int B, int X, int ACTION) {
   const double tiny = 2.2250738585072014e-308;
   const double rcond = 2.220446049250313e-16 * (c.restart + 1);

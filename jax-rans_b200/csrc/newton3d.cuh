@@ -1,7 +1,7 @@
 // The 3D pseudo-transient Newton step: right-preconditioned restarted GMRES with CGS2
 // and Givens least squares (src/jaxrans/solvers/krylov.py:34-137), the relaxation, the
 // acceptance test and the CFL ramp (src/jaxrans/solvers/implicit.py:54-168), driven on
-// the host over vector operations `Ops` supplies.  On the device (capi3d.cu) the
+// the host over vector operations `Ops` supplies.  On the device (newton3d.cu) the
 // operations are kernels; a test-only host harness supplies loops, so this logic is
 // checked against the reference without a GPU.
 #pragma once
@@ -50,63 +50,12 @@ inline void givens_lstsq(const std::vector<double>& Hc, int m, double beta, doub
   }
 }
 
-// Ops: vectors by index -- R_, Z_, W_, T_ (GMRES work), RES_, B_, DU_, ACT_ (the step's),
-// V(i) the basis -- each of the canvas length N = nvar * cells; the state U is the
-// caller's.  Operations: prepare(U, cfl) (V/dt, the line factor), residual, matvec
-// (V/dt z + J1 z), precondition, dot, mdot (the dots of V(0..count-1) with a vector, as
-// that many dots), maxpy (y += sum of coef_i V(i), as that many axpys in order), nrm2,
-// axpy, scale, copy, zero, density_norm, worst_ratio, physical_after, add_to_state.
-template <class Ops>
-int gmres3(Ops& ops, const double* U, double cfl, const Newton3Config& c, int B, int X, int ACTION) {
-  // solves (V/dt + J) X = B; ACTION = the Arnoldi action A X
-  const double tiny = 2.2250738585072014e-308;
-  const double rcond = 2.220446049250313e-16 * (c.restart + 1);
-  const int m = c.restart;
-  auto prec = [&](int src, int dst) {
-    if (c.preconditioner >= 1) ops.precondition(U, cfl, src, dst);
-    else ops.copy(src, dst);
-  };
-  const double bn = ops.nrm2(B);
-  ops.zero(X);
-  ops.copy(B, Ops::R_);
-  ops.zero(ACTION);
-  std::vector<double> H((size_t)(m + 1) * m), h(m + 1), h2(m + 1), neg(m + 1), y, Hy(m + 1);
-  for (int k = 0; k < c.maxiter; ++k) {
-    const double rn = ops.nrm2(Ops::R_);
-    if (!(rn > c.tol * bn)) break;
-    const double beta = rn;
-    ops.scale(1.0 / std::fmax(beta, tiny), Ops::R_, ops.V(0));
-    std::fill(H.begin(), H.end(), 0.0);
-    for (int j = 0; j < m; ++j) {
-      prec(ops.V(j), Ops::Z_);
-      ops.matvec(U, cfl, Ops::Z_, Ops::W_);
-      ops.mdot(j + 1, Ops::W_, h.data());
-      for (int i = 0; i <= j; ++i) neg[i] = -h[i];
-      ops.maxpy(j + 1, neg.data(), Ops::W_);
-      ops.mdot(j + 1, Ops::W_, h2.data());
-      for (int i = 0; i <= j; ++i) neg[i] = -h2[i];
-      ops.maxpy(j + 1, neg.data(), Ops::W_);
-      const double nrm = ops.nrm2(Ops::W_);
-      for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = h[i] + h2[i];
-      H[(size_t)(j + 1) * m + j] = nrm;
-      ops.scale(1.0 / std::fmax(nrm, tiny), Ops::W_, ops.V(j + 1));
-    }
-    givens_lstsq(H, m, beta, rcond, y);
-    ops.zero(Ops::T_);
-    ops.maxpy(m, y.data(), Ops::T_);
-    prec(Ops::T_, Ops::Z_);
-    ops.axpy(1.0, Ops::Z_, X);
-    for (int i = 0; i <= m; ++i) {
-      double s = 0.0;
-      for (int j = 0; j < m; ++j) s = s + H[(size_t)i * m + j] * y[j];
-      Hy[i] = s;
-    }
-    ops.maxpy(m + 1, Hy.data(), ACTION);
-    ops.copy(B, Ops::R_);
-    ops.axpy(-1.0, ACTION, Ops::R_);
-  }
-  return 0;
-}
+// Ops: vectors by index -- RES_, B_, DU_, ACT_ (the step's) and T_ (work) -- each of the
+// canvas length N = nvar * cells; the state U is the caller's.  Operations: prepare(U, cfl)
+// (V/dt, the line factor, the linearisation), residual, nrm2, axpy, scale, density_norm,
+// worst_ratio, physical_after, add_to_state; and gmres3(ops, U, cfl, c, B, X, ACTION), found by
+// its argument: X of (V/dt + J) X = B by restarted GMRES, ACTION = A X by the Arnoldi relation
+// (on the device newton3d.cu's, its scalars kept there).
 
 // One Newton step on the state (U in place); returns |R| before the update.
 template <class Ops>

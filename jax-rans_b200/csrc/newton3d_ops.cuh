@@ -56,7 +56,7 @@ struct DeviceOps3 {
   void bind(double* work, Gmres3* scalars, int m);
 };
 
-// the cycles of gmres3 (newton3d.cuh) on the device's scalars; newton_step3 takes this overload
+// the gmres3 newton_step3 (newton3d.cuh) finds for DeviceOps3
 int gmres3(DeviceOps3& ops, const double* U, double cfl, const Newton3Config& c, int B, int X, int ACTION);
 
 double newton_step3_device(DeviceOps3& ops, double* U, double& cfl, double& res_prev, const Newton3Config& c);

@@ -1,6 +1,9 @@
-// The physics of a 3D plan from its C-ABI descriptor (shared by the plan builder and
-// the host check of the 3D kernels' bodies).
+// What a 3D plan makes of its C-ABI descriptor on the host: the physics, the ghost programs,
+// the chains' tables (shared by the plan builder and the host check of the 3D kernels' bodies).
 #pragma once
+#include <algorithm>
+#include <vector>
+
 #include "../../include/jaxrans_b200.h"
 #include "device3d.cuh"
 
@@ -51,6 +54,55 @@ inline void force_coefficients3(const Physics3& P, int n_walls, const double* lo
   out[1] = cd / q_area;
   out[2] = cm / q_area;
   out[3] = ((drag[0] * shear[0] + drag[1] * shear[1]) + drag[2] * shear[2]) / q_area;
+}
+
+// Every ghost's program (Plan3Dev::ghost_of): the record that writes it last, back through
+// the records that had filled each source before its stage, to a cell of its own state.
+inline void ghost_programs(const jr_plan3d_desc* d, size_t n, std::vector<int>& ghost_of, std::vector<int>& root,
+                           std::vector<int>& off, std::vector<int>& rec) {
+  std::vector<int> last(n, -1), parent;
+  int at = 0, total = 0;
+  for (int s = 0; s < d->n_stages; ++s) total += d->stage_records[s];
+  parent.reserve(total);
+  for (int s = 0; s < d->n_stages; ++s) {
+    const int end = at + d->stage_records[s];
+    for (int r = at; r < end; ++r) parent.push_back(last[d->source[r]]);
+    for (int r = at; r < end; ++r) last[d->ghost[r]] = r;
+    at = end;
+  }
+  ghost_of.assign(n, -1);
+  off.assign(1, 0);
+  off.reserve((size_t)total + 1);
+  root.reserve(total);
+  std::vector<int> chain;
+  for (int w = 0; w < total; ++w) {
+    if (last[d->ghost[w]] != w) continue;   // written again by a later record
+    ghost_of[d->ghost[w]] = (int)root.size();
+    chain.clear();
+    int r = w;
+    for (;; r = parent[r]) {
+      if (d->kind[r] != 0) chain.push_back(r);
+      if (parent[r] < 0) break;
+    }
+    root.push_back(d->source[r]);
+    rec.insert(rec.end(), chain.rbegin(), chain.rend());
+    off.push_back((int)rec.size());
+  }
+}
+
+// each chain's length (to its first -1) and the cells on none
+inline void chain_tables(const jr_plan3d_desc* d, size_t n, std::vector<int>& len, std::vector<int>& offchain) {
+  std::vector<char> on(n, 0);
+  len.resize(d->n_chains);
+  for (int c = 0; c < d->n_chains; ++c) {
+    const int* cells = d->chain_cells + (size_t)c * d->chain_L;
+    int k = 0;
+    for (; k < d->chain_L && cells[k] >= 0; ++k) on[cells[k]] = 1;
+    len[c] = k;
+  }
+  offchain.reserve(n - std::min(n, (size_t)d->n_chains * d->chain_L));
+  for (size_t c = 0; c < n; ++c)
+    if (!on[c]) offchain.push_back((int)c);
 }
 
 }  // namespace jr

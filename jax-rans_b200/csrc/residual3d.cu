@@ -102,7 +102,7 @@ static void face_parts(const Plan3Dev& p, const T* A, int nf, cudaStream_t st) {
     const int nn = node_count(p);
     k3_node_phi<T, SA ? 5 : 4><<<(nn + 127) / 128, 128, 0, st>>>(p, A);
     if constexpr (sizeof(T) == sizeof(double)) {
-      k3_face_flux<T, VISC, SA, FO, 3><<<fblocks, 128, 0, st>>>(p, A, nf);
+      k3_face_flux<T, VISC, SA, FO, 0><<<fblocks, 128, 0, st>>>(p, A, nf);
     } else {
       counted3(1);
       k3_face_flux<T, VISC, SA, FO, 1><<<fblocks, 128, 0, st>>>(p, A, nf);

@@ -8,17 +8,8 @@
 
 namespace jr {
 
-// the primitive state of canvas cell c from conservative U (and the tangent dU for Dual)
-template <class T>
-__host__ __device__ __forceinline__ void prim_cell(const Plan3Dev& p, const double* U, const double* dU, T* Q, int c) {
-  const int n = p.NI * p.NJ * p.NK;
-  T u[NV3_MAX], q[NV3_MAX];
-  for (int v = 0; v < p.nvar; ++v) u[v] = mk<T>(U[(size_t)v * n + c], dU ? dU[(size_t)v * n + c] : 0.0);
-  to_prim3(u, q, p.nvar, p.P.gamma);
-  for (int v = 0; v < p.nvar; ++v) Q[(size_t)v * n + c] = q[v];
-}
-
-// the same with the plan's variable count NV (== p.nvar) fixed at compile time
+// the primitive state of canvas cell c from conservative U (and the tangent dU for Dual); NV ==
+// p.nvar, fixed at compile time
 template <int NV, class T>
 __host__ __device__ __forceinline__ void prim_cell_n(const Plan3Dev& p, const double* U, const double* dU, T* Q,
                                                      int c) {
@@ -29,41 +20,6 @@ __host__ __device__ __forceinline__ void prim_cell_n(const Plan3Dev& p, const do
   to_prim3(u, q, NV, p.P.gamma);
 #pragma unroll
   for (int v = 0; v < NV; ++v) Q[(size_t)v * n + c] = q[v];
-}
-
-// ghost record r of a stage: out[ghost] = condition(in[source]) (or a copy across a cut)
-template <class T>
-__host__ __device__ __forceinline__ void ghost_record(const Plan3Dev& p, const T* in, T* out, int r) {
-  const int n = p.NI * p.NJ * p.NK;
-  const int ghost = p.g_ghost[r], src = p.g_source[r], kind = p.g_kind[r];
-  if (ghost < 0 || ghost >= n || src < 0 || src >= n) return;   // validated on the host
-  T q[NV3_MAX], o[NV3_MAX];
-  for (int v = 0; v < p.nvar; ++v) q[v] = in[(size_t)v * n + src];
-  condition3(kind, q, p.g_normal[3 * r], p.g_normal[3 * r + 1], p.g_normal[3 * r + 2], p.P, p.nvar, o);
-  for (int v = 0; v < p.nvar; ++v) out[(size_t)v * n + ghost] = o[v];
-}
-
-// The same stage in place, in two passes: every record's value from the canvas as it was
-// before the stage (into buf, slot r - r0 of count), then every value to its ghost.  A
-// stage writes each ghost once, so the two passes give the double-buffered stage's canvas
-// without copying the canvas.
-template <class T>
-__host__ __device__ __forceinline__ void ghost_value(const Plan3Dev& p, const T* Q, int r, int r0, int count, T* buf) {
-  const int n = p.NI * p.NJ * p.NK;
-  const int ghost = p.g_ghost[r], src = p.g_source[r], kind = p.g_kind[r];
-  if (ghost < 0 || ghost >= n || src < 0 || src >= n) return;   // validated on the host
-  T q[NV3_MAX], o[NV3_MAX];
-  for (int v = 0; v < p.nvar; ++v) q[v] = Q[(size_t)v * n + src];
-  condition3(kind, q, p.g_normal[3 * r], p.g_normal[3 * r + 1], p.g_normal[3 * r + 2], p.P, p.nvar, o);
-  for (int v = 0; v < p.nvar; ++v) buf[(size_t)v * count + (r - r0)] = o[v];
-}
-
-template <class T>
-__host__ __device__ __forceinline__ void ghost_store(const Plan3Dev& p, const T* buf, int r, int r0, int count, T* Q) {
-  const int n = p.NI * p.NJ * p.NK;
-  const int ghost = p.g_ghost[r], src = p.g_source[r];
-  if (ghost < 0 || ghost >= n || src < 0 || src >= n) return;
-  for (int v = 0; v < p.nvar; ++v) Q[(size_t)v * n + ghost] = buf[(size_t)v * count + (r - r0)];
 }
 
 // The state of the ghost whose program is g (Plan3Dev::ghost_of), from U (and its tangent
@@ -111,10 +67,6 @@ __host__ __device__ __forceinline__ int face_flat(const Plan3Dev& p, int a, int 
 }
 
 __host__ __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
-
-struct Cell3 {
-  int i, j, k;
-};
 
 __host__ __device__ __forceinline__ int cell_index(const Plan3Dev& p, int i, int j, int k) {
   i = clampi(i, 0, p.NI - 1);
@@ -184,8 +136,9 @@ __host__ __device__ __forceinline__ T grad_var(const Plan3Dev& p, const T* Q, in
   return Q[(size_t)5 * n + c];
 }
 
-// component m of node_phi: the same three halvings of the eight cells' values, one
-// component at a time (a face's gradient then never holds all eight cells' values)
+// the mean of component m of grad_vars over the eight cells round node (I, J, K), averaged axis by
+// axis: i, then j, then k (one component at a time: a face's gradient then never holds all
+// eight cells' values)
 template <class T>
 __host__ __device__ __forceinline__ T node_phi_m(const Plan3Dev& p, const T* Q, int I, int J, int K, int m) {
   T jk[2][2];
@@ -199,22 +152,6 @@ __host__ __device__ __forceinline__ T node_phi_m(const Plan3Dev& p, const T* Q, 
 #pragma unroll
   for (int d = 0; d < 2; ++d) kk[d] = 0.5 * (jk[0][d] + jk[1][d]);
   return 0.5 * (kk[0] + kk[1]);
-}
-
-template <class T>
-__host__ __device__ __forceinline__ void node_phi(const Plan3Dev& p, const T* Q, int I, int J, int K, int nphi, T out[5]) {
-  T c[2][2][2][5];
-  for (int a = 0; a < 2; ++a)
-    for (int b = 0; b < 2; ++b)
-      for (int d = 0; d < 2; ++d) grad_vars(p, Q, cell_index(p, I - 1 + a, J - 1 + b, K - 1 + d), c[a][b][d]);
-  for (int m = 0; m < nphi; ++m) {
-    T jk[2][2];
-    for (int b = 0; b < 2; ++b)
-      for (int d = 0; d < 2; ++d) jk[b][d] = 0.5 * (c[0][b][d][m] + c[1][b][d][m]);
-    T kk[2];
-    for (int d = 0; d < 2; ++d) kk[d] = 0.5 * (jk[0][d] + jk[1][d]);
-    out[m] = 0.5 * (kk[0] + kk[1]);
-  }
 }
 
 __host__ __device__ __forceinline__ void cross3(const double a[3], const double b[3], double out[3]) {
@@ -395,11 +332,11 @@ __host__ __device__ __forceinline__ void qcr_extra(const T grad[3][5], const T& 
 }
 
 // FO: 1 first order, 2 second order, 0 as `first_order` says (the kernels fix it at
-// compile time, so a first-order flux loads only the two cells either side).  PART: 0 the
-// whole flux; 3 the same with its gradient from the plan's stored geometry; 1 its inviscid
-// part (with the SA row's upwind convection); 2 its viscous part alone, the terms the whole
-// flux subtracts, negated (0 - term), so that part 1 plus part 2 is the whole flux bitwise
-// (a + (0 - b) == a - b).
+// compile time, so a first-order flux loads only the two cells either side).  A viscous
+// gradient takes the plan's stored geometry and the evaluation's node values.  PART: 0 the
+// whole flux; 1 its inviscid part (with the SA row's upwind convection); 2 its viscous part
+// alone, the terms the whole flux subtracts, negated (0 - term), so that part 1 plus part 2
+// is the whole flux bitwise (a + (0 - b) == a - b).
 template <class T, bool VISC, bool SA, int FO = 0, int PART = 0>
 __host__ __device__ void face_flux(const Plan3Dev& p, const T* Q, int a, int fi, int fj, int fk, bool first_order_arg,
                                    T F[NV3_MAX]) {
@@ -452,8 +389,7 @@ __host__ __device__ void face_flux(const Plan3Dev& p, const T* Q, int a, int fi,
   }
   if constexpr (VISC && PART != 1) {
     T grad[3][5];
-    if constexpr (PART >= 2) face_gradient_stored<T, SA ? 5 : 4>(p, qm, qp, a, fi, fj, fk, grad);
-    else face_gradient<T, SA ? 5 : 4>(p, Q, a, fi, fj, fk, grad);
+    face_gradient_stored<T, SA ? 5 : 4>(p, qm, qp, a, fi, fj, fk, grad);
     // face means of the two cells either side
     T extra[3][3];
     T vel[3], Tl = g * qm[4] / qm[0], Th = g * qp[4] / qp[0];
@@ -550,36 +486,10 @@ __host__ __device__ T sa_cell_source(const Plan3Dev& p, const T* __restrict__ Q,
   return src * vol;
 }
 
-// R of block cell c; R = U - U_inf elsewhere (tangent: v).  Each of the cell's six faces
-// evaluated here (the fused form; the device runs the two phases below).
-template <class T, bool VISC, bool SA>
-__host__ __device__ void residual_cell(const Plan3Dev& p, const T* __restrict__ Q, const double* __restrict__ U,
-                                       const double* __restrict__ dU, double* __restrict__ R, int first_order, int c) {
-  const int n = p.NI * p.NJ * p.NK;
-  if (!p.interior[c]) {
-    for (int v = 0; v < p.nvar; ++v)
-      R[(size_t)v * n + c] = dU ? dU[(size_t)v * n + c] : U[(size_t)v * n + c] - p.P.U_inf[v];
-    return;
-  }
-  const int i = c / (p.NJ * p.NK), j = (c / p.NK) % p.NJ, k = c % p.NK;
-  T acc[NV3_MAX];
-  for (int v = 0; v < p.nvar; ++v) acc[v] = cst<T>(0.0);
-  for (int a = 0; a < 3; ++a) {
-    int f0[3] = {i, j, k}, f1[3] = {i, j, k};
-    f1[a] += 1;
-    T Flo[NV3_MAX], Fhi[NV3_MAX];
-    face_flux<T, VISC, SA>(p, Q, a, f0[0], f0[1], f0[2], first_order != 0, Flo);
-    face_flux<T, VISC, SA>(p, Q, a, f1[0], f1[1], f1[2], first_order != 0, Fhi);
-    for (int v = 0; v < p.nvar; ++v) acc[v] = a == 0 ? Fhi[v] - Flo[v] : acc[v] + (Fhi[v] - Flo[v]);
-  }
-  if constexpr (SA) acc[5] = acc[5] - sa_cell_source(p, Q, c);
-  for (int v = 0; v < p.nvar; ++v) R[(size_t)v * n + c] = tangent_or_value(acc[v]);
-}
-
 // Phase 1 of the two-phase residual: the flux through face `flat` -- its value, or for
 // Dual its tangent -- stored at Fb[v * nf + flat], for a face with a block cell on
 // either side (no cell reads the others).  Every face is evaluated once instead of once
-// from each side, with the same arithmetic, so phase 2's sums are residual_cell's.
+// from each side, with the same arithmetic.
 // (PART 2: the viscous part added to the stored inviscid part; the mass row has none)
 template <class T, bool VISC, bool SA, int FO = 0, int PART = 0>
 __host__ __device__ void store_face_flux(const Plan3Dev& p, const T* __restrict__ Q, int first_order, int flat,
@@ -604,7 +514,8 @@ __host__ __device__ void store_face_flux(const Plan3Dev& p, const T* __restrict_
   }
 }
 
-// Phase 2: R of cell c from the stored face fluxes (residual_cell's sums and SA source)
+// Phase 2: R of block cell c from the stored face fluxes and the SA source; R = U - U_inf
+// elsewhere (tangent: v)
 template <class T, bool SA>
 __host__ __device__ void residual_cell_from_faces(const Plan3Dev& p, const T* __restrict__ Q,
                                                   const double* __restrict__ Fb, size_t nf,

@@ -359,8 +359,8 @@ def test_the_two_phase_residual_is_the_fused_one_bit_for_bit(harness, z, cases, 
 
 @pytest.mark.parametrize("name", NAMES)
 def test_the_in_place_ghost_fill_is_the_double_buffered_one(harness, z, cases, described, name):
-    """The device's ghost stages in place (each stage's values first, then its stores)
-    give the double-buffered stages' canvas bit for bit: a stage writes each ghost once."""
+    """The device's ghost fill, each ghost's chain of conditions applied to one cell's own state,
+    gives the double-buffered stages' canvas bit for bit; a stage writes each ghost once."""
     desc, _ = described[name]
     U = np.ascontiguousarray(z[f"{name}_U"])
     inplace, copying = np.zeros_like(U), np.zeros_like(U)

@@ -234,3 +234,35 @@ def test_newton_steps_with_the_coupled_and_mixed_line_solve(harness, case3d):
     assert plain[0] == coupled[0]                       # the same state before the first step
     assert np.all(np.isfinite(coupled)) and coupled[-1] < coupled[0]
     assert np.allclose(coupled, plain, rtol=5e-2)
+
+
+@pytest.mark.parametrize("state", ["sin", "rand0"])
+@pytest.mark.parametrize("sutherland,c_cr1", [(-1.0, 0.0), (0.38, 0.0), (0.38, 0.3)])
+def test_the_stored_factors_give_the_dual_number_jvp(harness, case3d, state, sutherland, c_cr1):
+    """The Newton step's product through linearize_face3's and linearize_cell3's factors against the
+    forward-mode J.v, constant viscosity, Sutherland's law and QCR2000."""
+    z, plan, desc, _ = case3d
+    harness.jr3_host_lin_jvp.restype = C.c_int
+    harness.jr3_host_lin_jvp.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    U, v = np.ascontiguousarray(z[f"{state}_U"]), np.ascontiguousarray(z[f"{state}_v"])
+    keep = desc.sutherland, desc.c_cr1
+    desc.sutherland, desc.c_cr1 = sutherland, c_cr1
+    try:
+        Jv, ref = np.zeros_like(U), evaluate(harness, desc, U, v)
+        assert harness.jr3_host_lin_jvp(C.addressof(desc), U.ctypes.data, v.ctypes.data, Jv.ctypes.data) == 0
+    finally:
+        desc.sutherland, desc.c_cr1 = keep
+    assert rows_rel(Jv[:5], ref[:5]) < 1e-12     # the bounds of the forward-mode J.v's own test
+    assert rows_rel(Jv[5:], ref[5:]) < 1e-10
+
+
+@pytest.mark.parametrize("state", ["sin", "rand0"])
+def test_the_line_terms_are_the_forms_they_restate(harness, case3d, state):
+    """line_face_terms' wave speed against wave_speed, and the closed-form coupling against the
+    flux's forward-mode Jacobian, on every face."""
+    z, plan, desc, _ = case3d
+    harness.jr3_host_line_terms.restype = C.c_int
+    harness.jr3_host_line_terms.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    U, out = np.ascontiguousarray(z[f"{state}_U"]), np.zeros(2)
+    assert harness.jr3_host_line_terms(C.addressof(desc), U.ctypes.data, out.ctypes.data) == 0
+    assert out.max() < 1e-14     # a few roundings of entries of the largest's size
