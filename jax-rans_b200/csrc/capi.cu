@@ -459,6 +459,7 @@ static BatchDims dims_of(const std::vector<CaseDev>& cases, int n_slots) {
     d.tiles_x = std::max(d.tiles_x, cd.tiles_x);
     d.tiles_y = std::max(d.tiles_y, cd.tiles_y);
     d.tiles += cd.n_tiles;
+    d.qcr |= cd.P.c_cr1 != 0.0;
     d.ghost_records = std::max(d.ghost_records, c.n_ghost[0] + c.n_ghost[1]);
     d.faces = std::max(d.faces, (c.NI + 1) * c.NJ + c.NI * (c.NJ + 1));
     d.cells = std::max(d.cells, c.NI * c.NJ);
@@ -944,6 +945,7 @@ int jr_case_load(jr_plan* plan, int32_t c, const jr_plan_desc* d) {
     upload_table(plan);
     return rc;
   }
+  compute_dims(plan);
   return upload_table(plan);
 }
 

@@ -777,11 +777,11 @@ int jac_cell_coefficients(int visc) { return visc == 2 ? JCELL : 0; }
 
 // Columns of the inviscid flux's Jacobian per evaluation (Duals): the flux's divisions and
 // roots are shared by the columns of one evaluation.
-constexpr int LIN_COLUMNS = 4;
+template <bool QCR> constexpr int LIN_COLUMNS = QCR ? 2 : 4;
 
 // Coefficients of one face at flat face index f (i-faces first, then j-faces); the face
 // lies between staged cells (ai, aj) and the next along `axis` of a double tile.
-template <int NV, int VISC, class TJ>
+template <int NV, int VISC, class TJ, bool QCR>
 __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double, NV>& s, int axis, int ai, int aj,
                                                double sx, double sy, TJ* __restrict__ jac, size_t stride,
                                                int f) {
@@ -795,23 +795,24 @@ __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double
     qb[v] = s.q[v][bi][bj];
   }
   double mass = 0.0;
-  using D = Duals<LIN_COLUMNS>;
+  constexpr int NC = LIN_COLUMNS<QCR>;
+  using D = Duals<NC>;
 #pragma unroll 1
-  for (int s0 = 0; s0 < 8; s0 += LIN_COLUMNS) {
+  for (int s0 = 0; s0 < 8; s0 += NC) {
     D qL[4], qR[4], F[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       qL[v].v = qa[v];
       qR[v].v = qb[v];
 #pragma unroll
-      for (int t = 0; t < LIN_COLUMNS; ++t) {
+      for (int t = 0; t < NC; ++t) {
         qL[v].d[t] = s0 + t == v ? 1.0 : 0.0;
         qR[v].d[t] = s0 + t == 4 + v ? 1.0 : 0.0;
       }
     }
     riemann(P.flux, qL, qR, sx, sy, g, F);
 #pragma unroll
-    for (int t = 0; t < LIN_COLUMNS; ++t) {
+    for (int t = 0; t < NC; ++t) {
       const int seed = s0 + t, base = seed < 4 ? seed : 12 + seed;   // AL[r][v] at r * 4 + v, AR[r][v] at 16 + r * 4 + v
 #pragma unroll
       for (int r = 0; r < 4; ++r) jac[(size_t)(base + 4 * r) * stride + f] = TJ(F[r].d[t]);
@@ -837,11 +838,11 @@ __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double
     double x[NX];
     face_intermediates<double, VISC>(q, phi, cxv, cyv, axis, ai, aj, x);
     using S = ViscShape<VISC>;
-    if (VISC < 2 || P.c_cr1 == 0.0) {
+    if (!QCR || P.c_cr1 == 0.0) {
       viscous_derivatives<VISC>(P, x, sx, sy, [&](int r, int k, double d) {
         jac[(size_t)(J::VBASE + S::slot(r, k)) * stride + f] = TJ(d);
       });
-    } else {   // QCR2000's stress: one evaluation a direction
+    } else if constexpr (QCR) {   // QCR2000's stress: one evaluation a direction
 #pragma unroll 1
       for (int k = 0; k < NX; ++k) {
         Dual xd[NX], out[NR];
@@ -860,9 +861,11 @@ __device__ __forceinline__ void linearize_face(const Physics& P, TileSmem<double
 // registers, some spilled): 79 us on a 385 x 97 SA case, 537 us on nine cases' 442k cells in
 // the mixed form, 31 us on a 257 x 65 Euler case, ghost maps included (one column and one
 // direction of the viscous terms at a time: 209, 2329 and 75 us; two columns and three CTAs:
-// 71, 640 and 39 us).
-template <int NV, int VISC, class TJ>
-__global__ void __launch_bounds__(TILE_THREADS, 2) k_linearize(const CaseDev* __restrict__ cases) {
+// 71, 640 and 39 us).  QCR (a launch with a case of QCR2000's stress): its fourteen directions
+// one at a time are most of the work, and need the third CTA: two columns, 205 us on a 385 x 97 case
+// and 1449 on eight, 321 and 1713 us as above.
+template <int NV, int VISC, class TJ, bool QCR = false>
+__global__ void __launch_bounds__(TILE_THREADS, QCR ? 3 : 2) k_linearize(const CaseDev* __restrict__ cases) {
   __shared__ CaseDev scase;
   if (idle_block(cases[blockIdx.z],
                  (int)blockIdx.x >= cases[blockIdx.z].tiles_x || (int)blockIdx.y >= cases[blockIdx.z].tiles_y, 0))
@@ -908,7 +911,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_linearize(const CaseDev* __
     int i = i0 + fi, j = j0 + fj;
     if (j < NJ && (interior_at(c, i - 1, j) || interior_at(c, i, j))) {
       int f = i * NJ + j;
-      linearize_face<NV, VISC, TJ>(P, s, 0, fi + 1, fj + 2, c.fi[f], c.fi[nfi + f], jac, stride, f);
+      linearize_face<NV, VISC, TJ, QCR>(P, s, 0, fi + 1, fj + 2, c.fi[f], c.fi[nfi + f], jac, stride, f);
     }
   }
   for (int e = tid; e < TILE_I * (TILE_J + 1); e += TILE_THREADS) {
@@ -916,7 +919,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 2) k_linearize(const CaseDev* __
     int i = i0 + fi, j = j0 + fj;
     if (i < NI && (interior_at(c, i, j - 1) || interior_at(c, i, j))) {
       int f = i * (NJ + 1) + j;
-      linearize_face<NV, VISC, TJ>(P, s, 1, fi + 2, fj + 1, c.fj[f], c.fj[c.nfj() + f], jac, stride, nfi + f);
+      linearize_face<NV, VISC, TJ, QCR>(P, s, 1, fi + 2, fj + 1, c.fj[f], c.fj[c.nfj() + f], jac, stride, nfi + f);
     }
   }
   if constexpr (VISC == 2) {
@@ -1436,6 +1439,8 @@ template <class T, int NV, bool SECOND, int VISC> static void configure_one() {
 }
 
 template <class TJ> static void configure_lin() {
+  cudaFuncSetAttribute(k_linearize<5, 2, TJ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(TileSmem<double, 5>));
   cudaFuncSetAttribute(k_linearize<5, 2, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(TileSmem<double, 5>));
   cudaFuncSetAttribute(k_linearize<4, 1, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1508,7 +1513,8 @@ void launch_residual_of(const CaseDev* cases, const BatchDims& d, int visc, bool
 template <class TJ>
 static void linearize_t(const CaseDev* cases, const BatchDims& d, int visc, cudaStream_t st) {
   dim3 grid(d.tiles_x, d.tiles_y, d.n_cases);
-  if (visc == 2) k_linearize<5, 2, TJ><<<grid, TILE_THREADS, sizeof(TileSmem<double, 5>), st>>>(cases);
+  if (visc == 2 && d.qcr) k_linearize<5, 2, TJ, true><<<grid, TILE_THREADS, sizeof(TileSmem<double, 5>), st>>>(cases);
+  else if (visc == 2) k_linearize<5, 2, TJ><<<grid, TILE_THREADS, sizeof(TileSmem<double, 5>), st>>>(cases);
   else if (visc == 1) k_linearize<4, 1, TJ><<<grid, TILE_THREADS, sizeof(TileSmem<double, 4>), st>>>(cases);
   else k_linearize<4, 0, TJ><<<grid, TILE_THREADS, sizeof(TileSmem<double, 4>), st>>>(cases);
 }
