@@ -18,7 +18,7 @@ static_assert(JR_STATUS_NONFINITE == ST_NONFINITE && JR_STATUS_REJECTED == ST_RE
 // residual.cu
 void launch_residual(const CaseDev*, const BatchDims&, int visc, bool second, int out_id, cudaStream_t);
 void launch_residual_of(const CaseDev*, const BatchDims&, int visc, bool second, const double* U, double* R,
-                        cudaStream_t);
+                        int own_ghosts, cudaStream_t);
 void launch_jvp(const CaseDev*, const BatchDims&, int visc, bool fp32, int tangent_id, int vdt_id, int out_id,
                 int check_active, int own_ghosts, cudaStream_t);
 void launch_ghosts(const CaseDev*, const BatchDims&, int tangent_id, int check_active, cudaStream_t);
@@ -460,6 +460,7 @@ static BatchDims dims_of(const std::vector<CaseDev>& cases, int n_slots) {
     d.tiles_y = std::max(d.tiles_y, cd.tiles_y);
     d.tiles += cd.n_tiles;
     d.qcr |= cd.P.c_cr1 != 0.0;
+    d.ghosts += c.n_ghost[0] + c.n_ghost[1];
     d.ghost_records = std::max(d.ghost_records, c.n_ghost[0] + c.n_ghost[1]);
     d.faces = std::max(d.faces, (c.NI + 1) * c.NJ + c.NI * (c.NJ + 1));
     d.cells = std::max(d.cells, c.NI * c.NJ);
@@ -750,15 +751,20 @@ int jr_residual(jr_plan* plan, const double* U, double* R, int first_order) {
   if (!plan || !U || !R) return fail(JR_EINVAL, "null argument");
   // One launch on the plan's own table: the tiles evaluate their halos' ghosts.  A case with the
   // point-vortex far field (its circulation a sum over the wall) has them filled by a launch,
-  // from a table that holds U.
-  bool vortex = false;
-  for (const CaseDev& cd : plan->host) vortex = vortex || cd.P.far_field == 1;
-  if (vortex) {
+  // from a table that holds U; so has a launch of many ghosts, whose tiles would take turns at them:
+  // one launch and two, 385 x 97 SA cases (1936 ghosts each), two 78 and 84 us a call, three 97 and 93, eight
+  // 214 and 176, one 769 x 193 case (3856) 105 and 112, two 173 and 162, 137 x 38 laminar cases (708), eight 56 and
+  // 64, 32 108 and 102, 257 x 65 Euler cases (1296), four 58 and 63, eight 78 and 76.
+  constexpr int OWN_GHOSTS = 5700;
+  bool fill = plan->dims.ghosts > OWN_GHOSTS;
+  const int own = !fill;
+  for (const CaseDev& cd : plan->host) fill = fill || cd.P.far_field == 1;
+  if (fill) {
     Adhoc a(plan);
     a.vec(&CaseDev::U, U);
     launch_ghosts(a.upload(), plan->dims, -1, 0, plan->st);
   }
-  launch_residual_of(plan->cases, plan->dims, plan->visc, first_order == 0, U, R, plan->st);
+  launch_residual_of(plan->cases, plan->dims, plan->visc, first_order == 0, U, R, own, plan->st);
   return cuda_check("jr_residual");
 }
 

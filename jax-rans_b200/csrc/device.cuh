@@ -186,6 +186,7 @@ struct BatchDims {
   int tiles_x, tiles_y;     // residual tiles
   int tiles;                // ... of all the cases together
   int ghost_records;        // both stages
+  int ghosts;               // ... of all the cases together
   int qcr;                  // some case has QCR2000's stress
   int faces, cells;         // canvas faces, canvas cells
   int n_vec;                // nvar * cells

@@ -599,7 +599,7 @@ template <> __device__ __forceinline__ double tangent_or_value<Dual>(const Dual&
 
 // out = R(U) (second or first order); partial[block] = sum vol R0^2.  T is the staged
 // scalar (double).
-template <class T, int NV, bool SECOND, int VISC>
+template <class T, int NV, bool SECOND, int VISC, bool OWN>
 __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
     k_residual(const CaseDev* __restrict__ cases, const double* U_batch, double* R_batch, int out_id, int with_partial,
                int check_active) {
@@ -622,14 +622,15 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
   const int NI = c.NI, NJ = c.NJ, N = c.ncanvas();
   const int i0 = blockIdx.y * TILE_I, j0 = blockIdx.x * TILE_J;
   const int tid = threadIdx.x;
-  // The tile's own ghosts, listed by the staging and then evaluated a thread each: in place they
-  // would be two long chains one after the other (a condition's loads, roots and quotients).  A
-  // call on a batch-long U is one launch so, without a ghost fill or a table of its own: 47.8 ->
-  // 44.4 us a call on a 65 x 17 Euler grid, 59.8 -> 55.0 us on a 385 x 97 SA grid, most of it the
-  // host's; in the Newton step the linearisation needs the filled ghosts anyway.
-  const bool own = U_batch != nullptr && P.far_field != 1;
-  __shared__ int n_own, own_list[HI * HJ];
-  if (tid == 0) n_own = 0;
+  // OWN: the tile's ghosts are listed by the staging and then evaluated a thread each (in
+  // place they would be two long chains one after the other: a condition's loads, roots and
+  // quotients), so a call on a batch-long U is one launch, without a ghost fill or a table of its
+  // own: 47.8 -> 44.4 us a call on a 65 x 17 Euler grid, 59.8 -> 55.0 us on a 385 x 97 SA grid, most of
+  // it the host's.  In the Newton step the linearisation needs the filled ghosts anyway (and the
+  // tile without this has no call frame: 1 to 2 % of its time on several cases).
+  const bool own = OWN && P.far_field != 1;
+  __shared__ int n_own, own_list[OWN ? HI * HJ : 1];
+  if (OWN && tid == 0) n_own = 0;
   if (own) __syncthreads();
   // 1. stage the primitive state of the tile and its halo
   for (int e = tid; e < HI * HJ; e += TILE_THREADS) {
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_BLOCKS)
       s.cy[li][lj] = c.centres[CI * CJ + ci * CJ + cj];
     }
   }
-  if (own) {
+  if constexpr (OWN) {
     __syncthreads();
     for (int t = tid; t < n_own; t += TILE_THREADS) {
       const int rec = own_list[t] / 256, e = own_list[t] % 256;
@@ -1434,7 +1435,9 @@ __global__ void k_cells(const CaseDev* __restrict__ cases) {
 dim3 tile_grid(const Canvas& c) { return dim3((c.NJ + TILE_J - 1) / TILE_J, (c.NI + TILE_I - 1) / TILE_I); }
 
 template <class T, int NV, bool SECOND, int VISC> static void configure_one() {
-  cudaFuncSetAttribute(k_residual<T, NV, SECOND, VISC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncSetAttribute(k_residual<T, NV, SECOND, VISC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(TileSmem<T, NV>));
+  cudaFuncSetAttribute(k_residual<T, NV, SECOND, VISC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(TileSmem<T, NV>));
 }
 
@@ -1475,37 +1478,39 @@ void configure_kernels() {
 // with fewer tiles returns at once from the excess ones).
 template <class T, int NV, bool SECOND, int VISC>
 static void launch_tile(const CaseDev* cases, const BatchDims& d, const double* U, double* R, int out_id,
-                        int with_partial, int check_active, cudaStream_t st) {
+                        int own_ghosts, cudaStream_t st) {
   dim3 grid(d.tiles_x, d.tiles_y, d.n_cases);
-  k_residual<T, NV, SECOND, VISC><<<grid, TILE_THREADS, sizeof(TileSmem<T, NV>), st>>>(cases, U, R, out_id,
-                                                                                     with_partial, check_active);
+  if (own_ghosts)
+    k_residual<T, NV, SECOND, VISC, true><<<grid, TILE_THREADS, sizeof(TileSmem<T, NV>), st>>>(cases, U, R, out_id, 1, 0);
+  else
+    k_residual<T, NV, SECOND, VISC, false><<<grid, TILE_THREADS, sizeof(TileSmem<T, NV>), st>>>(cases, U, R, out_id, 1, 0);
 }
 
 static void residual_of(const CaseDev* cases, const BatchDims& d, int visc, bool second, const double* U, double* R,
-                        int out_id, cudaStream_t st) {
+                        int out_id, int own_ghosts, cudaStream_t st) {
   if (visc == 2) {
-    if (second) launch_tile<double, 5, true, 2>(cases, d, U, R, out_id, 1, 0, st);
-    else launch_tile<double, 5, false, 2>(cases, d, U, R, out_id, 1, 0, st);
+    if (second) launch_tile<double, 5, true, 2>(cases, d, U, R, out_id, own_ghosts, st);
+    else launch_tile<double, 5, false, 2>(cases, d, U, R, out_id, own_ghosts, st);
   } else if (visc == 1) {
-    if (second) launch_tile<double, 4, true, 1>(cases, d, U, R, out_id, 1, 0, st);
-    else launch_tile<double, 4, false, 1>(cases, d, U, R, out_id, 1, 0, st);
+    if (second) launch_tile<double, 4, true, 1>(cases, d, U, R, out_id, own_ghosts, st);
+    else launch_tile<double, 4, false, 1>(cases, d, U, R, out_id, own_ghosts, st);
   } else {
-    if (second) launch_tile<double, 4, true, 0>(cases, d, U, R, out_id, 1, 0, st);
-    else launch_tile<double, 4, false, 0>(cases, d, U, R, out_id, 1, 0, st);
+    if (second) launch_tile<double, 4, true, 0>(cases, d, U, R, out_id, own_ghosts, st);
+    else launch_tile<double, 4, false, 0>(cases, d, U, R, out_id, own_ghosts, st);
   }
 }
 
 // R(U) of every case into `out_id` (second or first order), with the norm partials
 void launch_residual(const CaseDev* cases, const BatchDims& d, int visc, bool second, int out_id, cudaStream_t st) {
-  residual_of(cases, d, visc, second, nullptr, nullptr, out_id, st);
+  residual_of(cases, d, visc, second, nullptr, nullptr, out_id, 0, st);
 }
 
-// the same at U, into R: vectors over the whole batch in place of the table's own.  The tiles
-// evaluate their halos' ghosts, so none need have been filled, but for a case with the
+// the same at U, into R: vectors over the whole batch in place of the table's own.  own_ghosts: the
+// tiles evaluate their halos' ghosts, so none need have been filled, but for a case with the
 // point-vortex far field.
 void launch_residual_of(const CaseDev* cases, const BatchDims& d, int visc, bool second, const double* U, double* R,
-                        cudaStream_t st) {
-  residual_of(cases, d, visc, second, U, R, B_NONE, st);
+                        int own_ghosts, cudaStream_t st) {
+  residual_of(cases, d, visc, second, U, R, B_NONE, own_ghosts, st);
 }
 
 // The linearisation of every case's first-order residual at its U (ghosts of U filled);

@@ -64,3 +64,28 @@ def compare(DevicePlan, case, plan, flows):
         one.close()
     assert not np.array_equal(hist[:, 0], hist[:, 1])   # (the cases differ)
     batch.close()
+
+
+@pytest.mark.parametrize("cases,far", [(2, "freestream"), (9, "freestream"), (9, "point_vortex")])
+def test_a_batch_residual_is_bitwise_the_cases_alone(cuda, cases, far):
+    """The residual entry point's two ghost fills: by the tiles (few ghosts: 704 a case) or by a
+    launch (many, or a point-vortex far field; here in one case of the batch)."""
+    from jaxrans_b200.native import DevicePlan
+    case = o_grid("euler", 10)
+    plan = case.grid()
+    flows = [replace(case.flow, alpha_deg=float(a)) for a in np.linspace(-2.0, 4.0, cases)]
+    nums = [case.numerics] * cases
+    if far == "point_vortex":
+        nums[1] = replace(case.numerics, far_field="characteristic_point_vortex")
+    rng = np.random.default_rng(5)
+    states = [freestream_state(replace(case, flow=f), plan) for f in flows]
+    states = [np.where(plan.interior, u * (1.0 + 0.02 * rng.uniform(-1.0, 1.0, u.shape)), u) for u in states]
+    batch = DevicePlan.batch([plan] * cases, flows, nums, [case.implicit] * cases)
+    for first in (False, True):
+        got = batch.residual(np.concatenate([u.ravel() for u in states]), first_order=first)
+        for k in (0, 1, cases - 1):
+            one = DevicePlan(plan, flows[k], nums[k], case.implicit)
+            ref = one.residual(states[k], first_order=first)
+            one.close()
+            assert np.array_equal(got[k * ref.size:(k + 1) * ref.size], ref.ravel())
+    batch.close()
