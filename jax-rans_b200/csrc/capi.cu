@@ -28,7 +28,6 @@ int jac_cell_coefficients(int visc);
 void launch_faces(const CaseDev*, const BatchDims&, int visc, cudaStream_t);
 void launch_cells(const CaseDev*, const BatchDims&, int visc, cudaStream_t);
 dim3 tile_grid(const Canvas&);
-void configure_kernels();
 // linesolve.cu
 void launch_chain_factor(const CaseDev*, const BatchDims&, bool sa, bool fp32, cudaStream_t);
 void launch_chain_apply(const CaseDev*, const BatchDims&, bool sa, bool fp32, int src_id, int scale_on, int vout_j,
@@ -682,7 +681,6 @@ int jr_batch_create(const jr_plan_desc* descs, int32_t n_cases, jr_plan** out) {
     return rc;
   }
   compute_dims(plan);
-  configure_kernels();
   configure_line_kernels(MAX_CHAIN);
   if (cudaDeviceSynchronize() != cudaSuccess) {
     rc = cuda_check("plan create");

@@ -1434,45 +1434,9 @@ __global__ void k_cells(const CaseDev* __restrict__ cases) {
 
 dim3 tile_grid(const Canvas& c) { return dim3((c.NJ + TILE_J - 1) / TILE_J, (c.NI + TILE_I - 1) / TILE_I); }
 
-template <class T, int NV, bool SECOND, int VISC> static void configure_one() {
-  cudaFuncSetAttribute(k_residual<T, NV, SECOND, VISC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<T, NV>));
-  cudaFuncSetAttribute(k_residual<T, NV, SECOND, VISC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<T, NV>));
-}
-
-template <class TJ> static void configure_lin() {
-  cudaFuncSetAttribute(k_linearize<5, 2, TJ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<double, 5>));
-  cudaFuncSetAttribute(k_linearize<5, 2, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<double, 5>));
-  cudaFuncSetAttribute(k_linearize<4, 1, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<double, 4>));
-  cudaFuncSetAttribute(k_linearize<4, 0, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(TileSmem<double, 4>));
-  if constexpr (sizeof(TJ) == sizeof(float))
-    cudaFuncSetAttribute(k_jv<5, 2, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<5>));
-  cudaFuncSetAttribute(k_jv<4, 1, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
-  cudaFuncSetAttribute(k_jv<4, 0, TJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
-}
-
-// the tile kernels' dynamic shared memory limits, set once before any launch or capture
-void configure_kernels() {
-  cudaFuncSetAttribute(k_jv_full<5, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<5>));
-  cudaFuncSetAttribute(k_jv_full<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
-  cudaFuncSetAttribute(k_jv_full<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JvSmem<4>));
-  static bool done = false;
-  if (done) return;
-  configure_one<double, 5, true, 2>();
-  configure_one<double, 5, false, 2>();
-  configure_one<double, 4, true, 1>();
-  configure_one<double, 4, false, 1>();
-  configure_one<double, 4, true, 0>();
-  configure_one<double, 4, false, 0>();
-  configure_lin<double>();
-  configure_lin<float>();
-  done = true;
-}
+// (every tile's shared memory fits what a block may take without asking)
+static_assert(sizeof(TileSmem<double, 5>) + sizeof(CaseDev) < (46 << 10) && sizeof(JvSmem<5>) + sizeof(CaseDev) < (46 << 10),
+              "the tile kernels' shared memory");
 
 // One launch over every case of a batch: grid z = the case, x/y = the tiles (a case
 // with fewer tiles returns at once from the excess ones).
