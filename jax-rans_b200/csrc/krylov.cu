@@ -363,8 +363,12 @@ __global__ void __launch_bounds__(ORTH_THREADS, DENSE ? 4 : 2)
 #pragma unroll
       for (int i = 0; i < E; ++i)
 #pragma unroll
-        for (int k = 0; k < KB; ++k)   // (no branch: all in flight)
-          v[i][k] = V[(size_t)min(k0 + k, nk - 1) * ldv + min(e + i * ORTH_THREADS, hi - 1)];
+        for (int k = 0; k < KB; ++k) {
+          // (DENSE: the count alone would be a branch, and the loads after it wait; clamped, all are
+          // in flight.  Two elements: the second's bound is a thread's own, so the loads are predicated)
+          if constexpr (DENSE) v[i][k] = V[(size_t)min(k0 + k, nk - 1) * ldv + e];
+          else v[i][k] = k0 + k < nk && e + i * ORTH_THREADS < hi ? V[(k0 + k) * ldv + e + i * ORTH_THREADS] : 0.0;
+        }
 #pragma unroll
       for (int k = 0; k < KB; ++k)
         if (k0 + k < nk)
@@ -373,10 +377,9 @@ __global__ void __launch_bounds__(ORTH_THREADS, DENSE ? 4 : 2)
     }
 #pragma unroll
     for (int i = 0; i < E; ++i) {
-      if (e + i * ORTH_THREADS >= hi) break;
       x[i] -= s[i];
       acc[0] += x[i] * x[i];
-      w[e + i * ORTH_THREADS] = x[i];
+      if (e + i * ORTH_THREADS < hi) w[e + i * ORTH_THREADS] = x[i];
     }
   }
   if (!column || !finish_sums<8>(acc, cd.partial, cd.ticket, nb, total)) return;
