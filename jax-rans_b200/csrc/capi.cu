@@ -22,6 +22,7 @@ void launch_residual_of(const CaseDev*, const BatchDims&, int visc, bool second,
 void launch_jvp(const CaseDev*, const BatchDims&, int visc, bool fp32, int tangent_id, int vdt_id, int out_id,
                 int check_active, int own_ghosts, cudaStream_t);
 void launch_ghosts(const CaseDev*, const BatchDims&, int tangent_id, int check_active, cudaStream_t);
+void launch_ghosts_of(const CaseDev*, const BatchDims&, const double* U, cudaStream_t);
 void launch_linearize(const CaseDev*, const BatchDims&, int visc, bool fp32, cudaStream_t);
 int jac_coefficients(int visc);
 int jac_cell_coefficients(int visc);
@@ -747,21 +748,18 @@ int jr_synchronize(jr_plan* plan) {
 
 int jr_residual(jr_plan* plan, const double* U, double* R, int first_order) {
   if (!plan || !U || !R) return fail(JR_EINVAL, "null argument");
-  // One launch on the plan's own table: the tiles evaluate their halos' ghosts.  A case with the
-  // point-vortex far field (its circulation a sum over the wall) has them filled by a launch,
-  // from a table that holds U; so has a launch of many ghosts, whose tiles would take turns at them:
-  // one launch and two, 385 x 97 SA cases (1936 ghosts each), two 78 and 84 us a call, three 97 and 93, eight
-  // 214 and 176, one 769 x 193 case (3856) 105 and 112, two 173 and 162, 137 x 38 laminar cases (708), eight 56 and
-  // 64, 32 108 and 102, 257 x 65 Euler cases (1296), four 58 and 63, eight 78 and 76.
+  // On the plan's own table, U and R as arguments (nothing of a call outlives it on the host, so a
+  // caller may capture it).  One launch: the tiles evaluate their halos' ghosts.  A case with the
+  // point-vortex far field (its circulation a sum over the wall) has them filled by a launch before;
+  // so have the cases of a launch of many ghosts, whose tiles would take turns at them: one launch
+  // and two, 385 x 97 SA cases (1936 ghosts each), one 57 and 60 us a call, three 97 and 91, eight 212 and 165,
+  // one 769 x 193 case (3856) 105 and 107, two 172 and 154, eight 137 x 38 laminar cases (5664) 62 and 67, 32 107
+  // and 95, four 257 x 65 Euler cases (5184) 56 and 56, eight 77 and 67.
   constexpr int OWN_GHOSTS = 5700;
-  bool fill = plan->dims.ghosts > OWN_GHOSTS;
-  const int own = !fill;
+  const int own = plan->dims.ghosts <= OWN_GHOSTS;
+  bool fill = !own;
   for (const CaseDev& cd : plan->host) fill = fill || cd.P.far_field == 1;
-  if (fill) {
-    Adhoc a(plan);
-    a.vec(&CaseDev::U, U);
-    launch_ghosts(a.upload(), plan->dims, -1, 0, plan->st);
-  }
+  if (fill) launch_ghosts_of(plan->cases, plan->dims, U, plan->st);
   launch_residual_of(plan->cases, plan->dims, plan->visc, first_order == 0, U, R, own, plan->st);
   return cuda_check("jr_residual");
 }

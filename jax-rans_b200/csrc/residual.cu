@@ -206,8 +206,8 @@ __device__ __noinline__ void tile_ghost(const Canvas& c, const Physics& P, int t
 // corner) evaluates that stage-1 record itself rather than reading it, so no record
 // waits on another and every CTA works independently.
 template <class T>
-__global__ void __launch_bounds__(GHOST_THREADS) k_ghosts(const CaseDev* __restrict__ cases, int tangent_id,
-                                                          int check_active) {
+__global__ void __launch_bounds__(GHOST_THREADS) k_ghosts(const CaseDev* __restrict__ cases, const double* U_batch,
+                                                          int tangent_id, int check_active) {
   __shared__ CaseDev scase;
   {
     const Canvas& g = cases[blockIdx.y].c;
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(GHOST_THREADS) k_ghosts(const CaseDev* __restr
   if (!cd.enabled || (check_active && cd.sc->active == 0)) return;
   const Canvas& c = cd.c;
   const Physics& P = cd.P;
-  const double* U = cd.U;
+  const double* U = U_batch != nullptr ? U_batch + cd.vec_off : cd.U;
   const double* V = tangent_id >= 0 ? buf(cd, tangent_id) : nullptr;
   double* qg = cd.qg;
   double* dqg = cd.dqg;
@@ -1544,8 +1544,14 @@ void launch_jvp(const CaseDev* cases, const BatchDims& d, int visc, bool fp32, i
 // the ghosts of U (tangent_id < 0) or of the tangent in buffer `tangent_id`
 void launch_ghosts(const CaseDev* cases, const BatchDims& d, int tangent_id, int check_active, cudaStream_t st) {
   dim3 grid(max(1, (d.ghost_records + GHOST_THREADS - 1) / GHOST_THREADS), d.n_cases);
-  if (tangent_id >= 0) k_ghosts<Dual><<<grid, GHOST_THREADS, 0, st>>>(cases, tangent_id, check_active);
-  else k_ghosts<double><<<grid, GHOST_THREADS, 0, st>>>(cases, -1, check_active);
+  if (tangent_id >= 0) k_ghosts<Dual><<<grid, GHOST_THREADS, 0, st>>>(cases, nullptr, tangent_id, check_active);
+  else k_ghosts<double><<<grid, GHOST_THREADS, 0, st>>>(cases, nullptr, -1, check_active);
+}
+
+// the ghosts of U, a vector over the whole batch in place of the table's own
+void launch_ghosts_of(const CaseDev* cases, const BatchDims& d, const double* U, cudaStream_t st) {
+  dim3 grid(max(1, (d.ghost_records + GHOST_THREADS - 1) / GHOST_THREADS), d.n_cases);
+  k_ghosts<double><<<grid, GHOST_THREADS, 0, st>>>(cases, U, -1, 0);
 }
 
 void launch_faces(const CaseDev* cases, const BatchDims& d, int visc, cudaStream_t st) {

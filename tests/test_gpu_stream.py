@@ -55,3 +55,35 @@ def test_steps_on_a_callers_stream(cuda, name):
     finally:
         dev.lib.jr_plan_set_stream(dev.handle, None)
         dev.close()
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_a_captured_residual_call_reads_what_is_there_at_replay(cuda, many):
+    """jr_residual under a caller's stream capture, its ghosts by the tiles (one case) or by a launch
+    (more than 5700 ghosts): nothing of the captured call lives on in host memory."""
+    import torch
+    from jaxrans_b200.native import DevicePlan
+    z, case, plan = load("c_sa")
+    flows = [case.flow] * (1 + 5700 // int((~plan.interior).sum()) * 2 if many else 1)
+    dev = DevicePlan.batch(plan, flows, case.numerics, case.implicit) if many else \
+        DevicePlan(plan, case.flow, case.numerics, case.implicit)
+    rng = np.random.default_rng(9)
+    U = [np.concatenate([(freestream_state(case, plan) * (1.0 + 0.01 * rng.uniform(-1.0, 1.0, (5,) + plan.shape))).ravel()
+                         for _ in flows]) for _ in range(2)]
+    if not many:
+        U = [u.reshape((5,) + plan.shape) for u in U]
+    ref = [dev.residual(u) for u in U]
+    u, out = torch.as_tensor(U[0], device="cuda"), torch.zeros(U[0].shape, dtype=torch.float64, device="cuda")
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    assert dev.lib.jr_plan_set_stream(dev.handle, stream.cuda_stream) == 0
+    with torch.cuda.graph(graph, stream=stream):
+        assert dev.lib.jr_residual(dev.handle, u.data_ptr(), out.data_ptr(), 0) == 0
+    assert dev.lib.jr_plan_set_stream(dev.handle, None) == 0
+    for k in (0, 1, 0):
+        u.copy_(torch.as_tensor(U[k]))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy(), ref[k])
+    del graph
+    dev.close()
