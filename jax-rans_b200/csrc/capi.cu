@@ -37,6 +37,7 @@ int chain_grid_blocks(int n_chains, int n_offchain);
 bool apply_threads_valid(int threads, int max_L);
 bool apply_stage_fits(int max_L, bool fp32, int stage);
 int wait_limit_check(int tries, int* status, cudaStream_t st);
+void load_tile_kernels(int visc, bool fp32);
 void configure_line_kernels(int max_L);
 void launch_chain_couple(const CaseDev*, const BatchDims&, bool fp32, int out_id, int check_active, cudaStream_t);
 // krylov.cu
@@ -682,6 +683,7 @@ int jr_batch_create(const jr_plan_desc* descs, int32_t n_cases, jr_plan** out) {
     return rc;
   }
   compute_dims(plan);
+  load_tile_kernels(plan->visc, plan->mixed);
   configure_line_kernels(MAX_CHAIN);
   if (cudaDeviceSynchronize() != cudaSuccess) {
     rc = cuda_check("plan create");

@@ -1438,6 +1438,32 @@ dim3 tile_grid(const Canvas& c) { return dim3((c.NJ + TILE_J - 1) / TILE_J, (c.N
 static_assert(sizeof(TileSmem<double, 5>) + sizeof(CaseDev) < (46 << 10) && sizeof(JvSmem<5>) + sizeof(CaseDev) < (46 << 10),
               "the tile kernels' shared memory");
 
+// Loads the tile kernels a plan of this model and precision runs, when the plan is made: the first
+// one a process loads takes 10 ms, which would fall to its first call
+template <class K> static void load_kernel(K kernel) {
+  cudaFuncAttributes a;
+  cudaFuncGetAttributes(&a, kernel);
+}
+template <int NV, int VISC> static void load_tiles(bool fp32) {
+  load_kernel(k_residual<double, NV, true, VISC, true>);
+  load_kernel(k_residual<double, NV, true, VISC, false>);
+  load_kernel(k_residual<double, NV, false, VISC, true>);
+  load_kernel(k_residual<double, NV, false, VISC, false>);
+  if (fp32) {
+    load_kernel(k_linearize<NV, VISC, float>);
+    load_kernel(k_jv<NV, VISC, float>);
+  } else {
+    load_kernel(k_linearize<NV, VISC, double>);
+    load_kernel(k_jv_full<NV, VISC>);
+    if constexpr (VISC < 2) load_kernel(k_jv<NV, VISC, double>);
+  }
+}
+void load_tile_kernels(int visc, bool fp32) {
+  if (visc == 2) load_tiles<5, 2>(fp32);
+  else if (visc == 1) load_tiles<4, 1>(fp32);
+  else load_tiles<4, 0>(fp32);
+}
+
 // One launch over every case of a batch: grid z = the case, x/y = the tiles (a case
 // with fewer tiles returns at once from the excess ones).
 template <class T, int NV, bool SECOND, int VISC>
