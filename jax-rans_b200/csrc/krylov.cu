@@ -200,7 +200,8 @@ __global__ void k_cycle_gate(const CaseDev* __restrict__ cases, int n_cases, cud
 // rounds of loads, the sums' two stages; the three over 8, 15 and 30 vectors take 25, 29 and 37 us, on a
 // 769 x 193 case 35, 58 and 134 us (a warp a vector, the second pass reading the basis twice: 29, 38 and
 // 54 us; 45, 76 and 189 us).  E by those two cases: at one element a thread the 769 x 193 case takes 37
-// and 65 us over 8 and 15 vectors, over 30 the same (and two would spill).
+// and 65 us over 8 and 15 vectors, over 30 the same (two would spill; four of eight with the update
+// spill 20 bytes).
 
 // The dots of the NK vectors from k0 (nk of them) with w, after (UPDATE) w -= sum h V over the
 // same vectors.  second: h1 in, h2 out; else h1 out.

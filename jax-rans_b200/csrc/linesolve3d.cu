@@ -66,7 +66,8 @@ __global__ void __launch_bounds__(64) k3_line_factor(Plan3Dev p, const double* _
 // `row` holds its row's words and the vector's entry, the other rows' entries come by
 // shuffles, and the words of the two elements ahead are in flight.  Bound by the factor's
 // bytes where many chains run, by the sweeps' latency where few do: 61,440 coupled FP32 chains
-// of 64, 638 us (one thread a chain and a copy of the whole vector first: 1.14 ms); 3,072
+// of 64, 638 us back to back, 0.80 ms in a step under the power cap (one thread a chain and a copy
+// of the whole vector first: 1.14 ms); 3,072
 // FP64 chains of 16, 21 us (231 us).  The blocks after the chains' copy the cells on no chain.
 constexpr int LA_THREADS = 128, LA_CHAINS = LA_THREADS / 32 * LW_CHAINS;
 

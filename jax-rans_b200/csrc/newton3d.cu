@@ -64,7 +64,11 @@ __global__ void k3_dot_partial(size_t N, const double* __restrict__ a, const dou
 // sums fill the registers, and 32 x 16 bytes a thread are what the reads need in flight.  On
 // the 3.9M-cell wing (215 MB a vector) bound by HBM: pass 0 against 17 to 30 vectors reads
 // 6.8 TB/s, pass 1 4.9; a step's three passes over 30 vectors 1.9 ms on average where separate
-// dots (w read again for each vector) and updates took 2.8.  The sums are fixed by N alone.
+// dots (w read again for each vector) and updates took 2.8.  The two-element updates spill: 124
+// bytes a thread at 16 vectors (two blocks an SM), 116 at 32.  Means over the vectors each form
+// takes in a cycle of 30, passes 0 and 1: 1 to 8 vectors 9 and 7 us on a 49k-cell wing, 9 to 16
+// 14 and 13, 17 to 30 22 and 27; on the 3.9M-cell wing 9 to 16 409 and 538 us, 17 to 30 844 and 1194.
+// The sums are fixed by N alone.
 template <int E> struct Elems {
   double x[E];
 };
